@@ -49,8 +49,8 @@ def listed():
         # blobs of many sizes in float frames: the LoG scale space
         dict(name="log_1024_f32", kind="log", frames=64, height=1024, width=1024, spots=600, min_radius=2.0,
              max_radius=8.0, n_radii=10, link=6.0, memory=0),
-        # a folder of recordings of uneven size and length in one call
-        dict(name="folder_16_videos", kind="videos", videos=16, side_lo=256, side_hi=2048, frames_lo=13,
+        # a folder of recordings of uneven size and length in one call, for their trajectories alone
+        dict(name="folder_10_videos", kind="videos", videos=10, side_lo=256, side_hi=2048, frames_lo=13,
              frames_hi=125, diameter=11, link=7.0, memory=3),
         # properties of given points (found by another program) in every frame of a movie
         dict(name="points_1024_u16", kind="points", frames=64, height=1024, width=1024, spots=500, diameter=11,
@@ -99,7 +99,7 @@ def draw(rng):
                     spots=max(8, int(0.8 * density * h * w)), min_radius=2.0, max_radius=rng.choice([5.0, 6.5, 8.0]),
                     n_radii=rng.randint(4, 10), link=6.0, memory=rng.randint(0, 2))
     if kind == "videos":
-        return dict(kind="videos", videos=rng.randint(4, 20), side_lo=256, side_hi=_log_int(rng, 700, 2048),
+        return dict(kind="videos", videos=rng.randint(3, 10), side_lo=256, side_hi=_log_int(rng, 700, 2048),
                     frames_lo=10, frames_hi=_log_int(rng, 20, 100), diameter=rng.choice([9, 11]), link=7.0,
                     memory=rng.randint(0, 3))
     if kind == "points":
@@ -205,7 +205,8 @@ def _sigma(diameter):
 
 def _snr(diameter, kind):
     """Peak over noise, from what the smoothing of the diameter still tells from noise."""
-    return 12.0 if kind == "learned" else max(9.0, 9.0 * (11.0 / diameter) ** 2), 35.0
+    lowest = {"learned": 12.0, "vignette": 15.0}.get(kind, 9.0)
+    return max(lowest, 9.0 * (11.0 / diameter) ** 2), 35.0
 
 
 def _minmass(diameter, noise):
@@ -222,6 +223,8 @@ def _options(case):
             noise = 0.12  # of the frames divided by the smoothed mean
             kw.update(snr=case["snr"], correct_illumination=True)
         kw["minmass"] = _minmass(case["diameter"], noise)
+        if kind == "videos":
+            kw.update(characterize=False, doughnut_correction=False)
     elif kind == "log":
         kw.update(n_radii=case["n_radii"], log_spacing=True, minmass=150.0)
     if case.get("link") and kind != "link":
@@ -286,8 +289,8 @@ def prepare(case, seed):
         dtype = case.get("dtype", "f32" if kind == "log" else "u16")
         sigma = (2.0 / math.sqrt(2.0), case["max_radius"] / math.sqrt(2.0)) if kind == "log" else _sigma(d)
         bg = 50.0 if kind == "log" else case.get("bg", 100.0)
-        state["movie"] = _frames(seed, tracks, h, w, dtype, bg, sigma, _snr(d, kind),
-                                 case.get("vignette", False))
+        state["movie"] = _frames(seed, tracks, h, w, dtype, bg, sigma,
+                                 _snr(d, "vignette" if case.get("vignette") else kind), case.get("vignette", False))
         if case.get("host"):
             state["movie"] = state["movie"].cpu().numpy()
         if kind == "points":
@@ -330,8 +333,7 @@ def run(state):
         return _padded(_columns(gt.LoG(state["movie"], case["min_radius"], case["max_radius"], **kw)),
                        2 * case["frames"] * case["spots"] + 1000)
     if kind == "videos":
-        tables = [_columns(t) for t in gt.batch_videos(state["videos"], case["diameter"], **kw)]
-        return {name: np.concatenate([t[name] for t in tables]) for name in tables[0]}
+        return [_columns(table) for table in gt.batch_videos(state["videos"], case["diameter"], **kw)]
     if kind == "points":
         return _columns(gt.characterize_points(state["movie"], state["points"], case["diameter"], has_frames=True,
                                                **kw))
@@ -365,7 +367,7 @@ def work(case):
         pixels = case["frames"] * case["height"] * case["width"]
         rows = case["frames"] * case["spots"]
         taps, itemsize = case.get("diameter", 17), size[case.get("dtype", "f32" if kind == "log" else "u16")]
-    out = rows * (11 + 2 * bool(case.get("link"))) * 4
+    out = rows * ((4 if kind == "videos" else 11) + 2 * bool(case.get("link"))) * 4
     per_pixel = 2 * 2 * taps + 12  # two tap passes, two running sums, the window maxima
     if kind == "learned":
         per_pixel = cell_flops / 16
