@@ -301,6 +301,9 @@ struct PipeLink {
     int64_t C = 0, list_cap = 0, max_items = 0;
     size_t scan_bytes = 0;
     int64_t nwin = 0;   // windows issued in this call
+    bool segmented = false;
+    LinkSegs segs;      // segments of a window (link_segments_kernel)
+    int seg_len = 0, seg_len_last = 0;
     float bin_w = 1.0f;  // row-bin width of the neighbour search index
 
     gt_status setup(gt_ctx* c, int64_t NT, uint32_t feat_cap, int SC, float radius, int memory,
@@ -352,12 +355,35 @@ struct PipeLink {
         const int32_t vg[2] = {0, (int32_t)NT};
         CK(cudaMemcpyAsync(ctx->w_vgrp.p, vg, sizeof(vg), cudaMemcpyHostToDevice, ctx->lk));
         CK(cudaMemcpyAsync(ctx->w_reset.p, reset.data(), NT, cudaMemcpyHostToDevice, ctx->lk));
-        // the per-point linker arrays start cleared: stamps -1, first positions 0
-        size_t o_id, o_src, o_first;
-        link_scratch_point_arrays(S.max_group, S.max_edges, NS, memory, &o_id, &o_src, &o_first);
-        CK(cudaMemsetAsync(S.base + o_id, 0xFF, NS * 4, ctx->lk));
-        CK(cudaMemsetAsync(S.base + o_src, 0xFF, NS * 4, ctx->lk));
-        CK(cudaMemsetAsync(S.base + o_first, 0, NS * 8, ctx->lk));
+        // Without linker resets the frames of a window link in segments, one
+        // CTA each.  16 frames a segment beside locating (8 SMs for less than
+        // a millisecond a window); the shortest ones in the last window, which
+        // nothing is left to hide.
+        segmented = memory <= kLinkSegMemory && std::find(reset.begin(), reset.end(), 1) == reset.end();
+        out.dur_range = segmented ? 1 : 0;
+        if (segmented) {
+            seg_len_last = link_segment_min(memory);
+            seg_len = std::max(16, seg_len_last);
+            segs.prefix = link_segment_prefix(memory);
+            segs.max_segs = std::max((SC + seg_len_last - 1) / seg_len_last, 1);
+            segs.points = (int64_t)(seg_len + segs.prefix) * C;
+            segs.bytes = link_segment_bytes(S.max_group, S.max_edges, segs.points, memory);
+            CK(ctx->w_segs.ensure(segs.bytes * (size_t)(segs.max_segs - 1)));
+            CK(ctx->w_segst.ensure(sizeof(LinkSeg) * (size_t)segs.max_segs));
+            CK(ctx->w_segarr.ensure(4));
+            segs.base = ctx->w_segs.as<uint8_t>();
+            segs.seg = ctx->w_segst.as<LinkSeg>();
+            segs.arrived = ctx->w_segarr.as<uint32_t>();
+            CK(cudaMemsetAsync(segs.arrived, 0, 4, ctx->lk));
+            CK(cudaMemsetAsync(ctx->w_dur.p, 0, NS * 8, ctx->lk));
+        } else {
+            // the per-point linker arrays start cleared: stamps -1, first positions 0
+            size_t o_id, o_src, o_first;
+            link_scratch_point_arrays(S.max_group, S.max_edges, NS, memory, &o_id, &o_src, &o_first);
+            CK(cudaMemsetAsync(S.base + o_id, 0xFF, NS * 4, ctx->lk));
+            CK(cudaMemsetAsync(S.base + o_src, 0xFF, NS * 4, ctx->lk));
+            CK(cudaMemsetAsync(S.base + o_first, 0, NS * 8, ctx->lk));
+        }
         CK(cudaMemsetAsync(ctx->w_flags.p, 0, 4, ctx->lk));
         CK(cudaMemsetAsync(ctx->w_cnt.p, 0, 8, ctx->lk));
         // the host buffers above are read before the call returns
@@ -443,7 +469,12 @@ struct PipeLink {
         w.state = (LinkState*)ctx->w_state.p;
         {
             Prof pf(ctx, "link_video", ctx->lk);
-            CK(link_run_window(in, L, S, out, w, ctx->lk));
+            if (segmented) {
+                segs.len = last ? seg_len_last : seg_len;
+                CK(link_run_segments(in, L, S, out, w, segs, (int64_t)s0 * C, (int64_t)s1 * C, ctx->lk));
+            } else {
+                CK(link_run_window(in, L, S, out, w, ctx->lk));
+            }
         }
         CK(cudaEventRecord(ctx->w_linked[b], ctx->lk));
         return GT_OK;

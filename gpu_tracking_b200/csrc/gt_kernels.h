@@ -304,6 +304,42 @@ struct LinkOutput {
     int64_t* dur;        // per video region of npoints_video: durations by id
     int64_t* vpoff;      // per video: first point index (nvideos+1)
     uint32_t* flags;     // per video error flags
+    // dur holds, per id, two int32 instead of a duration: INT32_MAX - first
+    // frame and last frame + 1, each the maximum over the id's points
+    int32_t dur_range = 0;
+};
+
+// One segment of a video's frames (link_segments_kernel).
+struct LinkSeg {
+    long long c0, counter;   // the run's id counter at the segment's first frame and at its end
+    long long base;          // final id of the first id it gave in the segment
+    int32_t head;            // ring slot that the next frame replaces
+    int32_t final_ids;       // the ids it wrote are final
+    uint32_t flags;          // error flags of a speculative run
+};
+
+// Frames a speculative run starts early.  Without memory its state is the
+// detections of the frame before, whatever came earlier.  With memory the
+// ring has lost every entry from before the start after memory + 1 frames;
+// as many again, and two, for the matches that those entries would have
+// changed to stop mattering (fewer: more boundaries that do not hold).
+constexpr int link_segment_prefix(int memory) { return memory == 0 ? 1 : 2 * (memory + 1) + 2; }
+// Shortest segment: at least the prefix (half of the work is then the
+// segment's own) and, for the comparison at its end, memory + 2.
+constexpr int link_segment_min(int memory) {
+    return link_segment_prefix(memory) > 8 ? link_segment_prefix(memory) : 8;
+}
+constexpr int kLinkSegMemory = 16;   // larger memories keep the sequential linker (prefixes of 36 frames and more)
+
+// Segments of `len` frames (at least memory + 2), each run from `prefix`
+// frames before its first one.
+struct LinkSegs {
+    int32_t len = 0, prefix = 0, max_segs = 0;
+    uint8_t* base = nullptr;      // scratch of the speculative runs: nvideos x (max_segs - 1)
+    size_t bytes = 0;             // link_segment_bytes of one
+    int64_t points = 0;           // points that len + prefix frames hold at most (slot mode: slots)
+    LinkSeg* seg = nullptr;       // nvideos x max_segs
+    uint32_t* arrived = nullptr;  // per video, zero before the first launch
 };
 
 cudaError_t link_sort_groups(const LinkInput& in, uint32_t* srt, uint8_t* scratch, size_t scratch_per_group,
@@ -329,6 +365,12 @@ cudaError_t link_run(const LinkInput& in, const LinkLists& L, const LinkScratch&
                      cudaStream_t st);
 cudaError_t link_run_window(const LinkInput& in, const LinkLists& L, const LinkScratch& S, const LinkOutput& out,
                             const LinkWindow& w, cudaStream_t st);
+// The same ids from one CTA per segment of frames.  No frame may have its reset flag set
+// and memory is at most 64.  Points [p0, p1) are those of the frames linked;
+// with out.dur_range, out.dur is zero before the first window.
+size_t link_segment_bytes(int32_t max_group, int64_t max_edges, int64_t npoints, int32_t memory);
+cudaError_t link_run_segments(const LinkInput& in, const LinkLists& L, const LinkScratch& S, const LinkOutput& out,
+                              const LinkWindow& w, const LinkSegs& q, int64_t p0, int64_t p1, cudaStream_t st);
 cudaError_t link_durations(const LinkInput& in, const LinkOutput& out, int64_t* row_dur, cudaStream_t st);
 // slot mode: particle ids (through the f32 round trip) and durations of every
 // point written to table rows row_off[g] + j

@@ -10,14 +10,18 @@
 //                        forward (dests in group+k) and backward (sources in
 //                        group-k) neighbour lists in ascending point order; all
 //                        frame pairs in parallel.
-//   link_video_kernel    one CTA per video walks its frames in order (the
-//                        linker's only true sequential dependency) doing each
-//                        frame's work in parallel: memory merge, subnet
+//   link_frames          the frame loop: one CTA walks frames in order doing
+//                        each frame's work in parallel: memory merge, subnet
 //                        detection by union-find, the reference's DFS order
 //                        per subnet, the exact branch-and-bound per subnet
 //                        (one thread each, same float operation sequence),
 //                        new ids in destination order, memory ring and
 //                        duration bookkeeping.
+//   link_segments_kernel the loop over segments of a video's frames, one CTA
+//                        each, joined where their states agree.
+//   link_video_kernel    the loop over a whole video or window in one CTA:
+//                        videos with linker resets, memory above 16, videos of
+//                        one segment and callers without scratch.
 #include "gt_kernels.h"
 
 namespace gt {
@@ -253,13 +257,13 @@ __global__ void lists_kernel(LinkInput in, LinkLists L, int64_t* f_cnt, int64_t*
 // out_src, parent, comp_nd, comp_ns, comp_off, comp_soff, roots, tmp);
 // sblk: per-source sf0, sf1 (int64), src_pt (int32), srcUsed (u8), Smax each.
 struct Lay {
-    size_t start, idstamp, firstpos, srcidx, srcstamp, ring_pt, ring_n, ringpre, dblk, sblk, e_src, e_dist, pathD,
+    size_t pids, snap, start, idstamp, firstpos, srcidx, srcstamp, ring_pt, ring_n, ringpre, dblk, sblk, e_src, e_dist, pathD,
         pathS, srcLocal, vis_d, vis_s, stack, r2a, r2b, r2c, r2used, total;
 };
 
 __host__ __device__ inline size_t al(size_t x) { return (x + 15) & ~(size_t)15; }
 
-__host__ __device__ inline Lay make_lay(int64_t G, int64_t E, int64_t NP, int64_t M) {
+__host__ __device__ inline Lay make_lay(int64_t G, int64_t E, int64_t NP, int64_t M, bool spec) {
     Lay l;
     const int64_t Smax = G * (M + 1);
     size_t o = 0;
@@ -285,17 +289,20 @@ __host__ __device__ inline Lay make_lay(int64_t G, int64_t E, int64_t NP, int64_
     l.r2b = o; o = al(o + 4 * G);
     l.r2c = o; o = al(o + 4 * G);
     l.r2used = o; o = al(o + Smax);
+    // speculative runs: ids of the frames before their own, ring and ring sizes as they reach them
+    l.pids = o; o = spec ? al(o + 8 * NP) : o;
+    l.snap = o; o = spec ? al(o + 4 * (M * G + M + 1)) : o;
     l.total = o;
     return l;
 }
 
 size_t link_scratch_bytes(int32_t max_group, int64_t max_edges, int64_t npoints_video, int32_t memory) {
-    return make_lay(max_group, max_edges, npoints_video, memory).total;
+    return make_lay(max_group, max_edges, npoints_video, memory, false).total;
 }
 
 void link_scratch_point_arrays(int32_t max_group, int64_t max_edges, int64_t npoints_video, int32_t memory,
                                size_t* idstamp, size_t* srcstamp, size_t* firstpos) {
-    const Lay l = make_lay(max_group, max_edges, npoints_video, memory);
+    const Lay l = make_lay(max_group, max_edges, npoints_video, memory, false);
     *idstamp = l.idstamp;
     *srcstamp = l.srcstamp;
     *firstpos = l.firstpos;
@@ -322,30 +329,51 @@ __device__ __forceinline__ void uf_union(volatile int* parent, int a, int b) {
     }
 }
 
-template <typename SF>
-__global__ void __launch_bounds__(kLinkThreads)
-link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, LinkWindow W) {
+// Block-wide state of a linker run, carried from frame to frame.
+struct LinkShared {
+    int wsum[33];
+    long long wsum64[33];
+    int ring_n[kRingSmem + 1], ringpre[kRingSmem + 2];
+    long long counter, frame, load;
+    int prevg, head, nroots, ringtot;
+};
+
+// What a run of consecutive frames works on.  A run of a whole video (or of
+// the window that follows one) has spec = false and lp0 = own_g = gfirst's
+// video start.  A speculative run (spec) starts `prefix` frames before the
+// frames it owns with an empty state and numbers its ids from 0: its
+// per-point arrays cover the points from lp0 on, the ids of the points before
+// frame own_g go to its own scratch, and its state as it reaches own_g is kept
+// for the comparison with the run before it.
+struct LinkRun {
+    uint8_t* base;      // scratch, make_lay(G, E, NP, M, spec)
+    int64_t NP;         // points (and ids) the per-point arrays cover
+    int64_t lp0;        // first point they cover, relative to the video
+    int gfirst;         // first frame whose points can be sources
+    int own_g;          // first frame whose ids the run writes to the output
+    uint32_t* flags;
+    long long* c0;      // spec: id counter at own_g
+    bool spec;
+};
+
+// Links frames [g_lo, g_hi) of video v from the state in sh.  SEG: durations
+// are left to the caller (the ids of a speculative run are not final).
+template <typename SF, bool SEG>
+__device__ __forceinline__ void link_frames(const LinkInput& in, const LinkLists& L, const LinkScratch& S,
+                                            const LinkOutput& out, const int gb, const LinkRun& run, const int g_lo,
+                                            const int g_hi, LinkShared& sh) {
     constexpr int kLinkSmemD = LinkSmem<SF>::D, kLinkSmemS = LinkSmem<SF>::S;
-    __shared__ int wsum[33];
-    __shared__ long long wsum64[33];
-    __shared__ int sh_ring_n[kRingSmem + 1], sh_ringpre[kRingSmem + 2];
-    __shared__ long long sh_counter, sh_frame, sh_load;
-    __shared__ int sh_prevg, sh_head, sh_nroots, sh_ringtot;
-    const int v = blockIdx.x;
-    const int gb = in.vgrp[v], ge = in.vgrp[v + 1];
-    const int g_lo = (W.g0 < 0) ? gb : W.g0, g_hi = (W.g0 < 0) ? ge : W.g1;
-    if (out.flags[v] & kLinkStopFlags) return;  // an earlier window stopped this video
     const int64_t P0 = gbase(in, gb);
-    const int64_t NP = in.slot_stride ? (int64_t)(ge - gb) * in.slot_stride : in.goff[ge] - P0;
     const int M = in.memory, K = M + 1;
     const int G = S.max_group;
-    const Lay lay = make_lay(G, S.max_edges, S.max_points, M);
-    uint8_t* base = S.base + (size_t)v * S.bytes_per_video;
+    const Lay lay = make_lay(G, S.max_edges, run.NP, M, run.spec);
+    uint8_t* const base = run.base;
     int64_t* start = (int64_t*)(base + lay.start);
     int32_t* idstamp = (int32_t*)(base + lay.idstamp);
     unsigned long long* firstpos = (unsigned long long*)(base + lay.firstpos);
-    int32_t* srcidx = (int32_t*)(base + lay.srcidx);
-    int32_t* srcstamp = (int32_t*)(base + lay.srcstamp);
+    // the per-point arrays, indexed by the point's place in the video
+    int32_t* srcidx = (int32_t*)(base + lay.srcidx) - run.lp0;
+    int32_t* srcstamp = (int32_t*)(base + lay.srcstamp) - run.lp0;
     int32_t* ring_pt = (int32_t*)(base + lay.ring_pt);
     int32_t* ring_n = (int32_t*)(base + lay.ring_n);
     int32_t* ringpre = (int32_t*)(base + lay.ringpre);
@@ -376,56 +404,49 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
 
     // ring sizes and their prefix live in shared memory for memory <= kRingSmem
     const bool ring_smem = M <= kRingSmem;
-    int32_t* ringN = ring_smem ? sh_ring_n : ring_n;
-    int32_t* ringP = ring_smem ? sh_ringpre : ringpre;
-    if (W.first) {
-        if (W.init_points) {
-            for (int64_t i = tid; i < NP; i += nth) {
-                idstamp[i] = -1;
-                srcstamp[i] = -1;
-                firstpos[i] = 0ull;
-            }
-        }
-        for (int i = tid; i < Smax; i += nth) vis_s[i] = -1;
-        for (int i = tid; i < G; i += nth) vis_d[i] = -1;
-        for (int i = tid; i <= M; i += nth) ringN[i] = 0;
-        if (tid == 0) {
-            sh_counter = 0;
-            sh_frame = 0;
-            sh_prevg = -1;
-            sh_head = 0;
-        }
-    } else {
-        if (ring_smem)
-            for (int i = tid; i <= M; i += nth) ringN[i] = ring_n[i];
-    }
-    if (!W.first && tid == 0) {
-        const LinkState st = W.state[v];
-        sh_counter = st.counter;
-        sh_frame = st.frame;
-        sh_prevg = st.prevg;
-        sh_head = st.head;
-    }
-    __syncthreads();
+    int32_t* ringN = ring_smem ? sh.ring_n : ring_n;
+    int32_t* ringP = ring_smem ? sh.ringpre : ringpre;
+    int64_t* const pids = SEG ? (int64_t*)(base + lay.pids) - run.lp0 : nullptr;
+    // first frame and point whose ids go to the output (true-state runs: all of them)
+    const int32_t own_g = (SEG && run.spec) ? run.own_g : INT32_MIN;
+    const int64_t own_lp = (SEG && run.spec) ? gbase(in, own_g) - P0 : INT64_MIN;
+    // id of point lp of the video
+    auto id_of = [&](int64_t lp) -> int64_t {
+        return (SEG && lp < own_lp) ? pids[lp] : ids[P0 + lp];
+    };
 
     for (int g = g_lo; g < g_hi; g++) {
         const int step = g - gb;
-        if (in.reset[g]) {
+        if (!SEG && in.reset[g]) {
             // Linker::reset (src/linking.rs:401-403, src/execute_gpu.rs:792-798)
             if (tid == 0) {
-                sh_counter = 0;
-                sh_frame = 0;
-                sh_prevg = -1;
-                sh_head = 0;
+                sh.counter = 0;
+                sh.frame = 0;
+                sh.prevg = -1;
+                sh.head = 0;
             }
             for (int i = tid; i <= M; i += nth) ringN[i] = 0;
             __syncthreads();
         }
         const int64_t a = gbase(in, g);
         const int D = (int)gsize(in, g);
-        const int prevg = sh_prevg;
+        const int prevg = sh.prevg;
         const int S0 = (prevg == g - 1 && prevg >= gb) ? (int)gsize(in, g - 1) : 0;
         const int64_t pa = (S0 > 0) ? gbase(in, g - 1) : 0;
+        if (SEG && g == own_g) {
+            int32_t* const snap_ring = (int32_t*)(base + lay.snap);
+            int32_t* const snap_n = snap_ring + M * (int64_t)G;
+            // the state this run reached just before its own frames
+            for (int q = 0; q < M; q++) {
+                const int slot = (sh.head + q) % M, n = ringN[slot];
+                for (int e = tid; e < n; e += nth) snap_ring[q * G + e] = ring_pt[slot * G + e];
+                if (tid == 0) snap_n[q] = n;
+            }
+            if (tid == 0) *run.c0 = sh.counter;
+        }
+        // points of frame g take their ids here, those of frame g - 1 have theirs here
+        int64_t* const idg = (SEG && g < own_g) ? pids + (a - P0) : ids + a;
+        const int64_t* const idp = (SEG && g - 1 < own_g) ? pids + (pa - P0) : ids + pa;
         // working arrays of this frame: shared memory when they fit
         int ring_all = 0;
         if (ring_smem)
@@ -455,7 +476,7 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
             int64_t idv[2];
 #pragma unroll
             for (int u = 0; u < 2; u++)
-                if (u < n2) idv[u] = ids[pa + i0 + u];
+                if (u < n2) idv[u] = idp[i0 + u];
 #pragma unroll
             for (int u = 0; u < 2; u++) {
                 if (u >= n2) break;
@@ -471,22 +492,22 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
             int tot = 0;
             for (int q = 0; q < M; q++) {
                 ringP[q] = tot;
-                tot += ringN[(sh_head + q) % M];
+                tot += ringN[(sh.head + q) % M];
             }
             ringP[M] = tot;
-            sh_ringtot = tot;
+            sh.ringtot = tot;
         }
         __syncthreads();
-        const int RT = (M > 0) ? sh_ringtot : 0;
+        const int RT = (M > 0) ? sh.ringtot : 0;
         // ring entries in ring order: position r -> (slot q, entry e)
         auto ring_lp = [&](int r) -> int32_t {
             int q = 0;
             while (ringP[q + 1] <= r) q++;
-            const int slot = (sh_head + q) % M;
+            const int slot = (sh.head + q) % M;
             return ring_pt[slot * G + (r - ringP[q])];
         };
         for (int r = tid; r < RT; r += nth) {
-            const int64_t id = ids[P0 + ring_lp(r)];
+            const int64_t id = id_of(ring_lp(r));
             if (idstamp[id] != step)
                 atomicMax(&firstpos[id], ((unsigned long long)(uint32_t)step << 32) | (0xFFFFFFFFull - (uint32_t)r));
         }
@@ -500,14 +521,14 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                 const int r = base0 + 2 * tid + u;
                 if (r < RT) {
                     lpv[u] = ring_lp(r);
-                    const int64_t id = ids[P0 + lpv[u]];
+                    const int64_t id = id_of(lpv[u]);
                     keep[u] = (idstamp[id] != step) &&
                               firstpos[id] ==
                                   (((unsigned long long)(uint32_t)step << 32) | (0xFFFFFFFFull - (uint32_t)r));
                 }
             }
             int tot;
-            const int pos = block_excl_scan(keep[0] + keep[1], &tot, wsum);
+            const int pos = block_excl_scan(keep[0] + keep[1], &tot, sh.wsum);
 #pragma unroll
             for (int u = 0; u < 2; u++) {
                 if (!keep[u]) continue;
@@ -525,8 +546,8 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
         // lists, whose size bounds the kept edges: [d_off[j], d_end[j]).
         const int64_t fb = L.b_off[lix(L, a, K, 0)];
         if (L.b_off[lix(L, a + D, K, 0)] - fb > S.max_edges) {
-            if (tid == 0) atomicOr(out.flags + v, in.slot_stride ? kFlagEdgeOverflow : kFlagScratch);
-            break;
+            if (tid == 0) atomicOr(run.flags, in.slot_stride ? kFlagEdgeOverflow : kFlagScratch);
+            return;
         }
         for (int j = tid; j < D; j += nth) {
             const int64_t pt = a + j;
@@ -551,7 +572,7 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                 float ed[kLagRegs][kEdgeRegs];
 #pragma unroll
                 for (int k = 1; k <= kLagRegs; k++) {
-                    const bool lag_on = k <= K && (k == 1 ? S0 > 0 : g - k >= gb);
+                    const bool lag_on = k <= K && (k == 1 ? S0 > 0 : g - k >= run.gfirst);
 #pragma unroll
                     for (int u = 0; u < kEdgeRegs; u++) {
                         const int64_t e = bo[k - 1] + u;
@@ -564,7 +585,7 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                 // or -1 when it is not a source of this step
 #pragma unroll
                 for (int k = 2; k <= kLagRegs; k++) {
-                    const int64_t ta = (k <= K && g - k >= gb) ? gbase(in, g - k) - P0 : 0;
+                    const int64_t ta = (k <= K && g - k >= run.gfirst) ? gbase(in, g - k) - P0 : 0;
 #pragma unroll
                     for (int u = 0; u < kEdgeRegs; u++) {
                         es[k - 1][u] = -1;
@@ -608,7 +629,7 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
             // lags K..2: only sources that are in this step's source list
             auto lag = [&](int k, int64_t o0, int64_t o1) {
                 const int t = g - k;
-                if (t < gb) return;
+                if (t < run.gfirst) return;
                 const int64_t ta = gbase(in, t) - P0;
                 for (int64_t e = o0; e < o1; e++) {
                     const int64_t lp = ta + L.b_pts[e];
@@ -692,8 +713,8 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                 const long long rd1 = (long long)isroot[1] + ((long long)nd[1] << 32);
                 long long trd;
                 int ts;
-                const long long prd = block_excl_scan64(rd0 + rd1, &trd, wsum64);
-                const int ps = block_excl_scan(ns[0] + ns[1], &ts, wsum);
+                const long long prd = block_excl_scan64(rd0 + rd1, &trd, sh.wsum64);
+                const int ps = block_excl_scan(ns[0] + ns[1], &ts, sh.wsum);
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
                     if (!isroot[u]) continue;
@@ -707,12 +728,12 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                 offs += ts;
             }
             if (tid == 0) {
-                sh_nroots = (int)(acc_rd & 0xFFFFFFFFll);
-                sh_load = 0;
+                sh.nroots = (int)(acc_rd & 0xFFFFFFFFll);
+                sh.load = 0;
             }
         }
         __syncthreads();
-        const int nroots = sh_nroots;
+        const int nroots = sh.nroots;
         // ---- P4: the reference's DFS order per subnet (recurse, linking.rs:595-621)
         for (int q = tid; q < nroots; q += nth) {
             const int r = roots[q];
@@ -760,13 +781,13 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                     if (!pushed) sp--;
                 }
             }
-            if (nd > 1) atomicAdd((unsigned long long*)&sh_load, (unsigned long long)((long long)nd * ns));
+            if (nd > 1) atomicAdd((unsigned long long*)&sh.load, (unsigned long long)((long long)nd * ns));
         }
         __syncthreads();
-        if (sh_load > 5000) {
+        if (sh.load > 5000) {
             // TooDenseToLink (src/linking.rs:677-682)
-            if (tid == 0) atomicOr(out.flags + v, kFlagTooDense);
-            break;
+            if (tid == 0) atomicOr(run.flags, kFlagTooDense);
+            return;
         }
         // ---- P5: branch and bound per subnet (recurse2, linking.rs:687-766)
         for (int q = tid; q < nroots; q += nth) {
@@ -839,19 +860,19 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                     opt[level] = op + 1;
                 }
             }
-            if (over) atomicOr(out.flags + v, kFlagSubnetBudget);
+            if (over) atomicOr(run.flags, kFlagSubnetBudget);
             for (int l = 0; l < nd; l++) {
                 int ch = has_best ? bst[l] : -1;
                 out_src[pathD[od + l]] = (ch >= 0) ? pathS[os + ch] : -1;
             }
         }
         __syncthreads();
-        if (out.flags[v] & kFlagSubnetBudget) break;
+        if (*(volatile uint32_t*)run.flags & kFlagSubnetBudget) return;
         // ---- P6: ids (new ones in destination order, src/linking.rs:788-798)
         {
             int newtot = 0;
-            const long long counter = sh_counter;
-            const long long frame = sh_frame;
+            const long long counter = sh.counter;
+            const long long frame = sh.frame;
             for (int base0 = 0; base0 < D; base0 += 2 * nth) {
                 int osrc[2], isnew[2];
 #pragma unroll
@@ -861,34 +882,33 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                     isnew[u] = (j < D && osrc[u] < 0) ? 1 : 0;
                 }
                 int tot;
-                const int pos = block_excl_scan(isnew[0] + isnew[1], &tot, wsum);
+                const int pos = block_excl_scan(isnew[0] + isnew[1], &tot, sh.wsum);
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
                     const int j = base0 + 2 * tid + u;
                     if (j >= D) break;
-                    const int64_t pt = a + j;
                     if (isnew[u]) {
                         const long long id = counter + newtot + pos + (u ? isnew[0] : 0);
-                        ids[pt] = id;
-                        start[id] = frame;
+                        idg[j] = id;
+                        if (!SEG) start[id] = frame;
                     } else {
                         const int s = osrc[u];
-                        ids[pt] = ids[P0 + src_pt[s]];
+                        idg[j] = id_of(src_pt[s]);
                         srcUsed[s] = 1;
                     }
                 }
                 newtot += tot;
             }
             __syncthreads();
-            if (tid == 0) sh_counter = counter + newtot;
+            if (tid == 0) sh.counter = counter + newtot;
         }
         // ---- P7: memory ring and durations (src/linking.rs:481-503)
         {
-            const long long frame = sh_frame;
+            const long long frame = sh.frame;
             if (M > 0) {
-                const int hs = sh_head;
+                const int hs = sh.head;
                 const int nleave = ringN[hs];
-                for (int e = tid; e < nleave; e += nth) {
+                for (int e = tid; !SEG && e < nleave; e += nth) {
                     int64_t id = ids[P0 + ring_pt[hs * G + e]];
                     dur[id] = (frame - start[id]) - M;
                 }
@@ -902,7 +922,7 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                         un[u] = (s < S0 && !srcUsed[s]) ? 1 : 0;
                     }
                     int tot;
-                    const int pos = block_excl_scan(un[0] + un[1], &tot, wsum);
+                    const int pos = block_excl_scan(un[0] + un[1], &tot, sh.wsum);
 #pragma unroll
                     for (int u = 0; u < 2; u++)
                         if (un[u]) ring_pt[hs * G + ut + pos + (u ? un[0] : 0)] = src_pt[base0 + 2 * tid + u];
@@ -910,9 +930,9 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                 }
                 if (tid == 0) {
                     ringN[hs] = ut;
-                    sh_head = (hs + 1) % M;
+                    sh.head = (hs + 1) % M;
                 }
-            } else {
+            } else if (!SEG) {
                 for (int s = tid; s < S0; s += nth) {
                     if (!srcUsed[s]) {
                         int64_t id = ids[P0 + src_pt[s]];
@@ -922,32 +942,103 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
             }
             __syncthreads();
             if (tid == 0) {
-                sh_prevg = g;
-                sh_frame = frame + 1;
+                sh.prevg = g;
+                sh.frame = frame + 1;
             }
             __syncthreads();
         }
     }
+}
+
+// Every video (or the next window of one) by one CTA, frame after frame.
+template <typename SF>
+__global__ void __launch_bounds__(kLinkThreads)
+link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, LinkWindow W) {
+    __shared__ LinkShared sh;
+    const int v = blockIdx.x;
+    const int gb = in.vgrp[v], ge = in.vgrp[v + 1];
+    const int g_lo = (W.g0 < 0) ? gb : W.g0, g_hi = (W.g0 < 0) ? ge : W.g1;
+    if (out.flags[v] & kLinkStopFlags) return;  // an earlier window stopped this video
+    const int64_t P0 = gbase(in, gb);
+    const int64_t NP = in.slot_stride ? (int64_t)(ge - gb) * in.slot_stride : in.goff[ge] - P0;
+    const int M = in.memory, K = M + 1;
+    const int G = S.max_group;
+    const Lay lay = make_lay(G, S.max_edges, S.max_points, M, false);
+    uint8_t* base = S.base + (size_t)v * S.bytes_per_video;
+    const int64_t* start = (const int64_t*)(base + lay.start);
+    int32_t* idstamp = (int32_t*)(base + lay.idstamp);
+    unsigned long long* firstpos = (unsigned long long*)(base + lay.firstpos);
+    int32_t* srcstamp = (int32_t*)(base + lay.srcstamp);
+    int32_t* ring_pt = (int32_t*)(base + lay.ring_pt);
+    int32_t* ring_n = (int32_t*)(base + lay.ring_n);
+    int32_t* vis_d = (int32_t*)(base + lay.vis_d);
+    int32_t* vis_s = (int32_t*)(base + lay.vis_s);
+    int64_t* dur = out.dur + P0;
+    int64_t* ids = out.ids;
+    const int Smax = G * K;
+    const int tid = threadIdx.x, nth = blockDim.x;
+    const bool ring_smem = M <= kRingSmem;
+    int32_t* ringN = ring_smem ? sh.ring_n : ring_n;
+    if (W.first) {
+        if (W.init_points) {
+            for (int64_t i = tid; i < NP; i += nth) {
+                idstamp[i] = -1;
+                srcstamp[i] = -1;
+                firstpos[i] = 0ull;
+            }
+        }
+        for (int i = tid; i < Smax; i += nth) vis_s[i] = -1;
+        for (int i = tid; i < G; i += nth) vis_d[i] = -1;
+        for (int i = tid; i <= M; i += nth) ringN[i] = 0;
+        if (tid == 0) {
+            sh.counter = 0;
+            sh.frame = 0;
+            sh.prevg = -1;
+            sh.head = 0;
+        }
+    } else {
+        if (ring_smem)
+            for (int i = tid; i <= M; i += nth) ringN[i] = ring_n[i];
+    }
+    if (!W.first && tid == 0) {
+        const LinkState st = W.state[v];
+        sh.counter = st.counter;
+        sh.frame = st.frame;
+        sh.prevg = st.prevg;
+        sh.head = st.head;
+    }
+    __syncthreads();
+
+    LinkRun run;
+    run.base = base;
+    run.NP = S.max_points;
+    run.lp0 = 0;
+    run.gfirst = gb;
+    run.own_g = gb;
+    run.flags = out.flags + v;
+    run.c0 = nullptr;
+    run.spec = false;
+    link_frames<SF, false>(in, L, S, out, gb, run, g_lo, g_hi, sh);
     __syncthreads();
     if (!W.last) {
         if (ring_smem)
             for (int i = tid; i <= M; i += nth) ring_n[i] = ringN[i];
         if (tid == 0 && !(out.flags[v] & kLinkStopFlags)) {
             LinkState st;
-            st.counter = sh_counter;
-            st.frame = sh_frame;
-            st.prevg = sh_prevg;
-            st.head = sh_head;
+            st.counter = sh.counter;
+            st.frame = sh.frame;
+            st.prevg = sh.prevg;
+            st.head = sh.head;
             W.state[v] = st;
         }
         return;
     }
     // ---- Linker::finish (src/linking.rs:505-520)
     if (!(out.flags[v] & kLinkStopFlags)) {
-        const long long frame = sh_frame;
+        const long long frame = sh.frame;
         if (M > 0) {
             for (int q = 0; q < M; q++) {
-                int slot = (sh_head + q) % M;
+                int slot = (sh.head + q) % M;
                 int n = ringN[slot];
                 for (int e = tid; e < n; e += nth) {
                     int64_t id = ids[P0 + ring_pt[slot * G + e]];
@@ -956,8 +1047,8 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
                 __syncthreads();
             }
         }
-        if (sh_prevg >= gb) {
-            const int pg = sh_prevg;
+        if (sh.prevg >= gb) {
+            const int pg = sh.prevg;
             const int64_t pb = gbase(in, pg), pe = pb + gsize(in, pg);
             for (int64_t p = pb + tid; p < pe; p += nth) {
                 int64_t id = ids[p];
@@ -965,7 +1056,367 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
             }
         }
     }
-    if (tid == 0) out.counter[v] = sh_counter;
+    if (tid == 0) out.counter[v] = sh.counter;
+}
+
+// ------------------------------------------------------ segments of a video
+// The frame loop is serial (30-57 us a frame in one CTA), but what a frame
+// takes from the frames before it is only the detections of the last one and
+// the memory ring, and the linker compares ids for nothing but identity.  So
+// the frames are cut into segments of Q.len frames, one CTA each.  The first
+// runs from the true state; each other one starts Q.prefix frames early from
+// an empty state, which the prefix replaces by the true one up to the names
+// of the ids: old entries are out of the ring after memory + 1 frames, and a
+// match they would have changed stops mattering soon after.  The CTA that
+// ends last then goes through the boundaries in order.  Where the state a
+// segment had reached holds the same detections in the same ring order as the
+// end of the segment before it, with ids that correspond one to one, every
+// later match of the segment is the sequential linker's, and its ids are its
+// own ones renamed: those of the boundary's detections by that
+// correspondence, the new ones by an offset.  Where it does not, that CTA
+// links the segment again from the true state.  The result is the sequential
+// linker's in every case, a boundary that does not hold costs its frames.
+// Measured on a B200, one video: 400 frames of 2000 given points, memory 3,
+// 16.4 ms in one CTA and 1.64 ms here (40 segments of 10 frames, each run
+// with a prefix of 10, then about 20 us a boundary); 512 located frames of
+// 2048^2 with 2000 spots: 4.4 ms of linking left after the last frame is
+// located and 1.1 ms here.  Boundaries that did not hold: none of 39 at
+// search_range 7 and step 1.4 px, 4 of 39 at search_range 5 (3.7 ms).
+
+// Points of frames [g0, g1).
+__device__ __forceinline__ int64_t frames_points(const LinkInput& in, int g0, int g1) {
+    if (!in.slot_stride) return in.goff[g1] - in.goff[g0];
+    int64_t n = 0;
+    for (int g = g0; g < g1; g++) n += in.gcount[g];
+    return n;
+}
+
+// final id of id `id` of segment q, gmap: final ids of its first q.c0 ids
+__device__ __forceinline__ int64_t segment_id(const LinkSeg& q, const int32_t* gmap, int64_t id) {
+    if (q.final_ids) return id;
+    return id < q.c0 ? (int64_t)__ldcg(gmap + id) : q.base + (id - q.c0);
+}
+
+template <typename SF>
+__global__ void __launch_bounds__(kLinkThreads)
+link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, LinkWindow W, LinkSegs Q) {
+    __shared__ LinkShared sh;
+    __shared__ int sh_last;
+    const int v = blockIdx.y, s = blockIdx.x;
+    const int gb = in.vgrp[v], ge = in.vgrp[v + 1];
+    const int w_lo = (W.g0 < 0) ? gb : W.g0, w_hi = (W.g0 < 0) ? ge : W.g1;
+    const int nseg = max(1, (w_hi - w_lo + Q.len - 1) / Q.len);
+    if (s >= nseg) return;
+    const int64_t P0 = gbase(in, gb);
+    const int M = in.memory, K = M + 1;
+    const int G = S.max_group, Smax = G * K;
+    const int tid = threadIdx.x, nth = blockDim.x;
+    LinkSeg* const seg = Q.seg + (size_t)v * Q.max_segs;
+    int64_t* const ids = out.ids;
+    auto seg_first = [&](int t) { return w_lo + t * Q.len; };
+    auto seg_end = [&](int t) { return min(w_lo + (t + 1) * Q.len, w_hi); };
+    // the true-state scratch, and that of the speculative run of segment t >= 1
+    uint8_t* const mbase = S.base + (size_t)v * S.bytes_per_video;
+    const Lay ml = make_lay(G, S.max_edges, S.max_points, M, false);
+    const Lay pl = make_lay(G, S.max_edges, Q.points, M, true);
+    auto spec_base = [&](int t) { return Q.base + ((size_t)v * (Q.max_segs - 1) + (t - 1)) * Q.bytes; };
+    int32_t* const m_ring = (int32_t*)(mbase + ml.ring_pt);
+    int32_t* const m_ring_n = (int32_t*)(mbase + ml.ring_n);
+
+    __shared__ LinkRun run;   // in shared memory: the frame loop needs every register
+    __shared__ int sh_lo, sh_hi;
+    // clears the stamps that a run from the true state (in sh and the ring)
+    // over segment t reads before it writes them
+    auto begin_true = [&](int t) {
+        const int g_lo = seg_first(t), g_hi = seg_end(t);
+        if (tid == 0) {
+            sh_lo = g_lo;
+            sh_hi = g_hi;
+            run.base = mbase;
+            run.NP = S.max_points;
+            run.lp0 = 0;
+            run.gfirst = gb;
+            run.own_g = gb;
+            run.flags = out.flags + v;
+            run.c0 = nullptr;
+            run.spec = false;
+        }
+        int32_t* const idstamp = (int32_t*)(mbase + ml.idstamp);
+        int32_t* const srcstamp = (int32_t*)(mbase + ml.srcstamp);
+        unsigned long long* const firstpos = (unsigned long long*)(mbase + ml.firstpos);
+        if (g_hi > g_lo) {
+            const int64_t q0 = gbase(in, max(gb, g_lo - K)) - P0;
+            const int64_t q1 = gbase(in, g_hi - 1) + gsize(in, g_hi - 1) - P0;
+            for (int64_t i = q0 + tid; i < q1; i += nth) srcstamp[i] = -1;
+            const int64_t c = sh.counter, n = frames_points(in, g_lo, g_hi);
+            for (int64_t i = tid; i < n; i += nth) {
+                idstamp[c + i] = -1;
+                firstpos[c + i] = 0ull;
+            }
+            if (sh.prevg == g_lo - 1 && sh.prevg >= gb) {
+                const int64_t pa = gbase(in, sh.prevg), pn = gsize(in, sh.prevg);
+                for (int64_t i = tid; i < pn; i += nth) {
+                    const int64_t id = __ldcg(ids + pa + i);
+                    idstamp[id] = -1;
+                    firstpos[id] = 0ull;
+                }
+            }
+            for (int q = 0; q < M; q++)
+                for (int e = tid; e < sh.ring_n[q]; e += nth) {
+                    const int64_t id = __ldcg(ids + P0 + m_ring[q * G + e]);
+                    idstamp[id] = -1;
+                    firstpos[id] = 0ull;
+                }
+        }
+    };
+    const bool stopped = (*(volatile uint32_t*)(out.flags + v) & kLinkStopFlags) != 0;
+    if (tid == 0) {
+        seg[s].flags = 0;
+        seg[s].c0 = 0;
+        sh.counter = 0;
+        sh.frame = 0;
+        sh.prevg = -1;
+        sh.head = 0;
+        if (s == 0 && !W.first) {
+            const LinkState st = W.state[v];
+            sh.counter = st.counter;
+            sh.prevg = st.prevg;
+            sh.head = st.head;
+        }
+    }
+    for (int i = tid; i <= M; i += nth) sh.ring_n[i] = (s == 0 && !W.first) ? m_ring_n[i] : 0;
+    if (s == 0 && W.first) {
+        int32_t* const vis_d = (int32_t*)(mbase + ml.vis_d);
+        int32_t* const vis_s = (int32_t*)(mbase + ml.vis_s);
+        for (int i = tid; i < Smax; i += nth) vis_s[i] = -1;
+        for (int i = tid; i < G; i += nth) vis_d[i] = -1;
+    }
+    __syncthreads();
+    if (s == 0) {
+        begin_true(0);
+    } else {
+        const int g_lo = max(seg_first(s) - Q.prefix, w_lo), g_hi = seg_end(s);
+        uint8_t* const b = spec_base(s);
+        if (tid == 0) {
+            sh_lo = g_lo;
+            sh_hi = g_hi;
+            run.base = b;
+            run.NP = Q.points;
+            run.lp0 = gbase(in, g_lo) - P0;
+            run.gfirst = g_lo;
+            run.own_g = seg_first(s);
+            run.flags = &seg[s].flags;
+            run.c0 = &seg[s].c0;
+            run.spec = true;
+        }
+        int32_t* const idstamp = (int32_t*)(b + pl.idstamp);
+        int32_t* const srcstamp = (int32_t*)(b + pl.srcstamp);
+        unsigned long long* const firstpos = (unsigned long long*)(b + pl.firstpos);
+        int32_t* const vis_d = (int32_t*)(b + pl.vis_d);
+        int32_t* const vis_s = (int32_t*)(b + pl.vis_s);
+        const int64_t nlp = gbase(in, g_hi - 1) + gsize(in, g_hi - 1) - gbase(in, g_lo);
+        for (int64_t i = tid; i < nlp; i += nth) srcstamp[i] = -1;
+        const int64_t n = frames_points(in, g_lo, g_hi);
+        for (int64_t i = tid; i < n; i += nth) {
+            idstamp[i] = -1;
+            firstpos[i] = 0ull;
+        }
+        for (int i = tid; i < Smax; i += nth) vis_s[i] = -1;
+        for (int i = tid; i < G; i += nth) vis_d[i] = -1;
+    }
+    __syncthreads();
+
+    if (!stopped) link_frames<SF, true>(in, L, S, out, gb, run, sh_lo, sh_hi, sh);
+    __syncthreads();
+    {
+        int32_t* const rn = (int32_t*)(run.base + (run.spec ? pl.ring_n : ml.ring_n));
+        for (int i = tid; i <= M; i += nth) rn[i] = sh.ring_n[i];
+        if (tid == 0) {
+            seg[s].counter = sh.counter;
+            seg[s].head = sh.head;
+            seg[s].final_ids = run.spec ? 0 : 1;
+            seg[s].base = 0;
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        sh_last = atomicAdd(Q.arrived + v, 1u) == (uint32_t)nseg - 1u ? 1 : 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!sh_last) return;
+
+    // ---- the last CTA resolves the boundaries in order
+    if (tid == 0) Q.arrived[v] = 0;
+    int cur = 0;               // last segment whose ids are known
+    bool cur_true = true;      // its run worked in the true-state scratch
+    long long gcount = *(volatile long long*)&seg[0].counter;   // ids given so far
+    for (;;) {
+        if (*(volatile uint32_t*)(out.flags + v) & kLinkStopFlags) return;
+        bool again = false;
+        for (int t = cur + 1; t < nseg && !again; t++) {
+            // compare the end of segment cur = t - 1 with what segment t reached
+            const LinkSeg qc = seg[cur], qt = seg[t];
+            uint8_t* const cb = cur_true ? mbase : spec_base(cur);
+            const int64_t cNP = cur_true ? S.max_points : Q.points;
+            const int32_t* const c_ring = (const int32_t*)(cb + (cur_true ? ml.ring_pt : pl.ring_pt));
+            const int32_t* const c_ring_n = (const int32_t*)(cb + (cur_true ? ml.ring_n : pl.ring_n));
+            // two arrays of ids in the runs' unused start arrays: the final
+            // ids of a run's first ids, and the partner of an id at the
+            // boundary after the run
+            int32_t* const c_gmap = (int32_t*)(cb + (cur_true ? ml.start : pl.start));
+            int32_t* const c_inv = c_gmap + cNP;
+            uint8_t* const tb = spec_base(t);
+            int32_t* const t_gmap = (int32_t*)(tb + pl.start);
+            const int32_t* const t_ring = (const int32_t*)(tb + pl.snap);
+            const int32_t* const t_ring_n = t_ring + M * (int64_t)G;
+            const int64_t* const t_pids = (const int64_t*)(tb + pl.pids);
+            const int ta = seg_first(t);
+            const int64_t t_lp0 = gbase(in, max(ta - Q.prefix, w_lo)) - P0;
+            const int64_t pa = gbase(in, ta - 1) - P0, pn = gsize(in, ta - 1);
+            bool same = qt.flags == 0;
+            for (int q = 0; q < M; q++)
+                if (__ldcg(c_ring_n + (qc.head + q) % M) != __ldcg(t_ring_n + q)) same = false;
+            if (same) {
+                auto pair = [&](int64_t lp, bool check) -> bool {
+                    const int64_t idc = __ldcg(ids + P0 + lp), idt = __ldcg(t_pids + lp - t_lp0);
+                    const int32_t gid = (int32_t)segment_id(qc, c_gmap, idc);
+                    if (check) return __ldcg(t_gmap + idt) == gid && __ldcg(c_inv + idc) == (int32_t)idt;
+                    t_gmap[idt] = gid;
+                    c_inv[idc] = (int32_t)idt;
+                    return true;
+                };
+                for (int pass = 0; pass < 2 && same; pass++) {
+                    bool ok = true;
+                    for (int64_t i = tid; i < pn; i += nth) ok &= pair(pa + i, pass == 1);
+                    for (int q = 0; q < M; q++) {
+                        const int n = __ldcg(t_ring_n + q);
+                        const int32_t* const cr = c_ring + ((qc.head + q) % M) * (int64_t)G;
+                        for (int e = tid; e < n; e += nth) {
+                            const int32_t lp = __ldcg(cr + e);
+                            if (lp != __ldcg(t_ring + q * (int64_t)G + e)) {
+                                ok = false;
+                                break;
+                            }
+                            ok &= pair(lp, pass == 1);
+                        }
+                    }
+                    __threadfence_block();
+                    same = __syncthreads_and(ok) != 0;
+                }
+            }
+            if (same) {
+                if (tid == 0) seg[t].base = gcount;
+                gcount += qt.counter - qt.c0;
+                cur = t;
+                cur_true = false;
+                __syncthreads();
+                continue;
+            }
+            // final ids for all of segment cur, its ring to the true-state
+            // scratch, and segment t once more from there
+            if (!qc.final_ids)
+                for (int g = seg_first(cur); g < ta; g++) {
+                    const int64_t x = gbase(in, g), n = gsize(in, g);
+                    for (int64_t i = x + tid; i < x + n; i += nth) ids[i] = segment_id(qc, c_gmap, __ldcg(ids + i));
+                }
+            if (!cur_true)
+                for (int q = 0; q < M; q++) {
+                    const int n = __ldcg(c_ring_n + q);
+                    for (int e = tid; e < n; e += nth) m_ring[q * G + e] = __ldcg(c_ring + q * (int64_t)G + e);
+                }
+            __syncthreads();
+            for (int i = tid; i <= M; i += nth) sh.ring_n[i] = __ldcg(c_ring_n + i);
+            if (tid == 0) {
+                seg[cur].final_ids = 1;
+                sh.counter = gcount;
+                sh.prevg = ta - 1;
+                sh.head = qc.head;
+            }
+            __syncthreads();
+            begin_true(t);
+            __syncthreads();
+            cur = t;
+            cur_true = true;
+            again = true;
+        }
+        if (!again) break;
+        link_frames<SF, true>(in, L, S, out, gb, run, sh_lo, sh_hi, sh);
+        __syncthreads();
+        gcount = sh.counter;
+        for (int i = tid; i <= M; i += nth) m_ring_n[i] = sh.ring_n[i];
+        if (tid == 0) {
+            seg[cur].head = sh.head;
+            seg[cur].counter = gcount;
+            seg[cur].final_ids = 1;
+        }
+        __syncthreads();
+    }
+    // the state the next window starts from
+    if (!W.last && !cur_true) {
+        const uint8_t* const cb = spec_base(cur);
+        const int32_t* const c_ring = (const int32_t*)(cb + pl.ring_pt);
+        const int32_t* const c_ring_n = (const int32_t*)(cb + pl.ring_n);
+        for (int q = 0; q < M; q++) {
+            const int n = __ldcg(c_ring_n + q);
+            for (int e = tid; e < n; e += nth) m_ring[q * G + e] = __ldcg(c_ring + q * (int64_t)G + e);
+        }
+        for (int i = tid; i <= M; i += nth) m_ring_n[i] = __ldcg(c_ring_n + i);
+    }
+    if (tid == 0) {
+        if (W.last) {
+            out.counter[v] = gcount;
+        } else {
+            LinkState st;
+            st.counter = gcount;
+            st.frame = 0;
+            st.prevg = w_hi - 1;
+            st.head = seg[cur].head;
+            W.state[v] = st;
+        }
+    }
+}
+
+// Final ids of the points of a window whose segments are resolved and, with
+// out.dur_range, the frames their ids were first and last seen in.
+__global__ void segment_ids_kernel(LinkInput in, LinkScratch S, LinkOutput out, LinkWindow W, LinkSegs Q, int64_t p0,
+                                   int64_t p1) {
+    const int64_t p = p0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= p1) return;
+    const int g = ggroup(in, p);
+    if (in.slot_stride && p - gbase(in, g) >= gsize(in, g)) return;  // empty slot
+    int x = 0, y = in.nvideos;
+    while (y - x > 1) {
+        const int m = (x + y) >> 1;
+        if (in.vgrp[m] <= g) x = m; else y = m;
+    }
+    const int v = x;
+    if (out.flags[v] & kLinkStopFlags) return;
+    const int gb = in.vgrp[v];
+    const int w_lo = (W.g0 < 0) ? gb : W.g0;
+    const int t = (g - w_lo) / Q.len;
+    const LinkSeg q = Q.seg[(size_t)v * Q.max_segs + t];
+    int64_t id = out.ids[p];
+    if (!q.final_ids) {
+        const Lay pl = make_lay(S.max_group, S.max_edges, Q.points, in.memory, true);
+        const uint8_t* b = Q.base + ((size_t)v * (Q.max_segs - 1) + (t - 1)) * Q.bytes;
+        id = segment_id(q, (const int32_t*)(b + pl.start), id);
+        out.ids[p] = id;
+    }
+    if (out.dur_range) {
+        int32_t* const r = (int32_t*)(out.dur + gbase(in, gb) + id);
+        atomicMax(r, INT32_MAX - (g - gb));
+        atomicMax(r + 1, g - gb + 1);
+    }
+}
+
+// Duration of an id from its entry: as the sequential linker writes it, or
+// from the first and last frame.
+__device__ __forceinline__ int64_t id_duration(const LinkOutput& out, int64_t at) {
+    if (!out.dur_range) return out.dur[at];
+    const int32_t* const r = (const int32_t*)(out.dur + at);
+    return (int64_t)r[1] - (int64_t)(INT32_MAX - r[0]);
 }
 
 // Per-row durations through the reference's f32 round trip of the particle
@@ -982,12 +1433,12 @@ __global__ void durations_kernel(LinkInput in, LinkOutput out, int64_t* row_dur)
     const int v = x;
     const int64_t P0 = in.goff[in.vgrp[v]];
     const int64_t id = (int64_t)(float)out.ids[p];
-    if (id >= out.counter[v]) {
+    if ((uint64_t)id >= (uint64_t)out.counter[v]) {
         atomicOr(out.flags + v, kFlagScratch);
         row_dur[p] = -1;
         return;
     }
-    row_dur[p] = out.dur[P0 + id];
+    row_dur[p] = id_duration(out, P0 + id);
 }
 
 // Slot mode: the table rows of every point (row_off[g] + j) receive the
@@ -1003,12 +1454,12 @@ __global__ void slot_rows_kernel(LinkInput in, LinkOutput out, const int64_t* __
     const int64_t row = row_off[g] + j;
     const int64_t id = (int64_t)(float)out.ids[p];
     particle[row] = id;
-    if (id >= out.counter[0]) {
+    if ((uint64_t)id >= (uint64_t)out.counter[0]) {
         atomicOr(out.flags, kFlagScratch);
         row_dur[row] = -1;
         return;
     }
-    row_dur[row] = out.dur[id];
+    row_dur[row] = id_duration(out, id);
 }
 
 // --------------------------------------------------------------- launchers
@@ -1079,6 +1530,31 @@ cudaError_t link_run_window(const LinkInput& in, const LinkLists& L, const LinkS
         cudaFuncSetAttribute(link_video_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         link_video_kernel<int64_t><<<in.nvideos, kLinkThreads, bytes, st>>>(in, L, S, out, w);
     }
+    return cudaGetLastError();
+}
+
+size_t link_segment_bytes(int32_t max_group, int64_t max_edges, int64_t npoints, int32_t memory) {
+    return make_lay(max_group, max_edges, npoints, memory, true).total;
+}
+
+cudaError_t link_run_segments(const LinkInput& in, const LinkLists& L, const LinkScratch& S, const LinkOutput& out,
+                              const LinkWindow& w, const LinkSegs& q, int64_t p0, int64_t p1, cudaStream_t st) {
+    if (in.nvideos == 0) return cudaSuccess;
+    if (w.g0 >= 0 && (in.nvideos != 1 || !w.state)) return cudaErrorInvalidValue;
+    if (in.memory > kRingSmem || q.len < in.memory + 2 || q.prefix < 1 || q.max_segs < 1) return cudaErrorInvalidValue;
+    const dim3 grid(q.max_segs, in.nvideos);
+    const int64_t fmax = L.f_cap >= 0 ? L.f_cap : L.f_entries;
+    if (fmax >= 0 && fmax < (int64_t)INT32_MAX) {
+        constexpr size_t bytes = link_smem_bytes<int32_t>();
+        cudaFuncSetAttribute(link_segments_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        link_segments_kernel<int32_t><<<grid, kLinkThreads, bytes, st>>>(in, L, S, out, w, q);
+    } else {
+        constexpr size_t bytes = link_smem_bytes<int64_t>();
+        cudaFuncSetAttribute(link_segments_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        link_segments_kernel<int64_t><<<grid, kLinkThreads, bytes, st>>>(in, L, S, out, w, q);
+    }
+    if (p1 > p0)
+        segment_ids_kernel<<<(unsigned)((p1 - p0 + 255) / 256), 256, 0, st>>>(in, S, out, w, q, p0, p1);
     return cudaGetLastError();
 }
 

@@ -16,6 +16,8 @@ using namespace gt::rt;
 namespace gt {
 namespace rt {
 
+constexpr size_t kLinkSegScratch = (size_t)2 << 30;   // bytes of all speculative runs of a call
+
 // pgroup[i] = g for the points i of group g (goff: group offsets)
 __global__ void fill_pgroup_kernel(const int64_t* __restrict__ goff, int ngroups, int32_t* __restrict__ pgroup) {
     for (int g = blockIdx.x; g < ngroups; g += gridDim.x)
@@ -142,9 +144,43 @@ gt_status run_link(gt_ctx* ctx, const LinkJob& job, const float* px, const float
     out.dur = ctx->l_dur.as<int64_t>();
     out.vpoff = nullptr;
     out.flags = ctx->l_flags.as<uint32_t>();
+    // segments of the frame loop: as many CTAs as there are SMs for the
+    // videos, none shorter than link_segment_min, scratch bounded
+    LinkSegs segs;
+    int max_frames = 0;
+    for (int v = 0; v < nvideos; v++) max_frames = std::max(max_frames, job.vgrp[v + 1] - job.vgrp[v]);
+    if (job.memory <= kLinkSegMemory && std::find(job.reset.begin(), job.reset.end(), 1) == job.reset.end()) {
+        const int per_video = std::max(1, ctx->num_sms / std::max(nvideos, 1));
+        segs.prefix = link_segment_prefix(job.memory);
+        segs.len = std::max(link_segment_min(job.memory), (max_frames + per_video - 1) / per_video);
+        for (;; segs.len *= 2) {
+            segs.max_segs = (max_frames + segs.len - 1) / segs.len;
+            if (segs.max_segs < 2) break;
+            segs.points = 1;
+            for (int v = 0; v < nvideos; v++)
+                for (int a = job.vgrp[v] + segs.len; a < job.vgrp[v + 1]; a += segs.len)
+                    segs.points = std::max(segs.points, job.goff[std::min(a + segs.len, job.vgrp[v + 1])] -
+                                                            job.goff[std::max(a - segs.prefix, job.vgrp[v])]);
+            segs.bytes = link_segment_bytes(S.max_group, S.max_edges, segs.points, job.memory);
+            if (segs.bytes * (size_t)(segs.max_segs - 1) * nvideos <= kLinkSegScratch) break;
+        }
+    }
+    const bool segmented = segs.max_segs >= 2;
+    if (segmented) {
+        CK(ctx->l_segs.ensure(segs.bytes * (size_t)(segs.max_segs - 1) * nvideos));
+        CK(ctx->l_segst.ensure(sizeof(LinkSeg) * (size_t)segs.max_segs * nvideos));
+        CK(ctx->l_segarr.ensure((size_t)nvideos * 4));
+        segs.base = ctx->l_segs.as<uint8_t>();
+        segs.seg = ctx->l_segst.as<LinkSeg>();
+        segs.arrived = ctx->l_segarr.as<uint32_t>();
+        CK(cudaMemsetAsync(segs.arrived, 0, (size_t)nvideos * 4, ctx->st));
+        out.dur_range = row_dur ? 1 : 0;
+        if (row_dur) CK(cudaMemsetAsync(out.dur, 0, (size_t)std::max<int64_t>(N, 1) * 8, ctx->st));
+    }
     {
         Prof pf(ctx, "link_video");
-        CK(link_run(in, L, S, out, ctx->st));
+        if (segmented) CK(link_run_segments(in, L, S, out, LinkWindow(), segs, 0, N, ctx->st));
+        else CK(link_run(in, L, S, out, ctx->st));
     }
     std::vector<uint32_t> flags(nvideos);
     CK(cudaMemcpyAsync(flags.data(), out.flags, nvideos * 4, cudaMemcpyDeviceToHost, ctx->st));

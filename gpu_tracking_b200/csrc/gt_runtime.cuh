@@ -151,6 +151,8 @@ struct gt_ctx {
     int64_t last_walk_starts = 0;
     int32_t illum_rint = 0;
     DBuf w_srt, w_bins, w_scan, w_scratch, w_ids, w_dur, w_state, w_cnt, w_flags, w_vgrp, w_reset;
+    // segments of the linker's frame loop: scratch of the speculative runs, their states, arrivals
+    DBuf w_segs, w_segst, w_segarr, l_segs, l_segst, l_segarr;
     // two sets of window neighbour lists: the lists of window w + 1 are built
     // while the linker reads those of window w
     DBuf w_fcnt[2], w_bcnt[2], w_foff[2], w_boff[2], w_fpts[2], w_bpts[2], w_bdist[2];
