@@ -825,13 +825,48 @@ size_t strip_smem() {
     return StripCfg<T, R, KD>::smem_floats * sizeof(float);
 }
 
+// Rows per segment of a launch of nx strips over nframes frames of H rows.  A
+// tile takes its rows and KD - 1 + 2R halo rows, 8 a step.  A grid of many
+// waves runs segments of at most 512 rows: enough tiles for whole waves, 5 %
+// halo.  A smaller one is cut further while that shortens its longest SM: a
+// step takes about 2.4 us with one or two tiles on an SM, 2.7 us with three
+// and 3.7 us with four (measured at diameter 11, u16), so the cost of a height
+// is that of the rounds of resident tiles an SM gets.  Measured on a B200 with
+// 512 rows a tile and with this rule, bandpass of a whole call: one 512^2 u16
+// frame 168 -> 29 us, one 2048^2 frame 172 -> 69 us, 240 frames of 601 x 803
+// u8 1505 -> 1157 us, 160 frames of 1024^2 f32 2530 -> 2290 us; 512 frames of
+// 2048^2 keep 512 rows (15.3 ms).
+template <int R, int KD>
+int strip_rows(int nx, int H, int nframes, int resident) {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        cudaGetLastError();
+    const int first = (H + 511) / 512;
+    int best = 0;
+    int64_t best_cost = INT64_MAX;
+    for (int n = first; n <= 128; n++) {
+        const int rows = n == 1 ? H : ((H + n - 1) / n + kStepRows - 1) / kStepRows * kStepRows;
+        if (n > first && rows < kStepRows) break;
+        const int64_t tiles = (int64_t)nx * ((H + rows - 1) / rows) * nframes;
+        const int64_t per_sm = (tiles + sms - 1) / sms;
+        const int64_t steps = (rows + KD - 1 + 2 * R + kStepRows - 1) / kStepRows;
+        const int step_cost[5] = {0, 24, 24, 27, 37};
+        const int64_t cost = steps * (per_sm / resident * step_cost[resident] + step_cost[per_sm % resident]);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = rows;
+        }
+    }
+    return best;
+}
+
 template <typename T, int R, int KD, bool FAST>
 cudaError_t strip_launch(const T* frames, int64_t frame_stride, float* processed, const LocateConsts& c, int nframes,
                          uint32_t* cand_count, uint32_t* cand_keys, uint32_t cand_cap, uint32_t* flags,
                          cudaStream_t st) {
-    // row segments of at most 512 rows: enough CTAs for whole waves at 1024 rows and up
-    const int SH = c.H > 512 ? 512 : c.H;
-    dim3 grid((c.W + kStripTW - 1) / kStripTW, (c.H + SH - 1) / SH, nframes);
+    const int nx = (c.W + kStripTW - 1) / kStripTW;
+    const int SH = strip_rows<R, KD>(nx, c.H, nframes, StripCfg<T, R, KD>::min_blocks);
+    dim3 grid(nx, (c.H + SH - 1) / SH, nframes);
     const size_t smem = strip_smem<T, R, KD>();
     // 4-pixel loads need every row start (and the frames) aligned to 4 pixels
     const int vec_ok = (c.W % 4 == 0) && (frame_stride % 4 == 0) &&
