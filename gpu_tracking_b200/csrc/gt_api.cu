@@ -645,6 +645,7 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
     fc.H = H;
     fc.W = W;
     fc.log_style = log_style ? 1 : 0;
+    fc.n_slots = nslots;
     fc.prune = (log_style && p.overlap_threshold < 1.0f) ? 1 : 0;
     fc.overlap_threshold = p.overlap_threshold;
     fc.filter_close = (!log_style && p.filter_close) ? 1 : 0;

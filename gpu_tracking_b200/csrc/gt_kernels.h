@@ -20,6 +20,7 @@ struct FinalizeConsts {
     int32_t filter_close;
     float separation;
     int32_t band;               // candidate-row band holding every filter_close neighbour, -1 = all
+    int32_t n_slots;            // radii (LoG), 0 or 1: one
     int32_t doughnut;
     int32_t presorted;          // characterize_points: rows stay in input order
     uint64_t scratch_per_frame; // bytes of global sort scratch per frame (0 = shared memory only)

@@ -12,6 +12,8 @@
 //   scatter_kernel    per-frame results into the output table columns.
 #include <math.h>
 
+#include <algorithm>
+
 #include "gt_internal.cuh"
 #include "gt_kernels.h"
 
@@ -1128,16 +1130,11 @@ __device__ __forceinline__ float warp_upper_median_regs(const T* __restrict__ ra
             }
         }
     }
-    int nvalid = nv;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nvalid += __shfl_xor_sync(0xffffffffu, nvalid, o);
+    const int nvalid = (int)__reduce_add_sync(0xffffffffu, (unsigned)nv);
     *n_out = nvalid;
     if (nvalid == 0) return 0.0f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        kor |= __shfl_xor_sync(0xffffffffu, kor, o);
-        kand &= __shfl_xor_sync(0xffffffffu, kand, o);
-    }
+    kor = __reduce_or_sync(0xffffffffu, kor);
+    kand = __reduce_and_sync(0xffffffffu, kand);
     const uint32_t diff = kor ^ kand;
     if (diff == 0u) return MedKey<T>::value(kand);
     const uint32_t want = (uint32_t)(nvalid / 2);
@@ -1146,12 +1143,10 @@ __device__ __forceinline__ float warp_upper_median_regs(const T* __restrict__ ra
     if (hb == 31) prefix = 0u;
     for (int bit = hb; bit >= lb; bit--) {
         const uint32_t trial = prefix | (1u << bit);
-        int c = 0;
+        unsigned c = 0;
 #pragma unroll
-        for (int q = 0; q < kMedianRegs; q++) c += (key[q] < trial) ? 1 : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        if ((uint32_t)c <= want) prefix = trial;
+        for (int q = 0; q < kMedianRegs; q++) c += (key[q] < trial) ? 1u : 0u;
+        if (__reduce_add_sync(0xffffffffu, c) <= want) prefix = trial;
     }
     prefix |= kand & ((1u << lb) - 1u);                 // bits below lb: common to all keys
     return MedKey<T>::value(prefix);
@@ -1210,48 +1205,88 @@ __device__ __forceinline__ void doughnut_warp(const T* __restrict__ raw, int H, 
     ft.d_corr = __fsub_rn(sum, __fmul_rn(med, (float)nsig));
 }
 
-// Shared memory of finalize: sort keys, permutation, order, keep flags and
-// a histogram, then the filter_close positions and masses of up to
-// kFinalizeFcSmem detections.
+// Shared memory of finalize: sort keys, permutation, order and keep flags of
+// up to kFinalizeSmemSort detections, the bins of its counting sorts, and 14
+// bytes more a detection for up to kFinalizeFcSmem of them (prune: position,
+// radius and bin order) or 6 for all (filter_close: mass and canonical index).
 constexpr int kFinalizeFcSmem = 4096;
+constexpr int kFinalizeBins = 4096;
+constexpr int kFinalizeBinMax = 32;   // a fuller bin sends the order to the bitonic sort
 __host__ __device__ constexpr size_t finalize_smem_core_bytes() {
-    return (size_t)kFinalizeSmemSort * (8 + 4 + 4 + 1) + 32 * 256 * sizeof(uint32_t);
+    return (size_t)kFinalizeSmemSort * (8 + 4 + 4 + 1) + kFinalizeBins * sizeof(int32_t);
 }
 
-// One CTA per frame: canonical order, filter_close / prune_blobs_log, the
-// doughnut correction and compaction of the kept rows in output order.
-template <typename T>
+// Exclusive scan of the bin counts in place by the whole block; returns the
+// largest count (every thread).
+__device__ __forceinline__ int scan_bins(int32_t* bins, int* wsum, int* smax) {
+    static_assert(kFinalizeBins == 4 * kFinalizeThreads, "four bins a thread");
+    int4* const b4 = (int4*)bins;
+    int4 c = b4[threadIdx.x];
+    const int s = c.x + c.y + c.z + c.w;
+    if (threadIdx.x == 0) *smax = 0;
+    int tot;
+    const int base = block_excl_scan(s, &tot, wsum);   // its barriers order *smax
+    const int m = __reduce_max_sync(0xffffffffu, max(max(c.x, c.y), max(c.z, c.w)));
+    if ((threadIdx.x & 31) == 0) atomicMax(smax, m);
+    int4 o;
+    o.x = base;
+    o.y = o.x + c.x;
+    o.z = o.y + c.y;
+    o.w = o.z + c.z;
+    b4[threadIdx.x] = o;
+    __syncthreads();
+    return *smax;
+}
+
+// One CTA per frame: canonical order, filter_close / prune_blobs_log and
+// compaction of the kept rows in output order.  Latency of one CTA bounds it,
+// so every step is a few passes over the detections instead of a sorting
+// network or a scan of a whole band of rows: the canonical order is a counting
+// sort over bins of candidate pixels (ranks inside a bin by comparison),
+// filter_close bins the positions by row and looks at the rows within the
+// separation, prune settles all blobs in rounds, and the kept records move in
+// 16-byte pieces.  With the doughnut (median counts by warp reductions, few
+// frames spread over more CTAs), against a bitonic sort, bands of candidate
+// rows, one prune step per kept blob and records copied by a thread each
+// (B200, us a call): one frame of 1965 detections 172 -> 43, 512 frames of
+// them 1968 -> 1628, 64 frames of 4419 learned seeds 1616 -> 424, 64 frames
+// of 1075 LoG blobs 557 -> 258.
 __global__ void __launch_bounds__(kFinalizeThreads)
 finalize_kernel(const Feature* __restrict__ feats, const uint32_t* __restrict__ feat_count, uint32_t feat_cap,
                 Feature* __restrict__ out, uint32_t* __restrict__ kept_count, uint8_t* __restrict__ gscratch,
-                const FinalizeConsts fc, const T* __restrict__ frames, int64_t frame_stride,
-                const int32_t* __restrict__ frame_index, const short2* __restrict__ dn_inds,
-                const int4* __restrict__ dn_meta, uint32_t* __restrict__ flags, const RaggedFrame* __restrict__ rf) {
+                const FinalizeConsts fc, uint32_t* __restrict__ flags, const RaggedFrame* __restrict__ rf) {
     extern __shared__ uint64_t fsm[];
     __shared__ int wsum[33];
+    __shared__ int s_max;
     const int g = blockIdx.x;
-    const int fW = rf ? rf[g].W : fc.W;
+    const int fH = rf ? rf[g].H : fc.H, fW = rf ? rf[g].W : fc.W;
     const int og = rf ? rf[g].out_slot : g;   // result slot (ragged batches: the frame's slot of the call)
     const int n = (int)min(feat_count[g], feat_cap);
     const Feature* F = feats + (size_t)g * feat_cap;
+    const int tid = threadIdx.x;
+    if (n == 0) {
+        if (tid == 0) kept_count[og] = 0;
+        return;
+    }
     int np2 = 1;
     while (np2 < n) np2 <<= 1;
     // working arrays: keys (u64), perm (i32), order (i32), keep (u8)
     uint64_t* keys;
     int32_t *perm, *order;
     uint8_t* keep;
-    uint32_t* hist;
     const size_t need = (size_t)np2 * (8 + 4 + 4 + 1);
-    if (np2 <= kFinalizeSmemSort) {
+    const bool in_smem = np2 <= kFinalizeSmemSort;
+    int32_t* const bins = (int32_t*)((uint8_t*)fsm + (size_t)kFinalizeSmemSort * (8 + 4 + 4 + 1));
+    uint8_t* const extra = (uint8_t*)fsm + finalize_smem_core_bytes();
+    if (in_smem) {
         keys = fsm;
         perm = (int32_t*)(keys + kFinalizeSmemSort);
         order = perm + kFinalizeSmemSort;
         keep = (uint8_t*)(order + kFinalizeSmemSort);
-        hist = (uint32_t*)(keep + kFinalizeSmemSort);
     } else {
         if (need > fc.scratch_per_frame) {
-            if (threadIdx.x == 0) atomicOr(flags, kFlagFeatOverflow);
-            if (threadIdx.x == 0) kept_count[og] = 0;
+            if (tid == 0) atomicOr(flags, kFlagFeatOverflow);
+            if (tid == 0) kept_count[og] = 0;
             return;
         }
         uint8_t* base = gscratch + (size_t)g * fc.scratch_per_frame;
@@ -1259,47 +1294,108 @@ finalize_kernel(const Feature* __restrict__ feats, const uint32_t* __restrict__ 
         perm = (int32_t*)(keys + np2);
         order = perm + np2;
         keep = (uint8_t*)(order + np2);
-        uint8_t* sm_after = (uint8_t*)fsm;
-        hist = (uint32_t*)sm_after;
     }
     // 1. canonical order: (radius index, candidate pixel index), or input order
-    for (int i = threadIdx.x; i < np2; i += blockDim.x) {
-        if (i < n) {
-            const Feature& ft = F[i];
-            keys[i] = fc.presorted ? (uint64_t)i
-                                   : (((uint64_t)ft.key_hi << 56) | ((uint64_t)ft.key_lo << 24) | (uint64_t)i);
-        } else {
-            keys[i] = ~0ull;
-        }
-    }
-    __syncthreads();
-    if (!fc.presorted) block_sort_u64(keys, np2);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        perm[i] = (int32_t)(keys[i] & 0xFFFFFFull);
+    auto sort_key = [&](int i) -> uint64_t {
+        const uint2 k = *(const uint2*)&F[i].key_hi;
+        return ((uint64_t)k.x << 56) | ((uint64_t)k.y << 24) | (uint64_t)i;
+    };
+    for (int i = tid; i < n; i += blockDim.x) {
+        if (fc.presorted) perm[i] = i;
         keep[i] = 1;
         order[i] = i;
     }
-    __syncthreads();
-
-    if (!fc.log_style) {
-        // 2a. filter_close_trackpy (src/execute_gpu.rs:556-590) in canonical order
-        if (fc.filter_close) {
-            // positions and masses in canonical order, in shared memory when
-            // they fit: the neighbour scans then read no global memory
-            const bool fc_smem = np2 <= kFinalizeSmemSort && n <= kFinalizeFcSmem;
-            float* const fcx = (float*)((uint8_t*)fsm + finalize_smem_core_bytes());
-            float* const fcy = fcx + kFinalizeFcSmem;
-            float* const fcm = fcy + kFinalizeFcSmem;
-            if (fc_smem) {
-                for (int i = threadIdx.x; i < n; i += blockDim.x) {
-                    const Feature& ft = F[perm[i]];
-                    fcx[i] = ft.x;
-                    fcy[i] = ft.y;
-                    fcm[i] = ft.mass;
-                }
-                __syncthreads();
+    bool sorted = fc.presorted != 0;
+    if (!sorted && in_smem) {
+        // bins of equal shares of (radius, pixel): monotone in the key
+        const uint64_t npx = (uint64_t)fH * fW;
+        const uint64_t span = npx * (uint64_t)max(fc.n_slots, 1);   // a frame with detections has pixels
+        const uint64_t mul = ((uint64_t)kFinalizeBins << 32) / span;   // bin < kFinalizeBins for keys < span
+        auto key_bin = [&](uint64_t key) -> int {
+            const uint64_t v = (key >> 56) * npx + ((key >> 24) & 0xFFFFFFFFull);
+            return (int)min((uint64_t)(kFinalizeBins - 1), (v * mul) >> 32);   // v * mul <= 2^44
+        };
+        for (int i = tid; i < kFinalizeBins; i += blockDim.x) bins[i] = 0;
+        __syncthreads();
+        for (int i = tid; i < n; i += blockDim.x) atomicAdd(bins + key_bin(sort_key(i)), 1);
+        __syncthreads();
+        if (scan_bins(bins, wsum, &s_max) <= kFinalizeBinMax) {
+            for (int i = tid; i < n; i += blockDim.x) {
+                const uint64_t k = sort_key(i);
+                keys[atomicAdd(bins + key_bin(k), 1)] = k;
             }
-            for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            __syncthreads();
+            // bins[b] is now the end of bin b
+            for (int p = tid; p < n; p += blockDim.x) {
+                const uint64_t k = keys[p];
+                const int b = key_bin(k);
+                const int s0 = b ? bins[b - 1] : 0, s1 = bins[b];
+                int rank = s0;
+                for (int q = s0; q < s1; q++) rank += keys[q] < k ? 1 : 0;
+                perm[rank] = (int32_t)(k & 0xFFFFFFull);
+            }
+            sorted = true;
+        }
+    }
+    __syncthreads();
+    if (!sorted) {
+        for (int i = tid; i < np2; i += blockDim.x) keys[i] = i < n ? sort_key(i) : ~0ull;
+        __syncthreads();
+        block_sort_u64(keys, np2);
+        for (int i = tid; i < n; i += blockDim.x) perm[i] = (int32_t)(keys[i] & 0xFFFFFFull);
+        __syncthreads();
+    }
+
+    // bins of rows of a position, monotone in it (NaN: bin 0)
+    const float per_row = (float)kFinalizeBins / (float)fH;
+    auto row_bin = [&](float x) -> int {
+        const float t = __fmul_rn(x, per_row);
+        return t >= (float)(kFinalizeBins - 1) ? kFinalizeBins - 1 : (t > 0.0f ? (int)t : 0);
+    };
+    if (!fc.log_style) {
+        // 2a. filter_close_trackpy (src/execute_gpu.rs:556-590): a row goes when a
+        // row within the separation has more mass, or as much and an earlier
+        // place in canonical order
+        if (fc.filter_close && in_smem) {
+            // positions in order of their row's bin: a neighbour's row lies
+            // between those of the row minus and plus the separation (the box
+            // test of within_rd2), and the bin is monotone in the row
+            float2* const pos = (float2*)fsm;               // keys are done with
+            float* const mass = (float*)extra;
+            uint16_t* const idx = (uint16_t*)(mass + kFinalizeSmemSort);
+            for (int i = tid; i < kFinalizeBins; i += blockDim.x) bins[i] = 0;
+            __syncthreads();
+            for (int i = tid; i < n; i += blockDim.x) atomicAdd(bins + row_bin(F[perm[i]].x), 1);
+            __syncthreads();
+            scan_bins(bins, wsum, &s_max);
+            for (int i = tid; i < n; i += blockDim.x) {
+                const Feature& ft = F[perm[i]];
+                const float x = ft.x;
+                const int p = atomicAdd(bins + row_bin(x), 1);
+                pos[p] = make_float2(x, ft.y);
+                mass[p] = ft.mass;
+                idx[p] = (uint16_t)i;
+            }
+            __syncthreads();
+            for (int p = tid; p < n; p += blockDim.x) {
+                const float2 q = pos[p];
+                const float qm = mass[p];
+                const int qi = idx[p];
+                const int b0 = row_bin(__fsub_rn(q.x, fc.separation)), b1 = row_bin(__fadd_rn(q.x, fc.separation));
+                bool kp = true;
+                for (int j = b0 ? bins[b0 - 1] : 0, hi = bins[b1]; j < hi && kp; j++) {
+                    if (j == p) continue;
+                    const float2 nb = pos[j];
+                    float dist;
+                    if (!within_rd2(nb.x, nb.y, q.x, q.y, fc.separation, &dist)) continue;
+                    if (qm < mass[j]) kp = false;
+                    else if (qm == mass[j] && qi > (int)idx[j]) kp = false;
+                }
+                keep[qi] = kp ? 1 : 0;
+            }
+            __syncthreads();
+        } else if (fc.filter_close) {
+            for (int i = tid; i < n; i += blockDim.x) {
                 const Feature& q = F[perm[i]];
                 int lo = 0, hi = n;
                 if (fc.band >= 0) {
@@ -1316,24 +1412,13 @@ finalize_kernel(const Feature* __restrict__ feats, const uint32_t* __restrict__ 
                     hi = a;
                 }
                 bool kp = true;
-                if (fc_smem) {
-                    const float qx = fcx[i], qy = fcy[i], qm = fcm[i];
-                    for (int j = lo; j < hi && kp; j++) {
-                        if (j == i) continue;
-                        float dist;
-                        if (!within_rd2(fcx[j], fcy[j], qx, qy, fc.separation, &dist)) continue;
-                        if (qm < fcm[j]) kp = false;
-                        else if (qm == fcm[j] && i > j) kp = false;
-                    }
-                } else {
-                    for (int j = lo; j < hi && kp; j++) {
-                        if (j == i) continue;
-                        const Feature& nb = F[perm[j]];
-                        float dist;
-                        if (!within_rd2(nb.x, nb.y, q.x, q.y, fc.separation, &dist)) continue;
-                        if (q.mass < nb.mass) kp = false;
-                        else if (q.mass == nb.mass && i > j) kp = false;
-                    }
+                for (int j = lo; j < hi && kp; j++) {
+                    if (j == i) continue;
+                    const Feature& nb = F[perm[j]];
+                    float dist;
+                    if (!within_rd2(nb.x, nb.y, q.x, q.y, fc.separation, &dist)) continue;
+                    if (q.mass < nb.mass) kp = false;
+                    else if (q.mass == nb.mass && i > j) kp = false;
                 }
                 keep[i] = kp ? 1 : 0;
             }
@@ -1341,7 +1426,7 @@ finalize_kernel(const Feature* __restrict__ feats, const uint32_t* __restrict__ 
         }
     } else if (fc.prune) {
         // 2b. sort by (r desc, mass desc), stable w.r.t. the canonical order
-        for (int i = threadIdx.x; i < np2; i += blockDim.x) {
+        for (int i = tid; i < np2; i += blockDim.x) {
             if (i < n) {
                 const Feature& ft = F[perm[i]];
                 uint64_t rk = (uint64_t)fc.radius_rank_desc[ft.ridx];
@@ -1352,44 +1437,140 @@ finalize_kernel(const Feature* __restrict__ feats, const uint32_t* __restrict__ 
             }
         }
         __syncthreads();
-        block_sort_u64(keys, np2);
-        for (int i = threadIdx.x; i < n; i += blockDim.x) order[i] = (int32_t)(keys[i] & 0xFFFFFFull);
+        if (n <= 2048 && in_smem) {
+            // up to two detections a thread: ranks by comparison with all of
+            // them (one shared word a step for the whole warp)
+            for (int i = tid; i < n; i += blockDim.x) {
+                const uint64_t k = keys[i];
+                int rank = 0;
+#pragma unroll 4
+                for (int q = 0; q < n; q++) rank += keys[q] < k ? 1 : 0;
+                order[rank] = i;
+            }
+        } else {
+            block_sort_u64(keys, np2);
+            for (int i = tid; i < n; i += blockDim.x) order[i] = (int32_t)(keys[i] & 0xFFFFFFull);
+        }
         __syncthreads();
         // prune_blobs_log (src/execute_gpu.rs:592-669): greedy in priority
-        // order, one step per kept blob.  Positions and radii in priority
-        // order sit in shared memory when they fit, so a step's scan reads no
-        // global memory.
-        const bool pr_smem = np2 <= kFinalizeSmemSort && n <= kFinalizeFcSmem;
+        // order; a blob whose turn comes while it is still there drops every
+        // other blob that it overlaps.  Positions and radii in priority
+        // order sit in shared memory when they fit.
+        const bool pr_smem = in_smem && n <= kFinalizeFcSmem;
         if (pr_smem) {
-            float* const bx = (float*)((uint8_t*)fsm + finalize_smem_core_bytes());
+            float* const bx = (float*)extra;
             float* const by = bx + kFinalizeFcSmem;
             float* const br = by + kFinalizeFcSmem;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            uint16_t* const slot = (uint16_t*)(br + kFinalizeFcSmem);
+            for (int i = tid; i < kFinalizeBins; i += blockDim.x) bins[i] = 0;
+            __syncthreads();
+            for (int i = tid; i < n; i += blockDim.x) {
                 const Feature& ft = F[perm[order[i]]];
                 bx[i] = ft.x;
                 by[i] = ft.y;
                 br[i] = ft.r;
+                atomicAdd(bins + row_bin(ft.x), 1);
             }
             __syncthreads();
-            for (int q = 0; q < n; q++) {
-                if (!keep[q]) continue;  // uniform: keep[] only changes between barriers
-                const float Qx = bx[q], Qy = by[q], Qr = br[q];
-                const float qr = __fmul_rn(Qr, 2.0f);
-                for (int j = threadIdx.x; j < n; j += blockDim.x) {
-                    if (j == q || !keep[j]) continue;
+            scan_bins(bins, wsum, &s_max);
+            for (int i = tid; i < n; i += blockDim.x) slot[atomicAdd(bins + row_bin(bx[i]), 1)] = (uint16_t)i;
+            __syncthreads();
+            // Rounds instead of one step per blob: for every blob the others
+            // that would drop it; a blob has its turn once all such blobs of
+            // higher priority are settled and none of them had one.  The
+            // lists (keys are done with) hold `cap` blobs each.
+            uint16_t* const list = (uint16_t*)fsm;
+            const int cap = min(64, (int)(kFinalizeSmemSort * 4 / max(n, 1)));
+            uint8_t* const state = keep;                    // 0 open, 1 had its turn, 2 did not
+            uint8_t* const count = keep + kFinalizeFcSmem;
+            bool over = false;
+            for (int j = tid; j < n; j += blockDim.x) {
+                const float x = bx[j], y = by[j], r = br[j];
+                // twice the largest radius reaches every blob that could drop
+                // this one, a pixel and a share of the row for rounding
+                const float reach = 2.0f * br[0] + 1.0f + fabsf(x) * (1.0f / 1048576.0f);
+                const int b0 = row_bin(x - reach), b1 = row_bin(x + reach);
+                int c = 0;
+                for (int e = b0 ? bins[b0 - 1] : 0, hi = bins[b1]; e < hi; e++) {
+                    const int q = slot[e];
+                    const float Qr = br[q];
                     float d2;
-                    if (!within_rd2(bx[j], by[j], Qx, Qy, qr, &d2)) continue;
-                    float ov = blob_overlap(Qr, br[j], __fsqrt_rn(d2));
-                    if (ov > fc.overlap_threshold) keep[j] = 0;
+                    if (!within_rd2(x, y, bx[q], by[q], __fmul_rn(Qr, 2.0f), &d2) || q == j) continue;
+                    if (!(blob_overlap(Qr, r, __fsqrt_rn(d2)) > fc.overlap_threshold)) continue;
+                    if (c < cap) list[j * cap + c] = (uint16_t)q;
+                    c++;
+                }
+                over |= c > cap;
+                count[j] = (uint8_t)min(c, cap);
+                state[j] = 0;
+            }
+            if (!__syncthreads_or(over)) {
+                bool open = true;
+                while (open) {
+                    open = false;
+                    uint8_t now[kFinalizeFcSmem / kFinalizeThreads];
+#pragma unroll
+                    for (int k = 0; k < kFinalizeFcSmem / kFinalizeThreads; k++) {
+                        const int j = tid + k * kFinalizeThreads;
+                        now[k] = 0;
+                        if (j >= n || state[j]) continue;
+                        uint8_t v = 1;
+                        for (int e = 0; e < (int)count[j]; e++) {
+                            const int q = list[j * cap + e];
+                            if (q > j) continue;
+                            if (state[q] == 1) {
+                                v = 2;
+                                break;
+                            }
+                            if (state[q] == 0) v = 0;
+                        }
+                        now[k] = v;
+                        open |= v == 0;
+                    }
+                    __syncthreads();
+#pragma unroll
+                    for (int k = 0; k < kFinalizeFcSmem / kFinalizeThreads; k++)
+                        if (now[k]) state[tid + k * kFinalizeThreads] = now[k];
+                    open = __syncthreads_or(open) != 0;
+                }
+                // a blob that had its turn stays unless a later one drops it
+                for (int j = tid; j < n; j += blockDim.x) {
+                    bool kp = state[j] == 1;
+                    for (int e = 0; kp && e < (int)count[j]; e++) {
+                        const int q = list[j * cap + e];
+                        if (q > j && state[q] == 1) kp = false;
+                    }
+                    order[j] |= kp ? 0 : INT32_MIN;   // keep[] still holds the turns
                 }
                 __syncthreads();
+                for (int j = tid; j < n; j += blockDim.x) {
+                    keep[j] = order[j] >= 0 ? 1 : 0;
+                    order[j] &= INT32_MAX;
+                }
+                __syncthreads();
+            } else {
+                for (int j = tid; j < n; j += blockDim.x) keep[j] = 1;
+                __syncthreads();
+                for (int q = 0; q < n; q++) {
+                    if (!keep[q]) continue;  // uniform: keep[] only changes between barriers
+                    const float Qx = bx[q], Qy = by[q], Qr = br[q];
+                    const float qr = __fmul_rn(Qr, 2.0f);
+                    for (int j = tid; j < n; j += blockDim.x) {
+                        if (j == q || !keep[j]) continue;
+                        float d2;
+                        if (!within_rd2(bx[j], by[j], Qx, Qy, qr, &d2)) continue;
+                        float ov = blob_overlap(Qr, br[j], __fsqrt_rn(d2));
+                        if (ov > fc.overlap_threshold) keep[j] = 0;
+                    }
+                    __syncthreads();
+                }
             }
         } else {
             for (int q = 0; q < n; q++) {
                 if (!keep[q]) continue;  // uniform: keep[] only changes between barriers
                 const Feature& Q = F[perm[order[q]]];
                 const float qr = __fmul_rn(Q.r, 2.0f);
-                for (int j = threadIdx.x; j < n; j += blockDim.x) {
+                for (int j = tid; j < n; j += blockDim.x) {
                     if (j == q || !keep[j]) continue;
                     const Feature& Nb = F[perm[order[j]]];
                     float d2;
@@ -1402,30 +1583,34 @@ finalize_kernel(const Feature* __restrict__ feats, const uint32_t* __restrict__ 
         }
     }
 
-    // 3. doughnut correction of the kept rows, one warp per row
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    // 4. compaction in output order
+    // 3. the kept rows in output order: their places first, then the 64-byte
+    // records four lanes each
     int total = 0;
     for (int base = 0; base < n; base += blockDim.x) {
-        int i = base + threadIdx.x;
-        int k = (i < n) ? keep[i] : 0;
+        const int i = base + tid;
+        const int k = (i < n) ? keep[i] : 0;
+        const int src = (i < n) ? perm[order[i]] : 0;
         int tot;
-        int pos = block_excl_scan(k, &tot, wsum);
-        if (k) {
-            Feature ft = F[perm[order[i]]];
-            out[(size_t)og * feat_cap + total + pos] = ft;
-        }
+        const int p = block_excl_scan(k, &tot, wsum);   // its barriers end the reads above
+        if (k) keys[total + p] = (uint64_t)src;
         total += tot;
-        __syncthreads();
     }
-    if (threadIdx.x == 0) kept_count[og] = (uint32_t)total;
+    __syncthreads();
+    const uint4* const src4 = (const uint4*)F;
+    uint4* const dst4 = (uint4*)(out + (size_t)og * feat_cap);
+    static_assert(sizeof(Feature) == 4 * sizeof(uint4), "a record is four 16-byte pieces");
+    for (int e = tid; e < 4 * total; e += blockDim.x) dst4[e] = src4[4 * (size_t)keys[e >> 2] + (e & 3)];
+    if (tid == 0) kept_count[og] = (uint32_t)total;
 }
 
 // Doughnut correction of the kept rows (src/execute_gpu.rs:717-790): one warp
 // per row, kDoughnutBlocks x 8 warps per frame walking the frame's rows, so the
 // per-row latency (gathers, median bits) overlaps across the whole GPU.
 constexpr int kDoughnutWarps = 8;
-constexpr int kDoughnutBlocks = 16;
+// CTAs per frame: 16 fill the GPU at 64 frames and more; fewer frames are
+// spread wider, down to one row a warp (a frame's rows are a chain of gathers
+// and counts of some microseconds each).
+constexpr int kDoughnutBlocks = 16, kDoughnutMaxBlocks = 256, kDoughnutTarget = 2048;
 template <typename T>
 __global__ void __launch_bounds__(32 * kDoughnutWarps)
 doughnut_kernel(Feature* __restrict__ out, const uint32_t* __restrict__ kept_count, uint32_t feat_cap,
@@ -1488,7 +1673,7 @@ size_t bandpass_smem_bytes(int R, int kd, bool cand) {
     return fl * sizeof(float);
 }
 
-size_t finalize_smem_bytes() { return finalize_smem_core_bytes() + (size_t)kFinalizeFcSmem * 3 * sizeof(float); }
+size_t finalize_smem_bytes() { return finalize_smem_core_bytes() + (size_t)kFinalizeFcSmem * (3 * sizeof(float) + sizeof(uint16_t)); }
 
 template <typename T>
 cudaError_t launch_bandpass(const T* frames, int64_t frame_stride, float* processed, const LocateConsts& c,
@@ -1596,12 +1781,12 @@ cudaError_t launch_finalize(const Feature* feats, const uint32_t* feat_count, ui
                             const int4* dn_meta, uint32_t* flags, int ngroups, cudaStream_t st,
                             const RaggedFrame* rf) {
     size_t smem = finalize_smem_bytes();
-    cudaFuncSetAttribute(finalize_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    finalize_kernel<T><<<ngroups, kFinalizeThreads, smem, st>>>(feats, feat_count, feat_cap, out, kept_count,
-                                                                gscratch, fc, frames, frame_stride, frame_index,
-                                                                dn_inds, dn_meta, flags, rf);
+    cudaFuncSetAttribute(finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    finalize_kernel<<<ngroups, kFinalizeThreads, smem, st>>>(feats, feat_count, feat_cap, out, kept_count, gscratch,
+                                                             fc, flags, rf);
     if (fc.doughnut && ngroups > 0) {
-        dim3 grid(kDoughnutBlocks, ngroups);
+        const int want = std::min(kDoughnutMaxBlocks, std::max(kDoughnutBlocks, kDoughnutTarget / ngroups));
+        dim3 grid(std::min<unsigned>(want, (feat_cap + kDoughnutWarps - 1) / kDoughnutWarps), ngroups);
         doughnut_kernel<T><<<grid, 32 * kDoughnutWarps, 0, st>>>(out, kept_count, feat_cap, fc, frames,
                                                                   frame_stride, frame_index, dn_inds, dn_meta, rf);
     }
