@@ -102,7 +102,10 @@ class _Frames:
         self.T, self.H, self.W = t.shape
 
 
-def _run(ctx, fn, show_progress):
+_SHORT_PIXELS = 1 << 23   # locating these takes about a millisecond
+
+
+def _run(ctx, fn, show_progress, short=False):
     """Run a blocking library call on a worker thread; Ctrl-C interrupts it
     cooperatively (the reference's ScopedProgressFuture, macros lib.rs:75-129)."""
     result = {}
@@ -111,6 +114,10 @@ def _run(ctx, fn, show_progress):
         result["status"] = fn()
 
     ctx.interrupt(False)
+    if short and not show_progress:
+        # a call of a few milliseconds ends before an interrupt could be
+        # passed on; a thread would cost as much as the call
+        return fn()
     th = threading.Thread(target=work, daemon=True)
     th.start()
     bar = None
@@ -146,16 +153,22 @@ def _table_to_frame(ctx, handle, params, has_r=None):
         if has_r is not None and not has_r:
             cols = [c for c in cols if c[0] != "r"]
         # the DataFrame's own dtypes (int64 / float64) filled by one library
-        # call; the frame takes the arrays as they are, without a copy
-        data = {name: np.empty(n, np.int64 if ty == "int" else np.float64) for name, ty in cols}
+        # call, column after column in one block of host memory; the frame
+        # takes the columns as they are, without a copy
+        block = _ffi.results.take(8 * n * len(cols))
+        columns = np.asarray(block)[:8 * n * len(cols)].reshape(len(cols), 8 * n)
         if n and cols:
             idx = (ctypes.c_int32 * len(cols))(*[COLUMN_INDEX[name] for name, _ in cols])
-            ptrs = (ctypes.c_void_p * len(cols))(*[data[name].ctypes.data for name, _ in cols])
-            ctx.check(L.gt_table_export(handle, idx, len(cols), ptrs))
+            if block.pinned:
+                ctx.check(L.gt_table_export_pinned(handle, idx, len(cols), block.address))
+            else:
+                ptrs = (ctypes.c_void_p * len(cols))(*[block.address + 8 * n * k for k in range(len(cols))])
+                ctx.check(L.gt_table_export(handle, idx, len(cols), ptrs))
     finally:
         L.gt_table_free(handle)
+    data = {name: columns[k].view(np.int64 if ty == "int" else np.float64) for k, (name, ty) in enumerate(cols)}
     pd = _pandas()
-    return pd.DataFrame(data, columns=[c[0] for c in cols], copy=False)
+    return pd.DataFrame(data, index=pd.RangeIndex(n), copy=False)
 
 
 def _locate(video, params, kw):
@@ -175,7 +188,7 @@ def _locate(video, params, kw):
                                    reset_arr.ctypes.data_as(P64) if len(reset_arr) else None, len(reset_arr),
                                    ctypes.byref(out))
 
-    st = _run(ctx, call, bool(kw.get("tqdm", True)) and fr.T > 1)
+    st = _run(ctx, call, bool(kw.get("tqdm", True)) and fr.T > 1, fr.T * fr.H * fr.W <= _SHORT_PIXELS)
     ctx.check(st)
     return _table_to_frame(ctx, out, params)
 
@@ -295,7 +308,7 @@ def characterize_points(file_or_array, points_to_characterize, diameter=None, **
                                                  fr.W, pts.ctypes.data_as(ctypes.POINTER(ctypes.c_float)),
                                                  len(pts), int(has_frames), int(has_r), ctypes.byref(out))
 
-    ctx.check(_run(ctx, call, bool(kwargs.get("tqdm", True)) and fr.T > 1))
+    ctx.check(_run(ctx, call, bool(kwargs.get("tqdm", True)) and fr.T > 1, fr.T * fr.H * fr.W <= _SHORT_PIXELS))
     return _table_to_frame(ctx, out, params)
 
 
@@ -310,7 +323,7 @@ def link(to_link, search_range, memory=0):
     if arr.ndim != 2 or arr.shape[1] != 3:
         raise ValueError("link expects (N, 3) rows of frame, y, x")
     ctx = _ffi.context(_DEVICE)
-    ids = np.empty(len(arr), np.int64)
+    ids = np.asarray(_ffi.results.take(8 * len(arr)))[:8 * len(arr)].view(np.int64)
     ctx.check(_ffi.lib().gt_link(ctx.handle, arr.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), len(arr),
                                  float(search_range), int(memory or 0),
                                  ids.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))))

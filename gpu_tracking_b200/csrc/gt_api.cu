@@ -721,11 +721,12 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
         int64_t f0 = (int64_t)sc * SC;
         int nf = (int)std::min<int64_t>(SC, NT - f0);
         CK(cudaStreamWaitEvent(ctx->cp, ctx->used[b], 0));
-        CK(cudaMemcpyAsync(ctx->stage[b].p, frames + f0 * npx, (size_t)nf * npx * sizeof(T), cudaMemcpyHostToDevice,
-                           ctx->cp));
+        CK(upload_host(ctx->device, ctx->stage[b].p, frames + f0 * npx, (size_t)nf * npx * sizeof(T), ctx->cp));
         CK(cudaEventRecord(ctx->filled[b], ctx->cp));
         return GT_OK;
     };
+    // a copy that keeps the host busy is issued after the launches that it runs beside
+    const bool late_copy = !on_device && upload_blocks(frames, super_bytes);
     if (!on_device) {
         // both staging buffers start free
         CK(cudaEventRecord(ctx->used[0], ctx->st));
@@ -747,7 +748,7 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
         if (on_device) {
             sbase = frames + s0 * npx;
         } else {
-            if (sc + 1 < nsuper) CKS(issue_copy(sc + 1));
+            if (sc + 1 < nsuper && !late_copy) CKS(issue_copy(sc + 1));
             CK(cudaStreamWaitEvent(ctx->st, ctx->filled[sc & 1], 0));
             sbase = ctx->stage[sc & 1].as<T>();
         }
@@ -899,6 +900,7 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
         }
         if (!on_device) CK(cudaEventRecord(ctx->used[sc & 1], ctx->st));
         if (pl) CKS(pl->window((int)s0, (int)(s0 + ns), sc == 0, sc == nsuper - 1));
+        if (late_copy && sc + 1 < nsuper) CKS(issue_copy(sc + 1));
         ctx->done = s0 + ns;
     }
     CK(cudaMemcpyAsync(out_flags, flags, 4, cudaMemcpyDeviceToHost, ctx->st));

@@ -24,6 +24,15 @@ __global__ void fill_pgroup_kernel(const int64_t* __restrict__ goff, int ngroups
         for (int64_t i = goff[g] + threadIdx.x; i < goff[g + 1]; i += blockDim.x) pgroup[i] = g;
 }
 
+// rows of (frame, y, x) -> columns of y and x
+__global__ void split_rows_kernel(const float* __restrict__ rows, int64_t n, float* __restrict__ py,
+                                  float* __restrict__ px) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    py[i] = rows[3 * i + 1];
+    px[i] = rows[3 * i + 2];
+}
+
 // out[g] = boff[goff[g] * K], g = 0..ngroups: where each group's backward lists start
 __global__ void group_list_starts_kernel(const int64_t* __restrict__ boff, const int64_t* __restrict__ goff, int K,
                                          int ngroups, int64_t* __restrict__ out) {
@@ -246,13 +255,16 @@ gt_status gt_link(gt_ctx* ctx, const float* frame_y_x, int64_t n, float search_r
     job.reset.assign(gframe.size(), 0);
     job.radius = search_range;
     job.memory = (int32_t)memory;
-    std::vector<float> px(N), py(N);
-    for (int64_t i = 0; i < N; i++) {
-        px[i] = frame_y_x[3 * i + 1];
-        py[i] = frame_y_x[3 * i + 2];
+    // the rows as they are; their coordinates become columns on the device
+    CK(ctx->l_rows.ensure(std::max<size_t>((size_t)N * 12, 12)));
+    CK(ctx->l_px.ensure(std::max<int64_t>(N, 1) * 4));
+    CK(ctx->l_py.ensure(std::max<int64_t>(N, 1) * 4));
+    CK(upload_host(ctx->device, ctx->l_rows.p, frame_y_x, (size_t)N * 12, ctx->st));
+    if (N > 0) {
+        split_rows_kernel<<<(unsigned)((N + 255) / 256), 256, 0, ctx->st>>>(
+            ctx->l_rows.as<float>(), N, ctx->l_px.as<float>(), ctx->l_py.as<float>());
+        CK(cudaGetLastError());
     }
-    CKS(upload(ctx, ctx->l_px, px));
-    CKS(upload(ctx, ctx->l_py, py));
     CK(ctx->l_ids.ensure(std::max<int64_t>(N, 1) * 8));
     CKS(run_link(ctx, job, ctx->l_px.as<float>(), ctx->l_py.as<float>(), ctx->l_ids.as<int64_t>(), nullptr, nullptr,
                  nullptr));

@@ -37,8 +37,19 @@ struct DBuf {
         if (p) cudaFree(p);
         p = nullptr;
         n = 0;
-        size_t want = std::max<size_t>(bytes, 256);
-        cudaError_t e = cudaMalloc(&p, want);
+        // an eighth of headroom at most, so that inputs of about the same size
+        // (detections differ from video to video) do not allocate again
+        size_t want = 256;
+        while (want < bytes) want <<= 1;
+        const size_t step = std::min<size_t>(std::max<size_t>(want / 16, 256), (size_t)64 << 20);
+        want = (bytes + step - 1) / step * step;
+        cudaError_t e = cudaMalloc(&p, std::max<size_t>(want, 256));
+        if (e != cudaSuccess && want > bytes) {
+            cudaGetLastError();
+            want = std::max<size_t>(bytes, 256);
+            e = cudaMalloc(&p, want);
+        }
+        want = std::max<size_t>(want, 256);
         if (e == cudaSuccess) n = want;
         return e;
     }
@@ -141,7 +152,7 @@ struct gt_ctx {
     DBuf stage[2], processed, planes, cand_count, cand_keys, feats_raw, feat_count, feats_out, kept_count,
         fin_scratch, flags, ident, tabs_f, tabs_i, tabs_s, tabs_m, row_off, frame_num;
     DBuf l_srt, l_sortscr, l_fcnt, l_bcnt, l_foff, l_boff, l_fpts, l_bpts, l_bdist, l_scan, l_scratch, l_ids, l_cnt,
-        l_dur, l_flags, l_goff, l_pgroup, l_vgrp, l_reset, l_vpoff, l_px, l_py, l_ge, l_rowdur, l_part;
+        l_dur, l_flags, l_goff, l_pgroup, l_vgrp, l_reset, l_vpoff, l_px, l_py, l_rows, l_ge, l_rowdur, l_part;
     // windowed linking inside gt_batch (slot mode)
     DBuf fstd, std_scratch, amask, astatus, acount;   // snr / minmass_snr / adaptive_background
     DBuf illum_taps, illum_shared, illum_prof, illum_corr;  // illumination correction
@@ -365,6 +376,13 @@ inline gt_status upload(gt_ctx* ctx, DBuf& b, const std::vector<T>& v) {
     return GT_OK;
 }
 
+// bytes from host memory to device memory dst, in the order of `st` as
+// cudaMemcpyAsync would.  Large pageable sources cross through pinned lanes
+// filled by host threads, and have landed when the call returns (gt_table.cu).
+cudaError_t upload_host(int device, void* dst, const void* src, size_t bytes, cudaStream_t st);
+// whether upload_host(src, bytes) would use the lanes, and so block
+bool upload_blocks(const void* src, size_t bytes);
+
 inline gt_status subset_groups(gt_ctx* ctx, const float* rows, int64_t n, int ncols, std::vector<int64_t>& goff,
                         std::vector<int64_t>& gframe) {
     goff.assign(1, 0);
@@ -374,6 +392,10 @@ inline gt_status subset_groups(gt_ctx* ctx, const float* rows, int64_t n, int nc
     while (true) {
         if (idx < n) {
             float f = rows[idx * ncols];
+            if (f == cur) {
+                idx++;
+                continue;
+            }
             if (f > cur) {
                 goff.push_back(idx);
                 gframe.push_back((int64_t)cur);

@@ -17,7 +17,7 @@ import numpy as np
 
 from . import _ffi
 from ._params import trackpy_params
-from .api import _DEVICE, _Frames, _run, _table_to_frame
+from .api import _DEVICE, _SHORT_PIXELS, _Frames, _run, _table_to_frame
 
 __all__ = ["ProposalNet", "batch_learned", "compare", "calibrate"]
 
@@ -173,7 +173,7 @@ def batch_learned(file_or_array, diameter, net, **kwargs):
                                            reset_arr.ctypes.data_as(_P64) if len(reset_arr) else None,
                                            len(reset_arr), ctypes.byref(out))
 
-    st = _run(ctx, call, bool(kwargs.get("tqdm", True)) and fr.T > 1)
+    st = _run(ctx, call, bool(kwargs.get("tqdm", True)) and fr.T > 1, fr.T * fr.H * fr.W <= _SHORT_PIXELS)
     ctx.check(st)
     return _table_to_frame(ctx, out, params)
 
