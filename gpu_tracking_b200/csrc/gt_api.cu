@@ -304,10 +304,9 @@ struct PipeLink {
     bool segmented = false;
     LinkSegs segs;      // segments of a window (link_segments_kernel)
     int seg_len = 0, seg_len_last = 0;
-    float bin_w = 1.0f;  // row-bin width of the neighbour search index
 
     gt_status setup(gt_ctx* c, int64_t NT, uint32_t feat_cap, int SC, float radius, int memory,
-                    const std::vector<uint8_t>& reset, int32_t H) {
+                    const std::vector<uint8_t>& reset) {
         ctx = c;
         C = feat_cap;
         K = memory + 1;
@@ -316,12 +315,9 @@ struct PipeLink {
         if (ctx->w_list_cap <= 0) ctx->w_list_cap = std::max<int64_t>(max_items, 1 << 20);
         if (ctx->w_edge_cap <= 0) ctx->w_edge_cap = std::max<int64_t>(C * 16, 1 << 16);
         list_cap = ctx->w_list_cap;
-        CK(ctx->w_srt.ensure(NS * 4));
-        // row bins of at least the search radius over the frame height: a
-        // neighbour search reads two bin offsets and scans about three bins
-        CK(ctx->w_bins.ensure((size_t)NT * (kLinkRowBins + 1) * 4));
-        bin_w = std::max(radius, (float)H / (float)kLinkRowBins);
-        if (!(bin_w > 0.0f) || !std::isfinite(bin_w)) bin_w = 1.0f;
+        CK(ctx->w_rec.ensure((size_t)NS * 16));
+        CK(ctx->w_cells.ensure((size_t)NT * (link_cells_per_slot(C) + 1) * 4));
+        CK(ctx->w_geo.ensure((size_t)NT * 16));
         // the previous call's list kernels may still read the buffers
         CK(cudaStreamSynchronize(ctx->ls));
         for (int b = 0; b < 2; b++) {
@@ -426,32 +422,32 @@ struct PipeLink {
         if (nwin >= 2) CK(cudaStreamWaitEvent(ctx->ls, ctx->w_linked[b], 0));
         nwin++;
         in.groups_ready = s1;
-        uint32_t* srt = ctx->w_srt.as<uint32_t>();
         {
             Prof pf(ctx, "link_sort", ctx->ls);
-            CK(link_sort_groups_range(in, srt, s0, s1, ctx->w_bins.as<int32_t>(), bin_w, ctx->ls));
+            CK(link_cells(in, ctx->w_rec.as<float4>(), ctx->w_cells.as<int32_t>(), ctx->w_geo.as<float4>(), s0, s1,
+                          ctx->ls));
         }
+        LinkLists L;
+        L.rec = ctx->w_rec.as<float4>();
+        L.cell_off = ctx->w_cells.as<int32_t>();
+        L.geo = ctx->w_geo.as<float4>();
+        L.pbase = p0;
         int64_t* fcnt = ctx->w_fcnt[b].as<int64_t>();
         int64_t* bcnt = ctx->w_bcnt[b].as<int64_t>();
         CK(cudaMemsetAsync(fcnt, 0, items * 8, ctx->ls));
         CK(cudaMemsetAsync(bcnt, 0, items * 8, ctx->ls));
         {
             Prof pf(ctx, "link_lists", ctx->ls);
-            CK(link_count_lists_range(in, srt, p0, p1, fcnt, bcnt, out.flags, ctx->ls));
+            CK(link_count_lists_range(in, L, p1, fcnt, bcnt, out.flags, ctx->ls));
         }
         size_t tb = scan_bytes;
         CK(cub::DeviceScan::ExclusiveSum(ctx->w_scan.p, tb, fcnt, ctx->w_foff[b].as<int64_t>(), items, ctx->ls));
         CK(cub::DeviceScan::ExclusiveSum(ctx->w_scan.p, tb, bcnt, ctx->w_boff[b].as<int64_t>(), items, ctx->ls));
-        LinkLists L;
         L.f_off = ctx->w_foff[b].as<int64_t>();
         L.b_off = ctx->w_boff[b].as<int64_t>();
         L.f_pts = ctx->w_fpts[b].as<int32_t>();
         L.b_pts = ctx->w_bpts[b].as<int32_t>();
         L.b_dist = ctx->w_bdist[b].as<float>();
-        L.srt = srt;
-        L.bins = ctx->w_bins.as<int32_t>();
-        L.bin_w = bin_w;
-        L.pbase = p0;
         L.f_cap = list_cap;
         L.b_cap = list_cap;
         {
@@ -598,7 +594,7 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
     CK(cudaMemsetAsync(ctx->flags.p, 0, 16, ctx->st));
     CK(ctx->walk_starts.ensure(8));
     CK(cudaMemsetAsync(ctx->walk_starts.p, 0, 8, ctx->st));
-    if (pl) CKS(pl->setup(ctx, NT, feat_cap, SC, p.search_range, (int)p.memory, *reset, H));
+    if (pl) CKS(pl->setup(ctx, NT, feat_cap, SC, p.search_range, (int)p.memory, *reset));
     // finalize scratch for frames with more detections than shared memory sorts
     size_t fin_per_frame = 0;
     if (feat_cap > (uint32_t)kFinalizeSmemSort) {

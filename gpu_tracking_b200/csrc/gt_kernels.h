@@ -10,7 +10,8 @@
 namespace gt {
 
 constexpr int kMaxRadii = 256;
-constexpr int kLinkRowBins = 512;   // row bins per group of the windowed linker's neighbour search
+// slot mode: cells a group's share of the cell offsets holds at most (as many as its slots need)
+__host__ __device__ constexpr int64_t link_cells_per_slot(int64_t slots) { return slots > 1024 ? 4096 : 4 * slots + 1; }
 
 struct FinalizeConsts {
     int32_t H, W;
@@ -269,12 +270,12 @@ struct LinkLists {
     int64_t pbase = 0;            // first point the offset arrays cover
     int64_t f_cap = -1, b_cap = -1;  // entries f_pts / b_pts hold (-1: sized exactly)
     int64_t f_entries = -1;          // forward entries of lists sized exactly (-1: not known)
-    // optional row-bin index of the sorted groups: for group g, entry
-    // g * (kLinkRowBins + 1) + b is the first sorted position whose row falls
-    // in bin b or later (bin = clamp(floor(row / bin_w), 0, kLinkRowBins - 1),
-    // rows that are NaN after every bin); nullptr = bisect the rows instead
-    const int32_t* bins = nullptr;
-    float bin_w = 0.0f;
+    // cell index of the groups (link_cells): per group, its points as (row,
+    // column, index) records cell by cell, the cells' offsets and the corner
+    // and scale of its grid; nullptr = bisect srt instead
+    const float4* rec = nullptr;
+    const int32_t* cell_off = nullptr;
+    const float4* geo = nullptr;
 };
 
 struct LinkScratch {
@@ -345,16 +346,17 @@ struct LinkSegs {
 
 cudaError_t link_sort_groups(const LinkInput& in, uint32_t* srt, uint8_t* scratch, size_t scratch_per_group,
                              int max_group, cudaStream_t st);
-// groups [g0, g1) only
-// groups [g0, g1) only; with bins, also their row-bin index (LinkLists::bins)
-cudaError_t link_sort_groups_range(const LinkInput& in, uint32_t* srt, int g0, int g1, int32_t* bins, float bin_w,
-                                   cudaStream_t st);
+// cell index of groups [g0, g1): rec holds a record per point (slot), cell_off
+// 4 * points + groups entries (slot mode: link_cells_per_slot + 1 a group),
+// geo one entry per group
+cudaError_t link_cells(const LinkInput& in, float4* rec, int32_t* cell_off, float4* geo, int g0, int g1,
+                       cudaStream_t st);
 cudaError_t link_count_lists(const LinkInput& in, const uint32_t* srt, int64_t* f_cnt, int64_t* b_cnt,
                              cudaStream_t st);
 cudaError_t link_fill_lists(const LinkInput& in, const LinkLists& L, cudaStream_t st);
-// points [p0, p1) only; f_cnt/b_cnt and L's offsets are relative to p0 (L.pbase == p0)
-cudaError_t link_count_lists_range(const LinkInput& in, const uint32_t* srt, int64_t p0, int64_t p1,
-                                   int64_t* f_cnt, int64_t* b_cnt, uint32_t* flags, cudaStream_t st);
+// points [L.pbase, p1) only; f_cnt/b_cnt and L's offsets are relative to L.pbase
+cudaError_t link_count_lists_range(const LinkInput& in, const LinkLists& L, int64_t p1, int64_t* f_cnt,
+                                   int64_t* b_cnt, uint32_t* flags, cudaStream_t st);
 cudaError_t link_fill_lists_range(const LinkInput& in, const LinkLists& L, int64_t p1, uint32_t* flags,
                                   cudaStream_t st);
 size_t link_scratch_bytes(int32_t max_group, int64_t max_edges, int64_t npoints_video, int32_t memory);

@@ -73,15 +73,17 @@ gt_status run_link(gt_ctx* ctx, const LinkJob& job, const float* px, const float
     in.radius = job.radius;
     in.memory = job.memory;
 
-    int np2 = 1;
-    while (np2 < max_group) np2 <<= 1;
-    size_t per_group = (np2 > 4096) ? (size_t)np2 * 8 : 0;
-    CK(ctx->l_srt.ensure(std::max<int64_t>(N, 1) * 4));
-    CK(ctx->l_sortscr.ensure(std::max<size_t>(per_group * ngroups, 8)));
+    CK(ctx->l_rec.ensure((size_t)std::max<int64_t>(N, 1) * 16));
+    CK(ctx->l_cells.ensure((size_t)(4 * N + ngroups + 1) * 4));
+    CK(ctx->l_geo.ensure((size_t)std::max(ngroups, 1) * 16));
+    LinkLists L;
+    L.rec = ctx->l_rec.as<float4>();
+    L.cell_off = ctx->l_cells.as<int32_t>();
+    L.geo = ctx->l_geo.as<float4>();
     {
         Prof pf(ctx, "link_sort");
-        CK(link_sort_groups(in, ctx->l_srt.as<uint32_t>(), ctx->l_sortscr.as<uint8_t>(), per_group, max_group,
-                            ctx->st));
+        CK(link_cells(in, ctx->l_rec.as<float4>(), ctx->l_cells.as<int32_t>(), ctx->l_geo.as<float4>(), 0, ngroups,
+                      ctx->st));
     }
     const size_t NK = (size_t)N * K;
     CK(ctx->l_fcnt.ensure((NK + 1) * 8));
@@ -92,8 +94,7 @@ gt_status run_link(gt_ctx* ctx, const LinkJob& job, const float* px, const float
     CK(cudaMemsetAsync(ctx->l_bcnt.p, 0, (NK + 1) * 8, ctx->st));
     {
         Prof pf(ctx, "link_lists");
-        CK(link_count_lists(in, ctx->l_srt.as<uint32_t>(), ctx->l_fcnt.as<int64_t>(), ctx->l_bcnt.as<int64_t>(),
-                            ctx->st));
+        CK(link_count_lists_range(in, L, N, ctx->l_fcnt.as<int64_t>(), ctx->l_bcnt.as<int64_t>(), nullptr, ctx->st));
     }
     size_t tmp_bytes = 0;
     CK(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, ctx->l_fcnt.as<int64_t>(), ctx->l_foff.as<int64_t>(),
@@ -121,13 +122,11 @@ gt_status run_link(gt_ctx* ctx, const LinkJob& job, const float* px, const float
     CK(ctx->l_fpts.ensure(std::max<int64_t>(ftot, 1) * 4));
     CK(ctx->l_bpts.ensure(std::max<int64_t>(btot, 1) * 4));
     CK(ctx->l_bdist.ensure(std::max<int64_t>(btot, 1) * 4));
-    LinkLists L;
     L.f_off = ctx->l_foff.as<int64_t>();
     L.b_off = ctx->l_boff.as<int64_t>();
     L.f_pts = ctx->l_fpts.as<int32_t>();
     L.b_pts = ctx->l_bpts.as<int32_t>();
     L.b_dist = ctx->l_bdist.as<float>();
-    L.srt = ctx->l_srt.as<uint32_t>();
     L.f_entries = ftot;
     {
         Prof pf(ctx, "link_lists");

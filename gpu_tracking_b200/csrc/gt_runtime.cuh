@@ -151,7 +151,7 @@ struct gt_ctx {
     // device buffers, grown on demand and kept for the next call
     DBuf stage[2], processed, planes, cand_count, cand_keys, feats_raw, feat_count, feats_out, kept_count,
         fin_scratch, flags, ident, tabs_f, tabs_i, tabs_s, tabs_m, row_off, frame_num;
-    DBuf l_srt, l_sortscr, l_fcnt, l_bcnt, l_foff, l_boff, l_fpts, l_bpts, l_bdist, l_scan, l_scratch, l_ids, l_cnt,
+    DBuf l_rec, l_cells, l_geo, l_fcnt, l_bcnt, l_foff, l_boff, l_fpts, l_bpts, l_bdist, l_scan, l_scratch, l_ids, l_cnt,
         l_dur, l_flags, l_goff, l_pgroup, l_vgrp, l_reset, l_vpoff, l_px, l_py, l_rows, l_ge, l_rowdur, l_part;
     // windowed linking inside gt_batch (slot mode)
     DBuf fstd, std_scratch, amask, astatus, acount;   // snr / minmass_snr / adaptive_background
@@ -161,7 +161,7 @@ struct gt_ctx {
     DBuf vd_src, vd_dec, vd_blk, vd_bad;  // video files decoded on the device: streams, bytes, blocks, flag
     int64_t last_walk_starts = 0;
     int32_t illum_rint = 0;
-    DBuf w_srt, w_bins, w_scan, w_scratch, w_ids, w_dur, w_state, w_cnt, w_flags, w_vgrp, w_reset;
+    DBuf w_rec, w_cells, w_geo, w_scan, w_scratch, w_ids, w_dur, w_state, w_cnt, w_flags, w_vgrp, w_reset;
     // segments of the linker's frame loop: scratch of the speculative runs, their states, arrivals
     DBuf w_segs, w_segst, w_segarr, l_segs, l_segst, l_segarr;
     // two sets of window neighbour lists: the lists of window w + 1 are built
