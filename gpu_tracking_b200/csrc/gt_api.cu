@@ -120,7 +120,6 @@ gt_status make_locate_consts(gt_ctx* ctx, const gt_params& p, int32_t H, int32_t
 template <typename T>
 void set_fast_div(gt_ctx* ctx, LocateConsts& c) {
     c.fast_div = 0;
-    if (std::is_same<T, float>::value) return;
     auto split = [](float d, float* zh, float* zl) {
         const double r = 1.0 / (double)d;
         *zh = (float)r;
@@ -128,6 +127,20 @@ void set_fast_div(gt_ctx* ctx, LocateConsts& c) {
     };
     split(c.gnorm, &c.zh_g, &c.zl_g);
     split(c.kk, &c.zh_k, &c.zl_k);
+    auto safe = [](double lo, double hi, double d, double zh, double zl) {
+        const double tiny = std::ldexp(1.0, -120), big = std::ldexp(1.0, 100);
+        if (zl != 0.0 && lo * std::fabs(zl) < tiny) return false;
+        if (lo / d < tiny || hi * zh > big || hi / d > big) return false;
+        return true;
+    };
+    if (std::is_same<T, float>::value) {
+        // float pixels: the kernel itself tells dividends in [2^-60, 2^60)
+        // from others, which it divides
+        const double lo = std::ldexp(1.0, -60), hi = std::ldexp(1.0, 60);
+        if (!(c.gnorm > 0.0f) || !safe(lo, hi, c.gnorm, c.zh_g, c.zl_g) || !safe(lo, hi, c.kk, c.zh_k, c.zl_k)) return;
+        c.fast_div = const_div_proven(c.gnorm, c.zh_g, c.zl_g, ctx->st) && const_div_proven(c.kk, c.zh_k, c.zl_k, ctx->st);
+        return;
+    }
     double tmin = INFINITY, tsum = 0.0;
     for (int i = 0; i <= 2 * c.R; i++) {
         if (!(c.taps[i] > 0.0f)) return;
@@ -139,12 +152,6 @@ void set_fast_div(gt_ctx* ctx, LocateConsts& c) {
     const double col_lo = tmin * (row_lo / gn), col_hi = tsum * (row_hi / gn);
     const double g_lo = 0.5 * std::min(row_lo, col_lo), g_hi = 2.0 * std::max(row_hi, col_hi);
     const double k_lo = 0.5, k_hi = 2.0 * 65535.0 * kk;
-    auto safe = [](double lo, double hi, double d, double zh, double zl) {
-        const double tiny = std::ldexp(1.0, -120), big = std::ldexp(1.0, 100);
-        if (zl != 0.0 && lo * std::fabs(zl) < tiny) return false;
-        if (lo / d < tiny || hi * zh > big || hi / d > big) return false;
-        return true;
-    };
     if (!safe(g_lo, g_hi, gn, c.zh_g, c.zl_g) || !safe(k_lo, k_hi, kk, c.zh_k, c.zl_k)) return;
     if (!const_div_proven(c.gnorm, c.zh_g, c.zl_g, ctx->st) || !const_div_proven(c.kk, c.zh_k, c.zl_k, ctx->st))
         return;
@@ -957,6 +964,8 @@ gt_status batch_impl(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_d
     CKS(make_locate_consts(ctx, p, H, W, c));
     set_fast_div<T>(ctx, c);
     if (net) {
+        // the seed patches' division has no test for float dividends
+        if (std::is_same<T, float>::value) c.fast_div = 0;
         const int ri = (c.circle - 1) / 2;
         if (ri < 2 || ri > 7)
             return set_err(ctx, GT_ERR_INVALID_ARGUMENT, "learned proposals need a diameter between 5 and 16");
@@ -966,7 +975,7 @@ gt_status batch_impl(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_d
     }
     if (p.has_illumination_sigma) {
         // the locate stages see the corrected f32 frames
-        c.fast_div = 0;
+        set_fast_div<float>(ctx, c);
         CKS(illumination_setup<T>(ctx, p, frames, on_device, NT, H, W));
     }
     LogTables lt;

@@ -8,26 +8,28 @@
 //      converted exactly to float), the next step's are prefetched;
 //   B  row pass: each thread makes 4 adjacent columns from float4 loads;
 //   C  column pass: each thread makes the step's 8 rows of one column;
-//   D  vertical dilation maximum, 8 rows of one column per thread;
+//   D  vertical dilation maximum, 8 rows of the same column by the same thread
+//      (the new rows from registers, no barrier after C);
 //   E  horizontal dilation maximum, the candidate test and the store of the
 //      segment's processed rows, 4 columns per thread; candidates gather in a
-//      shared-memory buffer of the tile (one shared atomic per warp) and go
-//      to the frame's list with one global reservation per tile.
-// Two ring layouts hold the row-pass rows and the processed rows:
-//   integer pixels (ring_tile): single-copy rings of RING rows, RING a
-//      multiple of the 8-row step, so step s writes ring rows
-//      8*(s % (RING/8)) .. +7 without wrapping; the column pass and the
-//      vertical maxima are compiled once per ring phase s % (RING/8) and
-//      picked by a uniform branch, so every ring row they touch is a
-//      compile-time offset.  Rows above and below the frame hold a Gaussian
-//      row sum of +0 instead of being skipped: integer pixels make every row
-//      sum >= +0, and fma(w, +0, acc) == acc for acc >= +0, so the column
-//      pass needs no per-row bounds test.  The smaller rings let 4 CTAs share
-//      an SM where the shared memory allows it;
-//   float pixels (strip_tile): rings that hold every row twice (at r and
-//      r + ring), so any window of consecutive rows is contiguous, with
-//      per-tap bounds tests at the frame's top and bottom (a float row sum
-//      may be -0, which the skipped term keeps and +0 would not).
+//      shared-memory buffer of the tile and go to the frame's list with one
+//      global reservation per tile.
+// The row-pass rows and the processed rows are in single-copy rings of RING
+// rows, RING a multiple of the 8-row step, so step s writes ring rows
+// 8*(s % (RING/8)) .. +7 without wrapping; C and D are compiled once per ring
+// phase s % (RING/8) and picked by a uniform branch, so every ring row they
+// touch is a compile-time offset.  Rows above and below the frame hold a
+// Gaussian row sum of +0 instead of being skipped: fma(w, +0, acc) == acc
+// unless acc is -0, which integer pixels cannot give and float pixels give only
+// with a zero sum, which a plain loop then makes again.
+// Bound by instruction issue and the four barriers of a step.  Bandpass of 128
+// frames on a B200, us a frame: 2048^2 u16 27.2 with a barrier between C and D
+// and candidates appended by warp scans, 25.6 so; float pixels with rows kept
+// twice, per-tap row tests and IEEE division 14.6 (1024^2, diameter 9), 15.2
+// (diameter 11) and 15.8 (smoothing radius 8, no candidates), 9.3, 10.3 and
+// 11.8 in the ring layout with the checked fast division.  Measured and not
+// kept: the column pass in packed FP32 pairs of columns (26.6, as many as
+// without it).
 // The tap loops are unrolled for the compile-time radius.
 // The floating-point operation sequence of every output is the oracle's:
 // sequential fused multiply-adds over the taps, sequential boxcar sums (for
@@ -65,17 +67,11 @@ struct StripGeom {
     static constexpr int NX4 = (4 + 2 * R + 3) / 4;       // float4 loads per row-pass group
     static constexpr int RWp = PWp + 4 * (NX4 - 1);       // staged raw columns (>= PWp + 2R)
     static constexpr int RW4 = RWp / 4;
-    static constexpr int XR = kStepRows + 2 * R;          // row-pass ring rows
-    static constexpr int PR = kStepRows + KD - 1;         // processed ring rows
     static constexpr int NV4 = (KD + 3 + 3) / 4;          // float4 loads per dilation group
     static constexpr int RAWV = kStepRows * RW4;          // 4-pixel loads per step
     static constexpr int RAWVPT = (RAWV + kStripThreads - 1) / kStripThreads;
     static constexpr int RAWN = kStepRows * RWp;
     static constexpr int RAWPT = (RAWN + kStripThreads - 1) / kStripThreads;
-    // the vertical maxima (stages D-E) reuse the staged raw rows (stages A-B)
-    static constexpr size_t smem_floats = (size_t)kStepRows * RWp + 2 * (size_t)(2 * XR) * PWp +
-                                          (size_t)(2 * PR) * PWp + 4 + kCandBuf;
-    static constexpr int min_blocks = (smem_floats * 4 + 1024) * 3 <= 227 * 1024 ? 3 : 2;
     static_assert(RWp % 4 == 0 && RWp >= PWp + 2 * R, "staged raw row");
     static_assert(RWp >= PWp, "vertical maxima fit in the staging rows");
     static_assert(4 * 31 + 4 * NV4 <= PWp, "dilation row reads stay in the row");
@@ -140,53 +136,42 @@ struct Tree<1> {
     __device__ __forceinline__ static float sum(const float* a) { return a[0]; }
 };
 
+// x / d for one of the call's two divisors.  FAST: as fma(x, zh, x * zl), equal
+// to IEEE division for every dividend of integer pixels; for a float dividend
+// where its magnitude lies in [2^-60, 2^60), the range the host's check covers,
+// and for +0 (fma(+0, zh, +-0) is +0 as well).
 template <bool FAST>
-__device__ __forceinline__ float div_gnorm(float x, const LocateConsts& c) {
-    return FAST ? __fmaf_rn(x, c.zh_g, __fmul_rn(x, c.zl_g)) : __fdiv_rn(x, c.gnorm);
+__device__ __forceinline__ float const_div(float x, float d, float zh, float zl) {
+    return FAST ? __fmaf_rn(x, zh, __fmul_rn(x, zl)) : __fdiv_rn(x, d);
 }
-template <bool FAST>
-__device__ __forceinline__ float div_kk(float x, const LocateConsts& c) {
-    return FAST ? __fmaf_rn(x, c.zh_k, __fmul_rn(x, c.zl_k)) : __fdiv_rn(x, c.kk);
+__device__ __forceinline__ bool outside_fast_div(float x) {
+    const uint32_t u = __float_as_uint(x);
+    return (u & 0x7FFFFFFFu) - ((127u - 60u) << 23) >= (120u << 23) && u != 0u;
 }
+// out of line: the rare other dividends must not bloat the loops
+__device__ __noinline__ float ieee_div(float x, float d) { return __fdiv_rn(x, d); }
 
 // Appends the candidates a thread found among its 4 columns (bits of cmask,
-// cnt of them) at row cd, columns ccol..ccol+3: warp-aggregated slots in the
-// tile's shared buffer (one shared atomic per warp); a full buffer sends the
-// warp's candidates straight to the frame's list.
-__device__ __forceinline__ void append_cands(const int tid, const int cnt, const uint32_t cmask, const int cd,
-                                             const int ccol, const int W, uint32_t* cbuf_n, uint32_t* cbuf,
+// cnt of them) at row cd, columns ccol..ccol+3 to the tile's shared buffer,
+// each lane for itself: a warp's 128 pixels hold a candidate every other
+// step and rarely two, so a warp scan cost more than the shared atomics it
+// saved (their order does not matter).  What the full buffer does not take goes
+// to the frame's list.
+__device__ __forceinline__ void append_cands(const int cnt, const uint32_t cmask, const int cd, const int ccol,
+                                             const int W, uint32_t* cbuf_n, uint32_t* cbuf,
                                              uint32_t* __restrict__ cand_slot, uint32_t* __restrict__ cout,
                                              const uint32_t cand_cap, uint32_t* __restrict__ flags) {
-    if (!__any_sync(0xffffffffu, cnt != 0)) return;
-    const int lane = tid & 31;
-    int incl = cnt;
-#pragma unroll
-    for (int dd = 1; dd < 32; dd <<= 1) {
-        int v = __shfl_up_sync(0xffffffffu, incl, dd);
-        if (lane >= dd) incl += v;
-    }
-    const int wtot = __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t base = 0;
-    if (lane == 31) base = atomicAdd(cbuf_n, (uint32_t)wtot);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    uint32_t pos = base + (uint32_t)(incl - cnt);
-    if (base + (uint32_t)wtot <= (uint32_t)kCandBuf) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            if (!(cmask & (1u << k))) continue;
-            cbuf[pos++] = (uint32_t)cd * (uint32_t)W + (uint32_t)(ccol + k);
-        }
-    } else {
-        uint32_t gb = 0;
-        if (lane == 31) gb = atomicAdd(cand_slot, (uint32_t)wtot);
-        gb = __shfl_sync(0xffffffffu, gb, 31);
-        pos = gb + (uint32_t)(incl - cnt);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            if (!(cmask & (1u << k))) continue;
-            if (pos < cand_cap) cout[pos] = (uint32_t)cd * (uint32_t)W + (uint32_t)(ccol + k);
+    if (cnt == 0) return;
+    const uint32_t key = (uint32_t)cd * (uint32_t)W + (uint32_t)ccol;
+    uint32_t pos = atomicAdd(cbuf_n, (uint32_t)cnt);
+    for (uint32_t m = cmask; m; m &= m - 1u, pos++) {
+        const uint32_t k = key + (uint32_t)(__ffs(m) - 1);
+        if (pos < (uint32_t)kCandBuf) {
+            cbuf[pos] = k;
+        } else {
+            const uint32_t q = atomicAdd(cand_slot, 1u);
+            if (q < cand_cap) cout[q] = k;
             else atomicOr(flags, kFlagCandOverflow);
-            pos++;
         }
     }
 }
@@ -339,210 +324,8 @@ __device__ __forceinline__ void extract_step(const int tid, const float* vb, Cen
             ccol = gc0;
         }
     }
-    append_cands(tid, cnt, cmask, cd, ccol, W, cbuf_n, cbuf, cand_slot, cout, cand_cap, flags);
+    append_cands(cnt, cmask, cd, ccol, W, cbuf_n, cbuf, cand_slot, cout, cand_cap, flags);
 }
-
-// One tile: the strip of output columns [c0, c0 + 128) and rows [R0, R1) of
-// an H x W frame (img: its pixels, proc: its processed image), candidates
-// appended to the list counted by *cand_slot (keys at cout).
-template <typename T, int R, int KD, bool FAST>
-__device__ __forceinline__ void strip_tile(const T* __restrict__ img, float* __restrict__ proc, const LocateConsts& c,
-                                           const int H, const int W, const int c0, const int R0, const int R1,
-                                           const int vec_ok, const float thr, uint32_t* __restrict__ cand_slot,
-                                           uint32_t* __restrict__ cout, const uint32_t cand_cap,
-                                           uint32_t* __restrict__ flags) {
-    using G = StripGeom<R, KD>;
-    constexpr int O = G::O, E = G::E, PWp = G::PWp, RWp = G::RWp, XR = G::XR, PR = G::PR, SH4 = G::SH4;
-    constexpr bool kInt = IsIntPix<T>::value;
-    extern __shared__ float4 sm4[];
-    float* sm = (float*)sm4;
-    float* stage = sm;                          // [8][RWp]      raw columns xa .. xa+RWp
-    float* xg = stage + kStepRows * RWp;        // [2XR][PWp]    row pass g / gnorm, rows stored twice
-    float* xb = xg + 2 * XR * PWp;              // [2XR][PWp]    row pass boxcar
-    float* pr = xb + 2 * XR * PWp;              // [2PR][PWp]    processed rows, stored twice
-    float* vb = stage;                          // [8][PWp]      vertical maxima (pc0-relative columns)
-    uint32_t* cbuf_n = (uint32_t*)(pr + 2 * PR * PWp);   // [4]   buffered candidates, flush base
-    uint32_t* cbuf = cbuf_n + 4;                // [kCandBuf]    candidate keys of the tile
-
-    const int x0 = R0 - O - R;          // first raw / row-pass row
-    const int pc0 = c0 - O;             // first processed column of the strip's dilation windows
-    const int xa = pc0 - R - SH4;       // first staged raw column (a multiple of 4)
-    const int ps = xa + R;              // processed column of row-pass index 0 (= pc0 - SH4)
-    const int tid = threadIdx.x;
-    const bool edge_cols = (xa < 0) || (xa + RWp > W);
-    const bool vec = vec_ok && !edge_cols;
-    // 16-byte stores of processed rows: every row start is a multiple of 4 floats
-    const bool st4 = (W % 4 == 0) && ((uintptr_t)proc % 16 == 0);
-    // steps until the dilation rows reach R1: x0 + 8s - R - E + 8 >= R1
-    const int nsteps = (R1 - x0 + R + E + kStepRows - 1) / kStepRows;
-
-    // ---- A: staging of raw rows (registers hold the next step's pixels)
-    RawRows<T, R, KD> raw;
-    if (tid == 0) *cbuf_n = 0;
-    raw.load(img, H, W, x0, xa, vec, 0);
-    // The first column-pass groups read row-pass rows above x0 that no step
-    // writes.  The outputs that need them are never used, but the sliding
-    // boxcar sum of a group carries its first window into the rows after it
-    // (cs + new - old cancels exactly only for finite integers), so the rings
-    // start as zeros instead of whatever the previous kernel left.
-    for (int i = tid; i < 2 * 2 * XR * PWp / 4; i += kStripThreads)
-        ((float4*)xg)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const float trunc_thr = 1.0f / 255.0f;
-
-    for (int s = 0; s < nsteps; s++) {
-        raw.store(stage, vec);
-        __syncthreads();
-        if (s + 1 < nsteps) raw.load(img, H, W, x0, xa, vec, s + 1);
-
-        // ---- B: row pass (preprocess_rows.wgsl), 8 rows x PWp columns, 4 per thread
-        {
-            for (int t = tid; t < kStepRows * G::NG; t += kStripThreads) {
-                const int j = t / G::NG, gq = t - j * G::NG;
-                const int col = 4 * gq;
-                const float4* src = (const float4*)(stage + j * RWp + col);
-                float x[4 * G::NX4];
-#pragma unroll
-                for (int i = 0; i < G::NX4; i++) {
-                    const float4 v = src[i];
-                    x[4 * i] = v.x;
-                    x[4 * i + 1] = v.y;
-                    x[4 * i + 2] = v.z;
-                    x[4 * i + 3] = v.w;
-                }
-                float og[4], ob[4];
-                float cs = 0.0f;
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    float gs = 0.0f;
-                    if (!edge_cols) {
-#pragma unroll
-                        for (int i = 0; i <= 2 * R; i++) gs = __fmaf_rn(c.taps[i], x[k + i], gs);
-                    } else {
-                        // Gaussian taps outside the frame are skipped
-                        const int gcol = ps + col + k;
-#pragma unroll
-                        for (int i = 0; i <= 2 * R; i++) {
-                            const int gc = gcol + i - R;
-                            if (gc >= 0 && gc < W) gs = __fmaf_rn(c.taps[i], x[k + i], gs);
-                        }
-                    }
-                    if (kInt) {
-                        // exact integers: the window sum, then sliding differences
-                        if (k == 0) cs = Tree<2 * R + 1>::sum(x);
-                        else cs = __fadd_rn(cs, __fsub_rn(x[k + 2 * R], x[k - 1]));
-                    } else {
-                        cs = 0.0f;
-#pragma unroll
-                        for (int i = 0; i <= 2 * R; i++) cs = __fadd_rn(cs, x[k + i]);
-                    }
-                    og[k] = div_gnorm<FAST>(gs, c);
-                    ob[k] = cs;
-                }
-                const int xrow = (kStepRows * s + j) % XR;
-                const float4 g4 = make_float4(og[0], og[1], og[2], og[3]);
-                const float4 b4 = make_float4(ob[0], ob[1], ob[2], ob[3]);
-                *(float4*)(xg + xrow * PWp + col) = g4;
-                *(float4*)(xg + (xrow + XR) * PWp + col) = g4;
-                *(float4*)(xb + xrow * PWp + col) = b4;
-                *(float4*)(xb + (xrow + XR) * PWp + col) = b4;
-            }
-        }
-        __syncthreads();
-
-        // ---- C: column pass (preprocess_cols.wgsl) for the step's 8 processed
-        // rows q = x0 + 8s - R + k, one column per thread
-        if (tid < PWp) {
-            const int pc = tid;
-            const int q0 = x0 + kStepRows * s - R;
-            const int gcol = ps + pc;
-            // row-pass rows q0 - R .. q0 + 7 + R: relative index 8s - 2R + i
-            const int w0 = (kStepRows * s + (XR - 2 * R)) % XR;
-            const float* pg = xg + w0 * PWp + pc;
-            const float* pb = xb + w0 * PWp + pc;
-            float vg[kStepRows + 2 * R], vbx[kStepRows + 2 * R];
-#pragma unroll
-            for (int i = 0; i < kStepRows + 2 * R; i++) {
-                vg[i] = pg[i * PWp];
-                vbx[i] = pb[i * PWp];
-            }
-            const bool col_in = (gcol >= 0 && gcol < W);
-            const bool rows_in = (q0 >= R && q0 + kStepRows - 1 < H - R);
-            float cs = 0.0f;
-            // processed row q has relative index q - (x0 - R) = 8s + k
-            const int p0 = (kStepRows * s) % PR;
-#pragma unroll
-            for (int k = 0; k < kStepRows; k++) {
-                const int q = q0 + k;
-                float gs = 0.0f;
-                if (rows_in) {
-#pragma unroll
-                    for (int i = 0; i <= 2 * R; i++) gs = __fmaf_rn(c.taps[i], vg[k + i], gs);
-                } else {
-#pragma unroll
-                    for (int i = 0; i <= 2 * R; i++) {
-                        const int gr = q + i - R;
-                        if (gr >= 0 && gr < H) gs = __fmaf_rn(c.taps[i], vg[k + i], gs);
-                    }
-                }
-                if (kInt) {
-                    if (k == 0) cs = Tree<2 * R + 1>::sum(vbx);
-                    else cs = __fadd_rn(cs, __fsub_rn(vbx[k + 2 * R], vbx[k - 1]));
-                } else {
-                    cs = 0.0f;
-#pragma unroll
-                    for (int i = 0; i <= 2 * R; i++) cs = __fadd_rn(cs, vbx[k + i]);
-                }
-                float r = __fsub_rn(div_gnorm<FAST>(gs, c), div_kk<FAST>(cs, c));
-                if (c.truncate && r < trunc_thr) r = 0.0f;
-                const float v = (col_in && q >= 0 && q < H) ? r : -INFINITY;
-                int pp = p0 + k;
-                if (pp >= PR) pp -= PR;
-                pr[pp * PWp + pc] = v;
-                pr[(pp + PR) * PWp + pc] = v;
-            }
-        }
-        __syncthreads();
-
-        // ---- D: vertical maximum over KD processed rows for the step's 8
-        // dilation rows d = x0 + 8s - R - E + k, one column per thread
-        const int dbase = x0 + kStepRows * s - R - E;
-        if (tid < PWp - SH4) {
-            const int pc = tid + SH4;
-            const int vcol = tid;   // pc0-relative column
-            // output k: processed rows d + k - O .. d + k + E, relative index
-            // 8s - (KD - 1) + k + i
-            const int w0 = (kStepRows * s + (2 * PR - (KD - 1))) % PR;
-            const float* pp = pr + w0 * PWp + pc;
-            float a[KD + kStepRows - 1];
-#pragma unroll
-            for (int i = 0; i < KD + kStepRows - 1; i++) a[i] = pp[i * PWp];
-            // out k = max(a[k..6], mid = a[7..KD-1], a[KD..KD+k-1])
-            const float mid = Tree<KD - 7>::max(a + 7);
-            float sfx[7], pfx[8];
-            sfx[6] = a[6];
-#pragma unroll
-            for (int k = 5; k >= 0; k--) sfx[k] = fmaxf(a[k], sfx[k + 1]);
-            pfx[1] = a[KD];
-#pragma unroll
-            for (int k = 2; k < 8; k++) pfx[k] = fmaxf(pfx[k - 1], a[KD + k - 1]);
-            vb[vcol] = fmaxf(sfx[0], mid);
-#pragma unroll
-            for (int k = 1; k < 7; k++) vb[k * PWp + vcol] = fmaxf(fmaxf(sfx[k], mid), pfx[k]);
-            vb[7 * PWp + vcol] = fmaxf(mid, pfx[7]);
-        }
-        __syncthreads();
-
-        // ---- E: horizontal maximum, the candidate test and the processed rows
-        // (processed row d = dbase + jj is ring row (8s + jj - E) mod PR)
-        extract_step<R, KD>(tid, vb, [&](int jj) { return pr + ((kStepRows * s + jj + (PR - E)) % PR) * PWp; },
-                            dbase, R0, R1, c0, H, W, c, thr, st4, proc, cbuf_n, cbuf, cand_slot, cout, cand_cap,
-                            flags);
-        __syncthreads();
-    }
-    __syncthreads();
-    flush_tile_cands(tid, cbuf_n, cbuf, cand_slot, cout, cand_cap, flags);
-}
-
 
 // Calls f(std::integral_constant<int, p>) for the runtime phase p < PER.
 template <int PER, typename F>
@@ -575,18 +358,20 @@ struct RingGeom {
     static constexpr int rows = (kStepRows + 2 * R > KD + kStepRows - 1) ? kStepRows + 2 * R : KD + kStepRows - 1;
     static constexpr int RING = (rows + kStepRows - 1) / kStepRows * kStepRows;
     static constexpr int PER = RING / kStepRows;   // steps per ring period
+    // the vertical maxima reuse the staged raw rows
     static constexpr size_t smem_floats =
         (size_t)kStepRows * G::RWp + 3 * (size_t)RING * G::PWp + 4 + kCandBuf;
-    // 4 CTAs per SM (56 registers a thread) where the shared memory allows it
+    // 4 CTAs per SM (56 registers a thread, integer pixels) where the shared memory allows it
     // and the radius keeps the column pass's windows in registers
     static constexpr int min_blocks = (R <= 5 && (smem_floats * 4 + 1024) * 4 <= 227 * 1024) ? 4 : 3;
     static_assert(PER <= 4, "ring period");
     static_assert((smem_floats * 4 + 1024) * min_blocks <= 228 * 1024, "shared memory of the resident CTAs");
 };
 
-// The integer-pixel tile (same outputs as strip_tile; layout in the file
-// header): strip of output columns [c0, c0 + 128), rows [R0, R1).
-template <typename T, int R, int KD>
+// One tile: the strip of output columns [c0, c0 + 128) and rows [R0, R1) of
+// an H x W frame (img: its pixels, proc: its processed image), candidates
+// appended to the list counted by *cand_slot (keys at cout).
+template <typename T, int R, int KD, bool FAST>
 __device__ __forceinline__ void ring_tile(const T* __restrict__ img, float* __restrict__ proc, const LocateConsts& c,
                                           const int H, const int W, const int c0, const int R0, const int R1,
                                           const int vec_ok, const float thr, uint32_t* __restrict__ cand_slot,
@@ -596,7 +381,7 @@ __device__ __forceinline__ void ring_tile(const T* __restrict__ img, float* __re
     using RG = RingGeom<R, KD>;
     constexpr int O = G::O, E = G::E, PWp = G::PWp, RWp = G::RWp, SH4 = G::SH4;
     constexpr int RING = RG::RING, PER = RG::PER;
-    static_assert(IsIntPix<T>::value, "row sums >= +0 need non-negative pixels");
+    constexpr bool kInt = IsIntPix<T>::value;
     extern __shared__ float4 sm4[];
     float* sm = (float*)sm4;
     float* stage = sm;                          // [8][RWp]      raw columns xa .. xa+RWp
@@ -649,7 +434,7 @@ __device__ __forceinline__ void ring_tile(const T* __restrict__ img, float* __re
                 x[4 * i + 2] = v.z;
                 x[4 * i + 3] = v.w;
             }
-            float og[4], ob[4];
+            float og[4], ob[4], gv[4];
             float cs = 0.0f;
 #pragma unroll
             for (int k = 0; k < 4; k++) {
@@ -666,11 +451,23 @@ __device__ __forceinline__ void ring_tile(const T* __restrict__ img, float* __re
                         if (gc >= 0 && gc < W) gs = __fmaf_rn(c.taps[i], x[k + i], gs);
                     }
                 }
-                // exact integers: the window sum, then sliding differences
-                if (k == 0) cs = Tree<2 * R + 1>::sum(x);
-                else cs = __fadd_rn(cs, __fsub_rn(x[k + 2 * R], x[k - 1]));
-                og[k] = div_gnorm<true>(gs, c);
+                if (kInt) {
+                    // exact integers: the window sum, then sliding differences
+                    if (k == 0) cs = Tree<2 * R + 1>::sum(x);
+                    else cs = __fadd_rn(cs, __fsub_rn(x[k + 2 * R], x[k - 1]));
+                } else {
+                    cs = 0.0f;
+#pragma unroll
+                    for (int i = 0; i <= 2 * R; i++) cs = __fadd_rn(cs, x[k + i]);
+                }
+                og[k] = const_div<FAST>(gs, c.gnorm, c.zh_g, c.zl_g);
                 ob[k] = cs;
+                gv[k] = gs;
+            }
+            if (!kInt && FAST &&
+                (outside_fast_div(gv[0]) || outside_fast_div(gv[1]) || outside_fast_div(gv[2]) || outside_fast_div(gv[3]))) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) og[k] = ieee_div(gv[k], c.gnorm);
             }
             // rows outside the frame: Gaussian row sum +0 (the column pass
             // skips them), boxcar of the clamped row
@@ -683,7 +480,12 @@ __device__ __forceinline__ void ring_tile(const T* __restrict__ img, float* __re
         __syncthreads();
 
         // ---- C: column pass (preprocess_cols.wgsl) for the step's 8 processed
-        // rows q = x0 + 8s - R + k, one column per thread
+        // rows q = x0 + 8s - R + k, one column per thread, then
+        // ---- D: vertical maximum over KD processed rows for the step's 8
+        // dilation rows d = x0 + 8s - R - E + k of the same column: the 8 rows
+        // just made are in registers, the older ones are the thread's own
+        // writes, so no barrier separates the two
+        const int dbase = x0 + kStepRows * s - R - E;
         by_phase<PER>(phase, [&](auto ph) {
             constexpr int P = decltype(ph)::value;
             if (tid < PWp) {
@@ -699,53 +501,82 @@ __device__ __forceinline__ void ring_tile(const T* __restrict__ img, float* __re
                     vbx[i] = xb[rr * PWp + pc];
                 }
                 const bool col_in = (gcol >= 0 && gcol < W);
+                // float pixels take the plain loop below where a dividend is
+                // not one the fast division covers, and where a sum over rows
+                // outside the frame is zero: fma(w, +0, acc) is acc unless acc
+                // is -0, and then the sum ends as a zero of the wrong sign
+                const bool edge_rows = !kInt && !(q0 >= R && q0 + kStepRows - 1 < H - R);
+                bool plain = false;
                 float cs = 0.0f;
+                // output k: processed rows d + k - O .. d + k + E, ring rows
+                // 8P - (KD - 1) + i
+                float a[KD + kStepRows - 1];
 #pragma unroll
                 for (int k = 0; k < kStepRows; k++) {
                     const int q = q0 + k;
                     float gs = 0.0f;
 #pragma unroll
                     for (int i = 0; i <= 2 * R; i++) gs = __fmaf_rn(c.taps[i], vg[k + i], gs);
-                    if (k == 0) cs = Tree<2 * R + 1>::sum(vbx);
-                    else cs = __fadd_rn(cs, __fsub_rn(vbx[k + 2 * R], vbx[k - 1]));
-                    float r = __fsub_rn(div_gnorm<true>(gs, c), div_kk<true>(cs, c));
+                    if (kInt) {
+                        if (k == 0) cs = Tree<2 * R + 1>::sum(vbx);
+                        else cs = __fadd_rn(cs, __fsub_rn(vbx[k + 2 * R], vbx[k - 1]));
+                    } else {
+                        cs = 0.0f;
+#pragma unroll
+                        for (int i = 0; i <= 2 * R; i++) cs = __fadd_rn(cs, vbx[k + i]);
+                    }
+                    if (!kInt && FAST) plain |= outside_fast_div(gs) || outside_fast_div(cs);
+                    if (!kInt) plain |= edge_rows && gs == 0.0f;
+                    float r = __fsub_rn(const_div<FAST>(gs, c.gnorm, c.zh_g, c.zl_g),
+                                        const_div<FAST>(cs, c.kk, c.zh_k, c.zl_k));
                     if (c.truncate && r < trunc_thr) r = 0.0f;
                     const float v = (col_in && q >= 0 && q < H) ? r : -INFINITY;
                     pr[(kStepRows * P + k) * PWp + pc] = v;
+                    a[KD - 1 + k] = v;
                 }
-            }
-        });
-        __syncthreads();
-
-        // ---- D: vertical maximum over KD processed rows for the step's 8
-        // dilation rows d = x0 + 8s - R - E + k, one column per thread
-        const int dbase = x0 + kStepRows * s - R - E;
-        by_phase<PER>(phase, [&](auto ph) {
-            constexpr int P = decltype(ph)::value;
-            if (tid < PWp - SH4) {
-                const int pc = tid + SH4;
-                const int vcol = tid;   // pc0-relative column
-                // output k: processed rows d + k - O .. d + k + E, ring rows
-                // 8P - (KD - 1) + k + i
-                float a[KD + kStepRows - 1];
+                if (!kInt && plain && col_in) {
+#pragma unroll 1
+                    for (int k = 0; k < kStepRows; k++) {
+                        const int q = q0 + k;
+                        float gs = 0.0f;
+                        cs = 0.0f;
+                        int rr = ((kStepRows * P - 2 * R) % RING + RING) % RING + k;
+                        if (rr >= RING) rr -= RING;
+#pragma unroll 1
+                        for (int i = 0; i <= 2 * R; i++) {
+                            const int gr = q + i - R;
+                            if (gr >= 0 && gr < H) gs = __fmaf_rn(c.taps[i], xg[rr * PWp + pc], gs);
+                            cs = __fadd_rn(cs, xb[rr * PWp + pc]);
+                            if (++rr == RING) rr = 0;
+                        }
+                        float r = __fsub_rn(ieee_div(gs, c.gnorm), ieee_div(cs, c.kk));
+                        if (c.truncate && r < trunc_thr) r = 0.0f;
+                        pr[(kStepRows * P + k) * PWp + pc] = (col_in && q >= 0 && q < H) ? r : -INFINITY;
+                    }
 #pragma unroll
-                for (int i = 0; i < KD + kStepRows - 1; i++) {
-                    const int rr = ((kStepRows * P - (KD - 1) + i) % RING + RING) % RING;
-                    a[i] = pr[rr * PWp + pc];
+                    for (int k = 0; k < kStepRows; k++) a[KD - 1 + k] = pr[(kStepRows * P + k) * PWp + pc];
                 }
-                // out k = max(a[k..6], mid = a[7..KD-1], a[KD..KD+k-1])
-                const float mid = Tree<KD - 7>::max(a + 7);
-                float sfx[7], pfx[8];
-                sfx[6] = a[6];
+                if (tid >= SH4) {
+                    const int vcol = tid - SH4;   // pc0-relative column
 #pragma unroll
-                for (int k = 5; k >= 0; k--) sfx[k] = fmaxf(a[k], sfx[k + 1]);
-                pfx[1] = a[KD];
+                    for (int i = 0; i < KD - 1; i++) {
+                        const int rr = ((kStepRows * P - (KD - 1) + i) % RING + RING) % RING;
+                        a[i] = pr[rr * PWp + pc];
+                    }
+                    // out k = max(a[k..6], mid = a[7..KD-1], a[KD..KD+k-1])
+                    const float mid = Tree<KD - 7>::max(a + 7);
+                    float sfx[7], pfx[8];
+                    sfx[6] = a[6];
 #pragma unroll
-                for (int k = 2; k < 8; k++) pfx[k] = fmaxf(pfx[k - 1], a[KD + k - 1]);
-                vb[vcol] = fmaxf(sfx[0], mid);
+                    for (int k = 5; k >= 0; k--) sfx[k] = fmaxf(a[k], sfx[k + 1]);
+                    pfx[1] = a[KD];
 #pragma unroll
-                for (int k = 1; k < 7; k++) vb[k * PWp + vcol] = fmaxf(fmaxf(sfx[k], mid), pfx[k]);
-                vb[7 * PWp + vcol] = fmaxf(mid, pfx[7]);
+                    for (int k = 2; k < 8; k++) pfx[k] = fmaxf(pfx[k - 1], a[KD + k - 1]);
+                    vb[vcol] = fmaxf(sfx[0], mid);
+#pragma unroll
+                    for (int k = 1; k < 7; k++) vb[k * PWp + vcol] = fmaxf(fmaxf(sfx[k], mid), pfx[k]);
+                    vb[7 * PWp + vcol] = fmaxf(mid, pfx[7]);
+                }
             }
         });
         __syncthreads();
@@ -767,12 +598,12 @@ __device__ __forceinline__ void ring_tile(const T* __restrict__ img, float* __re
     flush_tile_cands(tid, cbuf_n, cbuf, cand_slot, cout, cand_cap, flags);
 }
 
-// Shared memory and CTAs per SM of the strip kernels for a pixel type.
+// CTAs per SM of the strip kernels for a pixel type: float pixels at most 3 (64
+// registers; 4 with 56 ran 3-4 % slower at radius 4 and 5).
 template <typename T, int R, int KD>
 struct StripCfg {
-    static constexpr bool ring = IsIntPix<T>::value;
-    static constexpr size_t smem_floats = ring ? RingGeom<R, KD>::smem_floats : StripGeom<R, KD>::smem_floats;
-    static constexpr int min_blocks = ring ? RingGeom<R, KD>::min_blocks : StripGeom<R, KD>::min_blocks;
+    static constexpr int ring_blocks = RingGeom<R, KD>::min_blocks;
+    static constexpr int min_blocks = IsIntPix<T>::value ? ring_blocks : (ring_blocks < 3 ? ring_blocks : 3);
 };
 
 template <typename T, int R, int KD, bool FAST>
@@ -785,14 +616,9 @@ strip_kernel(const T* __restrict__ frames, int64_t frame_stride, float* __restri
     const int R0 = blockIdx.y * SH;
     // extract_max.wgsl:37: pic_std * snr * rough_snr_factor
     const float thr = c.frame_std ? __fmul_rn(__fmul_rn(c.frame_std[f], c.snr), c.rough) : c.thr;
-    if constexpr (StripCfg<T, R, KD>::ring)
-        ring_tile<T, R, KD>(frames + (size_t)f * frame_stride, processed + (size_t)f * H * W, c, H, W,
-                            blockIdx.x * kStripTW, R0, min(R0 + SH, H), vec_ok, thr, cand_count + f,
-                            cand_keys + (size_t)f * cand_cap, cand_cap, flags);
-    else
-        strip_tile<T, R, KD, FAST>(frames + (size_t)f * frame_stride, processed + (size_t)f * H * W, c, H, W,
-                                   blockIdx.x * kStripTW, R0, min(R0 + SH, H), vec_ok, thr, cand_count + f,
-                                   cand_keys + (size_t)f * cand_cap, cand_cap, flags);
+    ring_tile<T, R, KD, FAST>(frames + (size_t)f * frame_stride, processed + (size_t)f * H * W, c, H, W,
+                              blockIdx.x * kStripTW, R0, min(R0 + SH, H), vec_ok, thr, cand_count + f,
+                              cand_keys + (size_t)f * cand_cap, cand_cap, flags);
 }
 
 // Many frames of different sizes (frames of many videos) in one persistent
@@ -809,20 +635,14 @@ strip_ragged_kernel(const RaggedFrame* __restrict__ frames, const StripTask* __r
     for (int t = blockIdx.x; t < n; t += gridDim.x) {
         const StripTask tk = tasks[t];
         const RaggedFrame d = frames[tk.slot];
-        if constexpr (StripCfg<T, R, KD>::ring)
-            ring_tile<T, R, KD>((const T*)d.raw, processed + d.proc_off, c, d.H, d.W, tk.c0, tk.r0, tk.r1,
-                                d.vec_ok, c.thr, cand_count + tk.slot, cand_keys + (size_t)tk.slot * cand_cap,
-                                cand_cap, flags);
-        else
-            strip_tile<T, R, KD, FAST>((const T*)d.raw, processed + d.proc_off, c, d.H, d.W, tk.c0, tk.r0, tk.r1,
-                                       d.vec_ok, c.thr, cand_count + tk.slot, cand_keys + (size_t)tk.slot * cand_cap,
-                                       cand_cap, flags);
+        ring_tile<T, R, KD, FAST>((const T*)d.raw, processed + d.proc_off, c, d.H, d.W, tk.c0, tk.r0, tk.r1, d.vec_ok,
+                                  c.thr, cand_count + tk.slot, cand_keys + (size_t)tk.slot * cand_cap, cand_cap, flags);
     }
 }
 
 template <typename T, int R, int KD>
 size_t strip_smem() {
-    return StripCfg<T, R, KD>::smem_floats * sizeof(float);
+    return RingGeom<R, KD>::smem_floats * sizeof(float);
 }
 
 // Rows per segment of a launch of nx strips over nframes frames of H rows.  A
@@ -886,7 +706,7 @@ cudaError_t strip_launch(const T* frames, int64_t frame_stride, float* processed
     X(2, 8) X(3, 11) X(4, 12) X(4, 14) X(5, 15) X(5, 16) X(6, 18) X(6, 19) X(7, 21) X(7, 22)
 
 // Integer pixels use the proven constant division (fast_div) and fall back to
-// the tile kernel when it is not proven; float pixels use IEEE division.
+// the tile kernel when it is not proven; float pixels then use IEEE division.
 template <typename T>
 bool launch_strip(const T* frames, int64_t frame_stride, float* processed, const LocateConsts& c, int nframes,
                   uint32_t* cand_count, uint32_t* cand_keys, uint32_t cand_cap, uint32_t* flags, cudaStream_t st,
@@ -895,8 +715,11 @@ bool launch_strip(const T* frames, int64_t frame_stride, float* processed, const
     if (kInt && !c.fast_div) return false;
 #define GT_STRIP_TRY(RR, KK)                                                                              \
     if (c.R == RR && c.kd == KK) {                                                                       \
-        *err = strip_launch<T, RR, KK, kInt>(frames, frame_stride, processed, c, nframes, cand_count,     \
-                                             cand_keys, cand_cap, flags, st);                             \
+        *err = (kInt || c.fast_div)                                                                       \
+                   ? strip_launch<T, RR, KK, true>(frames, frame_stride, processed, c, nframes, cand_count, \
+                                                   cand_keys, cand_cap, flags, st)                        \
+                   : strip_launch<T, RR, KK, kInt>(frames, frame_stride, processed, c, nframes, cand_count, \
+                                                   cand_keys, cand_cap, flags, st);                       \
         return true;                                                                                     \
     }
     GT_STRIP_CASES(GT_STRIP_TRY)
@@ -925,8 +748,11 @@ bool launch_strip_ragged(const RaggedFrame* frames, const StripTask* tasks, cons
     if (kInt && !c.fast_div) return false;
 #define GT_STRIP_TRY(RR, KK)                                                                                  \
     if (c.R == RR && c.kd == KK) {                                                                           \
-        *err = strip_ragged_launch<T, RR, KK, kInt>(frames, tasks, ntasks, grid, processed, c, cand_count,   \
-                                                    cand_keys, cand_cap, flags, st);                         \
+        *err = (kInt || c.fast_div)                                                                          \
+                   ? strip_ragged_launch<T, RR, KK, true>(frames, tasks, ntasks, grid, processed, c, cand_count, \
+                                                          cand_keys, cand_cap, flags, st)                    \
+                   : strip_ragged_launch<T, RR, KK, kInt>(frames, tasks, ntasks, grid, processed, c, cand_count, \
+                                                          cand_keys, cand_cap, flags, st);                   \
         return true;                                                                                         \
     }
     GT_STRIP_CASES(GT_STRIP_TRY)
@@ -976,8 +802,11 @@ bool launch_strip_processed(const T* frames, int64_t frame_stride, float* proces
     cb.thr = 0.0f;
 #define GT_STRIP_PROC_TRY(RR)                                                                                  \
     if (c.R == RR) {                                                                                           \
-        *err = strip_launch<T, RR, kStripProcKD, kInt>(frames, frame_stride, processed, cb, nframes, cand_count, \
-                                                       cand_keys, 0, flags, st);                               \
+        *err = (kInt || c.fast_div)                                                                            \
+                   ? strip_launch<T, RR, kStripProcKD, true>(frames, frame_stride, processed, cb, nframes,     \
+                                                             cand_count, cand_keys, 0, flags, st)              \
+                   : strip_launch<T, RR, kStripProcKD, kInt>(frames, frame_stride, processed, cb, nframes,     \
+                                                             cand_count, cand_keys, 0, flags, st);             \
         return true;                                                                                           \
     }
     GT_STRIP_PROC_CASES(GT_STRIP_PROC_TRY)
