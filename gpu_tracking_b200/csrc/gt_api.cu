@@ -633,7 +633,8 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
     CKS(upload(ctx, ctx->tabs_s, dn));
     CKS(upload(ctx, ctx->tabs_m, dmeta));
     // LoG tables
-    DBuf ltg, ltd, loff, lrint, lng, lnd, lrad;
+    DBuf &ltg = ctx->log_tab[0], &ltd = ctx->log_tab[1], &loff = ctx->log_tab[2], &lrint = ctx->log_tab[3],
+         &lng = ctx->log_tab[4], &lnd = ctx->log_tab[5], &lrad = ctx->log_tab[6];
     if (log_style) {
         CKS(upload(ctx, ltg, lt->taps_g));
         CKS(upload(ctx, ltd, lt->taps_d));
@@ -1210,6 +1211,7 @@ gt_status charpoints_impl(gt_ctx* ctx, const gt_params& p0, const T* frames, boo
     }
     LocateConsts c;
     CKS(make_locate_consts(ctx, p, H, W, c));
+    set_fast_div<T>(ctx, c);
     if (bandpass_smem_bytes(c.R, 1, false) > 227 * 1024)
         return set_err(ctx, GT_ERR_INVALID_ARGUMENT, "smoothing_size too large for the tile kernel");
     const size_t npx = (size_t)H * W;
@@ -1217,7 +1219,6 @@ gt_status charpoints_impl(gt_ctx* ctx, const gt_params& p0, const T* frames, boo
     const uint32_t feat_cap = (uint32_t)std::max<int64_t>(maxg, 1);
     if (feat_cap >= (1u << 24)) return set_err(ctx, GT_ERR_CAPACITY_EXCEEDED, "too many points in one frame");
     CK(ctx->processed.ensure((size_t)F * npx * 4));
-    CK(ctx->stage[0].ensure((size_t)F * npx * sizeof(T)));
     CK(ctx->feats_raw.ensure((size_t)F * feat_cap * sizeof(Feature)));
     CK(ctx->feat_count.ensure((size_t)F * 4));
     CK(ctx->feats_out.ensure((size_t)G * feat_cap * sizeof(Feature)));
@@ -1231,7 +1232,8 @@ gt_status charpoints_impl(gt_ctx* ctx, const gt_params& p0, const T* frames, boo
         fin_per_frame = (np2 * 17 + 255) & ~(size_t)255;
     }
     CK(ctx->fin_scratch.ensure(std::max<size_t>(fin_per_frame * F, 256)));
-    DBuf dpts, dgoff, dgloc;
+    DBuf &dpts = ctx->cp_pts, &dgoff = ctx->cp_goff, &dgloc = ctx->cp_gloc;
+    CK(ctx->cand_count.ensure((size_t)F * 4));
     CKS(upload(ctx, dpts, pts));
     CKS(upload(ctx, dgoff, goff));
     std::vector<int32_t> gloc(G);
@@ -1264,14 +1266,34 @@ gt_status charpoints_impl(gt_ctx* ctx, const gt_params& p0, const T* frames, boo
     for (int64_t g0 = 0; g0 < G; g0 += F) {
         if (interrupted(ctx)) return set_err(ctx, GT_ERR_INTERRUPTED, "Keyboard Interrupt, my custom version");
         const int ng = (int)std::min<int64_t>(F, G - g0);
-        T* stage = ctx->stage[0].as<T>();
-        for (int g = 0; g < ng; g++)
-            CK(cudaMemcpyAsync(stage + (size_t)g * npx, frames + (size_t)gframe[g0 + g] * npx, npx * sizeof(T),
-                               on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->st));
+        // the chunk's frames: a run of frames in device memory is read in place
+        bool run = true;
+        for (int g = 1; g < ng; g++) run = run && gframe[g0 + g] == gframe[g0] + g;
+        const T* stage = frames + (size_t)gframe[g0] * npx;
+        if (!on_device || !run) {
+            CK(ctx->stage[0].ensure((size_t)F * npx * sizeof(T)));
+            T* const dst = ctx->stage[0].as<T>();
+            if (run) {
+                CK(upload_host(ctx->device, dst, stage, (size_t)ng * npx * sizeof(T), ctx->st));
+            } else {
+                for (int g = 0; g < ng; g++)
+                    CK(cudaMemcpyAsync(dst + (size_t)g * npx, frames + (size_t)gframe[g0 + g] * npx, npx * sizeof(T),
+                                       on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->st));
+            }
+            stage = dst;
+        }
         CK(cudaMemsetAsync(ctx->feat_count.p, 0, (size_t)ng * 4, ctx->st));
         Prof pf1(ctx, "bandpass");
-        CK(launch_bandpass<T>(stage, (int64_t)npx, ctx->processed.as<float>(), c, ng, false, nullptr, nullptr, 0,
-                              ctx->flags.as<uint32_t>(), ctx->st));
+        // the strip kernel where it covers the smoothing radius (1024^2 u16,
+        // radius 5: 8.5 us a frame), the tile kernel otherwise (14.1)
+        cudaError_t es = cudaSuccess;
+        if (launch_strip_processed<T>(stage, (int64_t)npx, ctx->processed.as<float>(), c, ng,
+                                      ctx->cand_count.as<uint32_t>(), nullptr, ctx->flags.as<uint32_t>(), ctx->st, &es)) {
+            CK(es);
+        } else {
+            CK(launch_bandpass<T>(stage, (int64_t)npx, ctx->processed.as<float>(), c, ng, false, nullptr, nullptr, 0,
+                                  ctx->flags.as<uint32_t>(), ctx->st));
+        }
         Prof pf2(ctx, "characterize_points");
         CK(launch_characterize_points<T>(ctx->processed.as<float>(), stage, (int64_t)npx, c, dpts.as<float>(),
                                          dgoff.as<int64_t>(), dgloc.as<int32_t>(), (int32_t)g0, ng, maxg,
