@@ -560,6 +560,7 @@ gt_status illumination_setup(gt_ctx* ctx, const gt_params& p, const T* frames, b
     }
     CKS(upload(ctx, ctx->illum_taps, taps));
     ctx->illum_rint = rint;
+    CK(ctx->illum_norm.ensure((size_t)std::max(H, W) * 4));
     if (!p.illumination_correction_per_frame) {
         const size_t npx = (size_t)H * W;
         CK(ctx->illum_shared.ensure(npx * 4));
@@ -567,10 +568,10 @@ gt_status illumination_setup(gt_ctx* ctx, const gt_params& p, const T* frames, b
         float* mean = ctx->illum_shared.as<float>();
         CKS(mean_device<T>(ctx, frames, on_device, NT, H, W, mean));
         float* tmp = ctx->illum_prof.as<float>();
-        CK(launch_illum_smooth<float>(mean, (int64_t)npx, tmp, H, W, 0, ctx->illum_taps.as<float>(), rint, 1,
-                                      ctx->st));
-        CK(launch_illum_smooth<float>(tmp, (int64_t)npx, mean, H, W, 1, ctx->illum_taps.as<float>(), rint, 1,
-                                      ctx->st));
+        CK(launch_illum_smooth<float>(mean, (int64_t)npx, tmp, H, W, 0, ctx->illum_taps.as<float>(), rint,
+                                      ctx->illum_norm.as<float>(), 1, ctx->st));
+        CK(launch_illum_smooth<float>(tmp, (int64_t)npx, mean, H, W, 1, ctx->illum_taps.as<float>(), rint,
+                                      ctx->illum_norm.as<float>(), 1, ctx->st));
     }
     return GT_OK;
 }
@@ -880,9 +881,9 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
                     // the profile of each frame is the frame itself, smoothed
                     float* prof = ctx->illum_prof.as<float>();
                     CK(launch_illum_smooth<T>(csrc, (int64_t)npx, corr, H, W, 0, ctx->illum_taps.as<float>(),
-                                              illum_rint, nf, ctx->st));
+                                              illum_rint, ctx->illum_norm.as<float>(), nf, ctx->st));
                     CK(launch_illum_smooth<float>(corr, (int64_t)npx, prof, H, W, 1, ctx->illum_taps.as<float>(),
-                                                  illum_rint, nf, ctx->st));
+                                                  illum_rint, ctx->illum_norm.as<float>(), nf, ctx->st));
                     CK(launch_illum_divide<T>(csrc, (int64_t)npx, prof, (int64_t)npx, corr, (int64_t)npx, nf,
                                               ctx->st));
                 } else {

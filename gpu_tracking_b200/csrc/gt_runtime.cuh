@@ -155,7 +155,7 @@ struct gt_ctx {
         l_dur, l_flags, l_goff, l_pgroup, l_vgrp, l_reset, l_vpoff, l_px, l_py, l_rows, l_ge, l_rowdur, l_part;
     // windowed linking inside gt_batch (slot mode)
     DBuf fstd, std_scratch, amask, astatus, acount;   // snr / minmass_snr / adaptive_background
-    DBuf illum_taps, illum_shared, illum_prof, illum_corr;  // illumination correction
+    DBuf illum_taps, illum_shared, illum_prof, illum_corr, illum_norm;  // illumination correction
     DBuf cnn_x, cnn_p, cnn_q, cnn_head;   // learned proposals: network input, activations, outputs
     DBuf walk_starts;                     // walk starts of the current call (u64)
     DBuf vd_src, vd_dec, vd_blk, vd_bad;  // video files decoded on the device: streams, bytes, blocks, flag
