@@ -46,13 +46,38 @@ gt_status fail(gt_ctx* ctx, gt_status st, const std::string& msg) {
             return fail(ctx, GT_ERR_CUDA, std::string("CUDA error ") + cudaGetErrorString(e_) + " at " #expr); \
     } while (0)
 
-// Device buffers of one call, freed on every exit path.
+// Device buffers of one call, freed on every exit path.  With `keep` (a list of
+// buffers that outlives the call) the k-th request takes the k-th buffer of
+// the list where it is large enough, and the call's buffers stay there for the
+// next one unless they hold more than kScratchKeep bytes together.
+constexpr size_t kScratchKeep = (size_t)512 << 20;
 struct Scratch {
-    std::vector<void*> ptrs;
+    std::vector<ScratchBuf> bufs;
+    std::vector<ScratchBuf>* keep;
+    cudaStream_t stream;   // what runs on the buffers
+    explicit Scratch(std::vector<ScratchBuf>* k = nullptr, cudaStream_t st = nullptr) : keep(k), stream(st) {}
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
     cudaError_t get(void** p, size_t bytes) {
         *p = nullptr;
-        cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 256));
-        if (e == cudaSuccess) ptrs.push_back(*p);
+        const size_t at = bufs.size();
+        if (keep && at < keep->size()) {
+            ScratchBuf& b = (*keep)[at];
+            if (b.bytes >= bytes) {
+                bufs.push_back(b);
+                b = ScratchBuf();
+                *p = bufs.back().p;
+                return cudaSuccess;
+            }
+            if (b.p) cudaFree(b.p);
+            b = ScratchBuf();
+        }
+        ScratchBuf n;
+        n.bytes = std::max<size_t>(bytes, 256);
+        cudaError_t e = cudaMalloc(&n.p, n.bytes);
+        if (e != cudaSuccess) return e;
+        bufs.push_back(n);
+        *p = n.p;
         return e;
     }
     template <class T>
@@ -60,7 +85,18 @@ struct Scratch {
         return get((void**)p, bytes);
     }
     ~Scratch() {
-        for (void* p : ptrs) cudaFree(p);
+        if (keep) cudaStreamSynchronize(stream);   // a call that failed may have left work behind
+        size_t total = 0;
+        for (const ScratchBuf& b : bufs) total += b.bytes;
+        if (keep && total <= kScratchKeep) {
+            for (size_t i = 0; i < bufs.size(); i++) {
+                if (i >= keep->size()) keep->resize(i + 1);
+                if ((*keep)[i].p) cudaFree((*keep)[i].p);
+                (*keep)[i] = bufs[i];
+            }
+            return;
+        }
+        for (const ScratchBuf& b : bufs) cudaFree(b.p);
     }
 };
 
@@ -256,6 +292,7 @@ GT_API void gt_proposal_destroy(gt_proposal* p) {
     cudaSetDevice(p->device);
     for (void* q : {(void*)p->params, (void*)p->adam_m, (void*)p->adam_v, (void*)p->grad, (void*)p->packed})
         if (q) cudaFree(q);
+    for (const ScratchBuf& b : p->scratch) cudaFree(b.p);
     cudaSetDevice(cur);
     delete p;
 }
@@ -312,7 +349,7 @@ GT_API gt_status gt_proposal_train(gt_ctx* ctx, gt_proposal* p, const void* fram
     cudaStream_t st = gt__ctx_stream(ctx);
     const int sms = num_sms(p->device);
     const int Hc = (H + 3) / 4, Wc = (W + 3) / 4, CH = o.crop / 4, CW = o.crop / 4;
-    Scratch s;
+    Scratch s(&p->scratch, st);
     const void* dframes = nullptr;
     {
         gt_status r = device_frames(ctx, s, frames, dtype, T, H, W, &dframes, st);

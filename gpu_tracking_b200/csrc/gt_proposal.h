@@ -2,7 +2,15 @@
 // gt_proposal handle (device parameters, Adam state, packed UMMA operands).
 #pragma once
 
+#include <vector>
+
 #include "gt_kernels.h"
+
+// One device buffer of a call's working memory.
+struct ScratchBuf {
+    void* p = nullptr;
+    size_t bytes = 0;
+};
 
 struct gt_proposal {
     int device = 0;
@@ -18,6 +26,7 @@ struct gt_proposal {
     size_t off_f[gt::kCnnLayers] = {};
     size_t off_d[gt::kCnnLayers] = {};
     size_t packed_bytes = 0;
+    std::vector<ScratchBuf> scratch;   // training's working memory, kept between calls
 
     gt::CnnNet views() const {
         gt::CnnNet n;
