@@ -249,7 +249,7 @@ struct LogTables {
     int max_rint = 0;
     // the scale space runs as one fused kernel (gt_logss.cu) when its tiles
     // fit; otherwise as a plane per radius plus a maxima pass
-    bool fused() const { return log_scale_space_supported(max_rint, (int)taps_g.size()); }
+    bool fused() const { return log_scale_space_supported(max_rint); }
 };
 
 // separable_log.wgsl:27-76 tap values, computed per radius with sigma = r / sqrt(2)
@@ -635,8 +635,16 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
     CKS(upload(ctx, ctx->tabs_m, dmeta));
     // LoG tables
     DBuf &ltg = ctx->log_tab[0], &ltd = ctx->log_tab[1], &loff = ctx->log_tab[2], &lrint = ctx->log_tab[3],
-         &lng = ctx->log_tab[4], &lnd = ctx->log_tab[5], &lrad = ctx->log_tab[6];
+         &lng = ctx->log_tab[4], &lnd = ctx->log_tab[5], &lrad = ctx->log_tab[6], &ldg = ctx->log_tab[7],
+         &lgd = ctx->log_tab[8];
+    std::vector<float2> taps_dg, taps_gd;
     if (log_style) {
+        for (size_t i = 0; i < lt->taps_g.size(); i++) {
+            taps_dg.push_back(make_float2(lt->taps_d[i], lt->taps_g[i]));
+            taps_gd.push_back(make_float2(lt->taps_g[i], lt->taps_d[i]));
+        }
+        CKS(upload(ctx, ldg, taps_dg));
+        CKS(upload(ctx, lgd, taps_gd));
         CKS(upload(ctx, ltg, lt->taps_g));
         CKS(upload(ctx, ltd, lt->taps_d));
         CKS(upload(ctx, loff, lt->tap_off));
@@ -818,12 +826,12 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
                     }
                     if (lt->fused()) {
                         Prof pf(ctx, "log_scale_space");
-                        CK(launch_log_scale_space<TS>(src, (int64_t)npx, proc, lc, ltg.as<float>(), ltd.as<float>(),
+                        CK(launch_log_scale_space<TS>(src, (int64_t)npx, proc, lc, ldg.as<float2>(), lgd.as<float2>(),
                                                      loff.as<int32_t>(), lrint.as<int32_t>(), lng.as<float>(),
-                                                     lnd.as<float>(), lt->max_rint, (int)lt->taps_g.size(), nf,
+                                                     lnd.as<float>(), lt->max_rint, nf,
                                                      ctx->cand_count.as<uint32_t>(), ctx->cand_keys.as<uint32_t>(),
-                                                     cand_cap, flags, lt->taps_g.data(), lt->taps_d.data(),
-                                                     lt->tap_off.data(), lt->rints.data(), ctx->st));
+                                                     cand_cap, flags, taps_dg.data(), lt->tap_off.data(),
+                                                     lt->rints.data(), ctx->st));
                     } else {
                         {
                             Prof pf(ctx, "laplace");

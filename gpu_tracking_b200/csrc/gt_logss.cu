@@ -1,6 +1,6 @@
 // gt_logss.cu — fused multi-scale LoG scale space for sm_100a.
 //
-// One CTA owns a 16 x 128 output tile of one frame and computes, radius by
+// One CTA owns a 34 x 128 output tile of one frame and computes, radius by
 // radius, the Laplacian-of-Gaussian plane of every scale (separable_log.wgsl
 // as driven by Laplace<2>, src/utils.rs:252-296) and the 3x3x3 scale-space
 // maximum test (logspace_max.wgsl:97-154) without writing a plane to memory:
@@ -18,6 +18,13 @@
 //              centre) k-2 and k, strict, and appended to the candidate list
 //              of (frame, radius k-1).
 //
+// Scale space of 64 frames of 1024^2 float32 on a B200, us a frame: radii 2-8
+// (10) 137.7 with unpacked chains, 16-row tiles at two CTAs per SM and a maxima
+// test that looked at up to 26 neighbours a pixel; 125.0 with packed chains and
+// 34-row tiles; 98.8 with the maxima stage below (radii 2-5 (7): 93.6 -> 68.0).
+// 16-row tiles with both: 108.2.  Issue slots are 42 % used: what remains is
+// barriers between the stages and dependent issue at 16 warps a SM.
+//
 // Every sum is the reference's sequential fused multiply-add chain in tap
 // order, so the planes equal the reference's wherever the reference's result
 // is not a zero: taps that fall outside the frame read the zero padding
@@ -34,8 +41,9 @@ namespace gt {
 
 namespace {
 
-constexpr int kSSTH = 16, kSSTW = 128, kSSThreads = 256;
-constexpr int kSSCB = 10;                // pass B columns per task ((TW + 2) = 13 * 10: one round of 234 tasks)
+constexpr int kSSTH = 34, kSSTW = 128, kSSThreads = 512;
+constexpr int kSSCB = 10;                // pass B columns per task ((TW + 2) = 13 * 10: one round of 468 tasks)
+constexpr int kSSMaxRows = 9;            // rows a thread tests in the maxima stage
 constexpr int kSSBatch = 8;              // raw-tile loads a thread keeps in flight
 static_assert((kSSTW + 2) % kSSCB == 0, "pass B column blocks");
 constexpr int kSSPW = kSSTW + 2;         // plane tile width (tile +- 1)
@@ -44,32 +52,35 @@ constexpr int kSSPH = kSSTH + 2;
 // radius, so the vertical pass's tap loads are constant offsets
 constexpr int kSSRW = kSSPW + 2 * kLogSSMaxR;
 
-// Tap weights of every compile-time radius R (= rint) at offset R * R (radii
+// The two chains of a pass run as the halves of packed FP32 multiply-adds (each
+// half a separately rounded IEEE operation): pass A multiplies one pixel by the
+// pair (second-derivative tap, Gaussian tap), pass B the pair (a, b) of a
+// column by (Gaussian tap, second-derivative tap), so the pass A planes hold
+// pairs and half the multiply-adds are issued.
+//
+// Tap pairs of every compile-time radius R (= rint) at offset R * R (radii
 // 0 .. R-1 take sum(2r + 1) = R^2 slots), passed as a kernel parameter: a tap
-// chain then reads its weights as constant-bank operands instead of one
-// shared-memory load per tap.  Usable when the radii of a call have distinct
-// rints (the host falls back to shared-memory taps otherwise).
+// chain then reads its weights as constant-bank operands.  Usable when the
+// radii of a call have distinct rints (else the pairs come from global memory).
 constexpr int kSSParamTaps = (kLogSSMaxR + 1) * (kLogSSMaxR + 1);
 struct SSTaps {
-    float g[kSSParamTaps];
-    float d[kSSParamTaps];
+    float2 dg[kSSParamTaps];
+    float2 gd[kSSParamTaps];
 };
 
 struct SSGeom {
     int RMAX, RH, RW;   // raw tile: RH rows of RW used columns (row stride kSSRW, as the pass A planes)
-    size_t off_a, off_b, off_ring, off_taps, floats;
+    size_t off_ab, off_ring, floats;
 };
 
-__host__ __device__ inline SSGeom ss_geom(int rmax, int ntaps_total) {
+__host__ __device__ inline SSGeom ss_geom(int rmax) {
     SSGeom g;
     g.RMAX = rmax;
     g.RH = kSSPH + 2 * rmax;
     g.RW = kSSPW + 2 * rmax;
-    g.off_a = (size_t)g.RH * kSSRW;
-    g.off_b = g.off_a + (size_t)kSSPH * kSSRW;
-    g.off_ring = g.off_b + (size_t)kSSPH * kSSRW;
-    g.off_taps = g.off_ring + 3 * (size_t)kSSPH * kSSPW;
-    g.floats = g.off_taps + 2 * (size_t)ntaps_total;
+    g.off_ab = (size_t)g.RH * kSSRW;
+    g.off_ring = g.off_ab + 2 * (size_t)kSSPH * kSSRW;
+    g.floats = g.off_ring + 3 * (size_t)kSSPH * kSSPW;
     return g;
 }
 
@@ -90,33 +101,33 @@ struct SSRows {
     static constexpr int C = kSSPW + 2 * R;
     static constexpr int rounds(int rg) { return ((kSSPH / rg) * C + kSSThreads - 1) / kSSThreads * rg; }
     static constexpr int pick() {
-        int best = 9;
-        for (int rg : {6, 3, 2})
+        int best = 18;
+        for (int rg : {12, 9, 6})
             if (rounds(rg) < rounds(best)) best = rg;
         return best;
     }
     static constexpr int value = pick();
-    static_assert(kSSPH % value == 0, "row groups tile the plane rows");
+    static_assert(kSSPH % 18 == 0 && kSSPH % 12 == 0, "row groups tile the plane rows");
 };
 
 // pass A of one radius: column `col` of the pass A planes, rows grp*RG ..
 template <int R>
-__device__ __forceinline__ void ss_pass_a(const float* __restrict__ raw, const SSGeom& g, float* __restrict__ sa,
-                                          float* __restrict__ sb, const float* __restrict__ tg,
-                                          const float* __restrict__ td, float ng, float nd) {
+__device__ __forceinline__ void ss_pass_a(const float* __restrict__ raw, const SSGeom& g, float2* __restrict__ sab,
+                                          const float2* __restrict__ dg, float ng, float nd) {
     constexpr int NT = 2 * R + 1;
     constexpr int kSSChunk = SSChunk<R>::value;
     constexpr int kSSRG = SSRows<R>::value, NGRP = kSSPH / kSSRG;
     const int ncols = kSSPW + 2 * R;
+    const float2 nrm = make_float2(nd, ng);
     for (int task = threadIdx.x; task < NGRP * ncols; task += kSSThreads) {
         const int grp = task / ncols;
         const int col = task - grp * ncols;
         const int u0 = grp * kSSRG;
         // plane row u0 + k, column col <-> raw row u0 + k + RMAX - R + i, raw column col + RMAX - R
         const float* src = raw + (size_t)(u0 + g.RMAX - R) * kSSRW + (col + g.RMAX - R);
-        float aa[kSSRG], bb[kSSRG];
+        float2 ab[kSSRG];
 #pragma unroll
-        for (int k = 0; k < kSSRG; k++) aa[k] = bb[k] = 0.0f;
+        for (int k = 0; k < kSSRG; k++) ab[k] = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (int i0 = 0; i0 < NT; i0 += kSSChunk) {
             constexpr int NXC = kSSChunk + kSSRG - 1;
@@ -127,84 +138,69 @@ __device__ __forceinline__ void ss_pass_a(const float* __restrict__ raw, const S
 #pragma unroll
             for (int ii = 0; ii < kSSChunk; ii++) {
                 if (i0 + ii < NT) {
-                    const float d = td[i0 + ii], gg = tg[i0 + ii];
+                    const float2 t = dg[i0 + ii];
 #pragma unroll
-                    for (int k = 0; k < kSSRG; k++) {
-                        aa[k] = __fmaf_rn(d, x[k + ii], aa[k]);
-                        bb[k] = __fmaf_rn(gg, x[k + ii], bb[k]);
-                    }
+                    for (int k = 0; k < kSSRG; k++)
+                        ab[k] = __ffma2_rn(t, make_float2(x[k + ii], x[k + ii]), ab[k]);
                 }
             }
         }
 #pragma unroll
-        for (int k = 0; k < kSSRG; k++) {
-            sa[(u0 + k) * kSSRW + col] = __fmul_rn(aa[k], nd);
-            sb[(u0 + k) * kSSRW + col] = __fmul_rn(bb[k], ng);
-        }
-    }
-}
-
-// one horizontal chain block: acc[c] = sum_j t_j p[c + j], j = 0 .. NT-1 in order
-template <int R>
-__device__ __forceinline__ void ss_hchain(const float* __restrict__ p, const float* __restrict__ t, float* acc) {
-    constexpr int NT = 2 * R + 1;
-    constexpr int kSSChunk = SSChunk<R>::value;
-#pragma unroll
-    for (int c = 0; c < kSSCB; c++) acc[c] = 0.0f;
-#pragma unroll
-    for (int j0 = 0; j0 < NT; j0 += kSSChunk) {
-        // the window is read in 8-byte pairs (p + j0 is 8-byte aligned: even
-        // row stride, even task column, even chunk); a pair's second value
-        // past the window is a loaded but unused float of the same tile row
-        // or the next one
-        constexpr int NXC = kSSChunk + kSSCB - 1;
-        float x[NXC + 1];
-#pragma unroll
-        for (int m = 0; m < NXC; m += 2)
-            if (j0 + m < NT + kSSCB - 1) {
-                const float2 v2 = *reinterpret_cast<const float2*>(p + j0 + m);
-                x[m] = v2.x;
-                x[m + 1] = v2.y;
-            }
-#pragma unroll
-        for (int jj = 0; jj < kSSChunk; jj++) {
-            if (j0 + jj < NT) {
-                const float tv = t[j0 + jj];
-#pragma unroll
-                for (int c = 0; c < kSSCB; c++) acc[c] = __fmaf_rn(tv, x[c + jj], acc[c]);
-            }
-        }
+        for (int k = 0; k < kSSRG; k++) sab[(u0 + k) * kSSRW + col] = __fmul2_rn(ab[k], nrm);
     }
 }
 
 // pass B of one radius: row u, columns cb*CB .. of the plane tile
 template <int R>
-__device__ __forceinline__ void ss_pass_b(const float* __restrict__ sa, const float* __restrict__ sb,
-                                          const SSGeom& g, float* __restrict__ plane, const float* __restrict__ tg,
-                                          const float* __restrict__ td, float ng, float nd) {
-    constexpr int NB = kSSPW / kSSCB;
+__device__ __forceinline__ void ss_pass_b(const float2* __restrict__ sab, float* __restrict__ plane,
+                                          const float2* __restrict__ gd, float ng, float nd) {
+    constexpr int NB = kSSPW / kSSCB, NT = 2 * R + 1;
+    constexpr int kSSChunk = SSChunk<R>::value;
     for (int task = threadIdx.x; task < kSSPH * NB; task += kSSThreads) {
         const int u = task / NB;
         const int v0 = (task - u * NB) * kSSCB;
-        // plane column v, tap j <-> pass A column v + j
-        float ra[kSSCB], rb[kSSCB];
-        ss_hchain<R>(sa + (size_t)u * kSSRW + v0, tg, ra);
-        ss_hchain<R>(sb + (size_t)u * kSSRW + v0, td, rb);
+        // plane column v, tap j <-> pass A column v + j; two pairs a load
+        // (even row stride, task column and chunk; the second one past the
+        // window is a loaded but unused pair of the tile)
+        const float2* p = sab + (size_t)u * kSSRW + v0;
+        float2 acc[kSSCB];
+#pragma unroll
+        for (int c = 0; c < kSSCB; c++) acc[c] = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int j0 = 0; j0 < NT; j0 += kSSChunk) {
+            constexpr int NXC = kSSChunk + kSSCB - 1;
+            float2 x[NXC + 1];
+#pragma unroll
+            for (int m = 0; m < NXC; m += 2)
+                if (j0 + m < NT + kSSCB - 1) {
+                    const float4 v4 = *reinterpret_cast<const float4*>(p + j0 + m);
+                    x[m] = make_float2(v4.x, v4.y);
+                    x[m + 1] = make_float2(v4.z, v4.w);
+                }
+#pragma unroll
+            for (int jj = 0; jj < kSSChunk; jj++) {
+                if (j0 + jj < NT) {
+                    const float2 t = gd[j0 + jj];
+#pragma unroll
+                    for (int c = 0; c < kSSCB; c++) acc[c] = __ffma2_rn(t, x[c + jj], acc[c]);
+                }
+            }
+        }
 #pragma unroll
         for (int c = 0; c < kSSCB; c++) {
-            float L = __fsub_rn(0.0f, __fmul_rn(ra[c], ng));
-            L = __fsub_rn(L, __fmul_rn(rb[c], nd));
+            float L = __fsub_rn(0.0f, __fmul_rn(acc[c].x, ng));
+            L = __fsub_rn(L, __fmul_rn(acc[c].y, nd));
             plane[u * kSSPW + v0 + c] = L;
         }
     }
 }
 
 template <int R>
-__device__ void ss_radius(const float* raw, const SSGeom& g, float* sa, float* sb, float* plane, const float* tg,
-                          const float* td, float ng, float nd) {
-    ss_pass_a<R>(raw, g, sa, sb, tg, td, ng, nd);
+__device__ void ss_radius(const float* raw, const SSGeom& g, float2* sab, float* plane, const float2* dg,
+                          const float2* gd, float ng, float nd) {
+    ss_pass_a<R>(raw, g, sab, dg, ng, nd);
     __syncthreads();
-    ss_pass_b<R>(sa, sb, g, plane, tg, td, ng, nd);
+    ss_pass_b<R>(sab, plane, gd, ng, nd);
 }
 
 #define GT_SS_CASES(X)                                                                                    \
@@ -235,59 +231,78 @@ __device__ void ss_maxima(const float* __restrict__ ring, int km, int n, int f, 
     const float thr = lc.frame_std ? __fmul_rn(__fmul_rn(lc.frame_std[f], lc.snr), lc.rough) : lc.thr;
     const size_t slot = (size_t)f * n + km;
     uint32_t* keys = cand_keys + slot * cand_cap;
-    for (int e0 = 0; e0 < kSSTH * kSSTW; e0 += kSSThreads) {
-        const int e = e0 + threadIdx.x;
-        const int u = e / kSSTW + 1, v = e % kSSTW + 1;
-        const int gi = r0 + u - 1, gj = c0 + v - 1;
-        bool is = false;
-        if (gi > 0 && gi < H - 1 && gj > 0 && gj < W - 1) {
-            const float center = mid[u * kSSPW + v];
-            if (center > 0.0f && ss_max_in_plane(mid, u, v, center) && (!bot || ss_max_in_plane(bot, u, v, center)) &&
-                (!top || ss_max_in_plane(top, u, v, center)))
-                is = !(__ldg(proc + (size_t)gi * W + gj) < thr);
-        }
-        const unsigned ball = __ballot_sync(0xffffffffu, is);
-        if (ball) {
-            const int lane = threadIdx.x & 31;
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(cand_count + slot, (uint32_t)__popc(ball));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (is) {
-                const uint32_t q = base + __popc(ball & ((1u << lane) - 1u));
-                if (q < cand_cap) keys[q] = (uint32_t)gi * (uint32_t)W + (uint32_t)gj;
-                else atomicOr(flags, kFlagCandOverflow);
+    // A thread walks kSSMaxRows rows of one column: the largest of the three
+    // values a row has around the column serves the pixels above and below it,
+    // so the own plane's eight neighbours cost three loads and five maxima a
+    // pixel (a NaN among them drops out of a maximum as it fails every >=).
+    // The few pixels above them all look at the planes beside.
+    constexpr int NSTRIP = (kSSTH + kSSMaxRows - 1) / kSSMaxRows;
+    for (int t0 = 0; t0 < NSTRIP * kSSTW; t0 += kSSThreads) {
+        const int t = t0 + threadIdx.x;   // whole warps take a strip's columns
+        const int v = t % kSSTW + 1, ua = t / kSSTW * kSSMaxRows + 1;
+        const int gj = c0 + v - 1;
+        const bool col_in = t < NSTRIP * kSSTW && gj > 0 && gj < W - 1;
+        const float* p = mid + (col_in ? (ua - 1) * kSSPW + v : kSSPW + 1);
+        float wc, ec, cc;                     // west, east and centre of the current row
+        float above = fmaxf(fmaxf(p[-1], p[0]), p[1]);
+        wc = p[kSSPW - 1];
+        cc = p[kSSPW];
+        ec = p[kSSPW + 1];
+#pragma unroll
+        for (int k = 0; k < kSSMaxRows; k++) {
+            const int u = ua + k;
+            const bool last = u + 1 >= kSSPH;   // below the plane tile: not a pixel of the tile either
+            const float* q = p + (last ? 0 : (k + 2) * kSSPW);
+            const float wn = q[-1], cn = q[0], en = q[1];
+            const float side = fmaxf(wc, ec);
+            const float below = fmaxf(fmaxf(wn, cn), en);
+            const int gi = r0 + u - 1;
+            bool is = col_in && !last && u <= kSSTH && gi > 0 && gi < H - 1 && cc > 0.0f &&
+                      !(fmaxf(fmaxf(above, below), side) >= cc);
+            if (__any_sync(0xffffffffu, is)) {
+                if (is)
+                    is = (!bot || ss_max_in_plane(bot, u, v, cc)) && (!top || ss_max_in_plane(top, u, v, cc)) &&
+                         !(__ldg(proc + (size_t)gi * W + gj) < thr);
+                const unsigned ball = __ballot_sync(0xffffffffu, is);
+                if (ball) {
+                    const int lane = threadIdx.x & 31;
+                    uint32_t base = 0;
+                    if (lane == 0) base = atomicAdd(cand_count + slot, (uint32_t)__popc(ball));
+                    base = __shfl_sync(0xffffffffu, base, 0);
+                    if (is) {
+                        const uint32_t w = base + __popc(ball & ((1u << lane) - 1u));
+                        if (w < cand_cap) keys[w] = (uint32_t)gi * (uint32_t)W + (uint32_t)gj;
+                        else atomicOr(flags, kFlagCandOverflow);
+                    }
+                }
             }
+            above = fmaxf(side, cc);
+            wc = wn;
+            cc = cn;
+            ec = en;
         }
     }
 }
 
 template <typename T, bool kPT>
-__global__ void __launch_bounds__(kSSThreads, 2)
+__global__ void __launch_bounds__(kSSThreads, 1)
 log_scale_space_kernel(const T* __restrict__ frames, int64_t frame_stride, const float* __restrict__ processed,
-                       const LogConsts lc, const float* __restrict__ taps_g, const float* __restrict__ taps_d,
+                       const LogConsts lc, const float2* __restrict__ taps_dg, const float2* __restrict__ taps_gd,
                        const int32_t* __restrict__ tap_off, const int32_t* __restrict__ rints,
-                       const float* __restrict__ norm_g, const float* __restrict__ norm_d, int rmax, int ntaps_total,
+                       const float* __restrict__ norm_g, const float* __restrict__ norm_d, int rmax,
                        uint32_t* __restrict__ cand_count, uint32_t* __restrict__ cand_keys, uint32_t cand_cap,
                        uint32_t* __restrict__ flags, const __grid_constant__ SSTaps tp) {
     extern __shared__ float4 ss_sm4[];
     float* sm = (float*)ss_sm4;
-    const SSGeom g = ss_geom(rmax, ntaps_total);
+    const SSGeom g = ss_geom(rmax);
     float* raw = sm;
-    float* sa = sm + g.off_a;
-    float* sb = sm + g.off_b;
+    float2* sab = (float2*)(sm + g.off_ab);
     float* ring = sm + g.off_ring;
-    float* stg = sm + g.off_taps;              // Gaussian taps of every radius
-    float* std_ = stg + ntaps_total;           // second-derivative taps
     const int H = lc.H, W = lc.W, n = lc.n_radii;
     const int f = blockIdx.z;
     const int r0 = blockIdx.y * kSSTH, c0 = blockIdx.x * kSSTW;
     const T* img = frames + (size_t)f * frame_stride;
     const float* proc = processed + (size_t)f * H * W;
-    if (!kPT)
-        for (int i = threadIdx.x; i < ntaps_total; i += kSSThreads) {
-            stg[i] = taps_g[i];
-            std_[i] = taps_d[i];
-        }
     // raw tile: rows r0 - 1 - RMAX .., columns c0 - 1 - RMAX .., zero outside
     // the frame; kSSBatch independent loads per thread are in flight before
     // their shared-memory stores
@@ -313,16 +328,16 @@ log_scale_space_kernel(const T* __restrict__ frames, int64_t frame_stride, const
     __syncthreads();
     for (int k = 0; k < n; k++) {
         const int R = rints[k];
-        const float* tg = stg + tap_off[k];
-        const float* td = std_ + tap_off[k];
+        const float2* dg = taps_dg + tap_off[k];
+        const float2* gd = taps_gd + tap_off[k];
         float* plane = ring + (size_t)(k % 3) * kSSPH * kSSPW;
         switch (R) {
 #define GT_SS_CASE(RR)                                                                                 \
     case RR:                                                                                           \
         if (kPT)                                                                                       \
-            ss_radius<RR>(raw, g, sa, sb, plane, tp.g + RR * RR, tp.d + RR * RR, norm_g[k], norm_d[k]); \
+            ss_radius<RR>(raw, g, sab, plane, tp.dg + RR * RR, tp.gd + RR * RR, norm_g[k], norm_d[k]); \
         else                                                                                           \
-            ss_radius<RR>(raw, g, sa, sb, plane, tg, td, norm_g[k], norm_d[k]);                        \
+            ss_radius<RR>(raw, g, sab, plane, dg, gd, norm_g[k], norm_d[k]);                           \
         break;
             GT_SS_CASES(GT_SS_CASE)
 #undef GT_SS_CASE
@@ -337,27 +352,25 @@ log_scale_space_kernel(const T* __restrict__ frames, int64_t frame_stride, const
 
 }  // namespace
 
-size_t log_scale_space_smem_bytes(int max_rint, int ntaps_total) {
-    return ss_geom(max_rint, ntaps_total).floats * sizeof(float);
-}
+size_t log_scale_space_smem_bytes(int max_rint) { return ss_geom(max_rint).floats * sizeof(float); }
 
-bool log_scale_space_supported(int max_rint, int ntaps_total) {
-    return max_rint >= 0 && max_rint <= kLogSSMaxR && log_scale_space_smem_bytes(max_rint, ntaps_total) <= 227 * 1024;
+bool log_scale_space_supported(int max_rint) {
+    return max_rint >= 0 && max_rint <= kLogSSMaxR && log_scale_space_smem_bytes(max_rint) <= 227 * 1024;
 }
 
 template <typename T>
 cudaError_t launch_log_scale_space(const T* frames, int64_t frame_stride, const float* processed, const LogConsts& lc,
-                                   const float* taps_g, const float* taps_d, const int32_t* tap_off,
+                                   const float2* taps_dg, const float2* taps_gd, const int32_t* tap_off,
                                    const int32_t* rints, const float* norm_g, const float* norm_d, int max_rint,
-                                   int ntaps_total, int nframes, uint32_t* cand_count, uint32_t* cand_keys,
-                                   uint32_t cand_cap, uint32_t* flags, const float* h_taps_g, const float* h_taps_d,
+                                   int nframes, uint32_t* cand_count, uint32_t* cand_keys,
+                                   uint32_t cand_cap, uint32_t* flags, const float2* h_taps_dg,
                                    const int32_t* h_tap_off, const int32_t* h_rints, cudaStream_t st) {
     dim3 grid((lc.W + kSSTW - 1) / kSSTW, (lc.H + kSSTH - 1) / kSSTH, nframes);
-    const size_t smem = log_scale_space_smem_bytes(max_rint, ntaps_total);
+    const size_t smem = log_scale_space_smem_bytes(max_rint);
     // taps as a kernel parameter when every radius has its own rint
     static_assert(sizeof(SSTaps) + 512 <= 32764, "kernel parameters stay within the launch limit");
     SSTaps tp;
-    bool param_taps = h_taps_g && h_taps_d && h_tap_off && h_rints;
+    bool param_taps = h_taps_dg && h_tap_off && h_rints;
     uint64_t seen[(kLogSSMaxR + 64) / 64] = {};
     for (int k = 0; param_taps && k < lc.n_radii; k++) {
         const int R = h_rints[k];
@@ -367,31 +380,32 @@ cudaError_t launch_log_scale_space(const T* frames, int64_t frame_stride, const 
         }
         seen[R / 64] |= 1ull << (R % 64);
         for (int i = 0; i < 2 * R + 1; i++) {
-            tp.g[R * R + i] = h_taps_g[h_tap_off[k] + i];
-            tp.d[R * R + i] = h_taps_d[h_tap_off[k] + i];
+            const float2 t = h_taps_dg[h_tap_off[k] + i];
+            tp.dg[R * R + i] = t;
+            tp.gd[R * R + i] = make_float2(t.y, t.x);
         }
     }
     if (param_taps) {
         cudaFuncSetAttribute(log_scale_space_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         log_scale_space_kernel<T, true><<<grid, kSSThreads, smem, st>>>(
-            frames, frame_stride, processed, lc, taps_g, taps_d, tap_off, rints, norm_g, norm_d, max_rint, ntaps_total,
+            frames, frame_stride, processed, lc, taps_dg, taps_gd, tap_off, rints, norm_g, norm_d, max_rint,
             cand_count, cand_keys, cand_cap, flags, tp);
     } else {
         cudaFuncSetAttribute(log_scale_space_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
         log_scale_space_kernel<T, false><<<grid, kSSThreads, smem, st>>>(
-            frames, frame_stride, processed, lc, taps_g, taps_d, tap_off, rints, norm_g, norm_d, max_rint, ntaps_total,
+            frames, frame_stride, processed, lc, taps_dg, taps_gd, tap_off, rints, norm_g, norm_d, max_rint,
             cand_count, cand_keys, cand_cap, flags, tp);
     }
     return cudaGetLastError();
 }
 
 #define GT_SS_INST(T)                                                                                          \
-    template cudaError_t launch_log_scale_space<T>(const T*, int64_t, const float*, const LogConsts&, const float*, \
-                                                   const float*, const int32_t*, const int32_t*, const float*,       \
-                                                   const float*, int, int, int, uint32_t*, uint32_t*, uint32_t,      \
-                                                   uint32_t*, const float*, const float*, const int32_t*,            \
-                                                   const int32_t*, cudaStream_t);
+    template cudaError_t launch_log_scale_space<T>(const T*, int64_t, const float*, const LogConsts&, const float2*, \
+                                                   const float2*, const int32_t*, const int32_t*, const float*,      \
+                                                   const float*, int, int, uint32_t*, uint32_t*, uint32_t,           \
+                                                   uint32_t*, const float2*, const int32_t*, const int32_t*,         \
+                                                   cudaStream_t);
 GT_SS_INST(uint16_t)
 GT_SS_INST(float)
 GT_SS_INST(uint8_t)

@@ -162,7 +162,7 @@ struct gt_ctx {
     int64_t last_walk_starts = 0;
     int32_t illum_rint = 0;
     DBuf w_rec, w_cells, w_geo, w_scan, w_scratch, w_ids, w_dur, w_state, w_cnt, w_flags, w_vgrp, w_reset;
-    DBuf log_tab[7];                      // LoG: taps, offsets, norms and radii of the call
+    DBuf log_tab[9];                      // LoG: taps, offsets, norms, radii and tap pairs of the call
     DBuf cp_pts, cp_goff, cp_gloc;        // characterize_points: points, group offsets, group frames
     // segments of the linker's frame loop: scratch of the speculative runs, their states, arrivals
     DBuf w_segs, w_segst, w_segarr, l_segs, l_segst, l_segarr;
