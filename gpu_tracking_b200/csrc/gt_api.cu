@@ -159,11 +159,15 @@ void set_fast_div(gt_ctx* ctx, LocateConsts& c) {
 }
 
 // (sin 2θ, cos 2θ) tables per integer radius 0..max_rint (characterize.wgsl:120-124)
+// The tables of smaller radii are the first part of those of larger ones: one
+// list for the process, grown to the largest radius asked for.
 void angle_tables(int max_rint, std::vector<float2>& tab, std::vector<int32_t>& off) {
-    tab.clear();
-    off.clear();
-    for (int r = 0; r <= max_rint; r++) {
-        off.push_back((int32_t)tab.size());
+    static std::mutex mu;
+    static std::vector<float2> all;
+    static std::vector<int32_t> starts;
+    std::lock_guard<std::mutex> lock(mu);
+    for (int r = (int)starts.size(); r <= max_rint; r++) {
+        starts.push_back((int32_t)all.size());
         for (int i = -r; i <= r; i++)
             for (int j = -r; j <= r; j++) {
                 float x = (float)i, y = (float)j;
@@ -172,9 +176,12 @@ void angle_tables(int max_rint, std::vector<float2>& tab, std::vector<int32_t>& 
                     float theta = std::atan2(y, x);
                     v = make_float2(std::sin(2.0f * theta), std::cos(2.0f * theta));
                 }
-                tab.push_back(v);
+                all.push_back(v);
             }
     }
+    const int n = std::max(max_rint + 1, 0);
+    off.assign(starts.begin(), starts.begin() + n);
+    tab.assign(all.begin(), n < (int)starts.size() ? all.begin() + starts[(size_t)n] : all.end());
 }
 
 // circle_inds / annulus_inds (src/kernels.rs:138-171)
@@ -611,11 +618,7 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
         fin_per_frame = (np2 * 17 + 255) & ~(size_t)255;
     }
     CK(ctx->fin_scratch.ensure(std::max<size_t>(fin_per_frame * SC, 256)));
-    {
-        std::vector<int32_t> ident(SC);
-        for (int i = 0; i < SC; i++) ident[i] = i;
-        CKS(upload(ctx, ctx->ident, ident));
-    }
+    CKS(ensure_ident(ctx, SC));
     // constant tables
     std::vector<float2> atab;
     std::vector<int32_t> aoff;
@@ -916,11 +919,16 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
         if (late_copy && sc + 1 < nsuper) CKS(issue_copy(sc + 1));
         ctx->done = s0 + ns;
     }
-    CK(cudaMemcpyAsync(out_flags, flags, 4, cudaMemcpyDeviceToHost, ctx->st));
-    unsigned long long starts = 0;
-    CK(cudaMemcpyAsync(&starts, ctx->walk_starts.p, 8, cudaMemcpyDeviceToHost, ctx->st));
+    // one wait for all that the call reads before it goes on
+    if (!ctx->mail) CK(cudaHostAlloc((void**)&ctx->mail, sizeof(gt_ctx::Mail), cudaHostAllocDefault));
+    ctx->mail_kept = NT <= gt_ctx::kMailCounts;
+    CK(cudaMemcpyAsync(&ctx->mail->flags, flags, 4, cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&ctx->mail->starts, ctx->walk_starts.p, 8, cudaMemcpyDeviceToHost, ctx->st));
+    if (ctx->mail_kept)
+        CK(cudaMemcpyAsync(ctx->mail->kept, ctx->kept_count.p, (size_t)NT * 4, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    ctx->last_walk_starts = (int64_t)starts;
+    *out_flags = ctx->mail->flags;
+    ctx->last_walk_starts = (int64_t)ctx->mail->starts;
     drain_profile(ctx, false);
     return GT_OK;
 }
@@ -928,10 +936,15 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
 // Assemble the output table from per-frame results (kept_count, feats_out)
 // of the NT frame slots starting at slot0.
 gt_status assemble_table(gt_ctx* ctx, int64_t NT, const std::vector<int64_t>& frame_numbers, bool log_style,
-                         gt_table* tab, std::vector<int64_t>& row_off, int64_t slot0 = 0) {
+                         gt_table* tab, std::vector<int64_t>& row_off, int64_t slot0 = 0, bool have_kept = false) {
     std::vector<uint32_t> kept(NT);
-    CK(cudaMemcpyAsync(kept.data(), ctx->kept_count.as<uint32_t>() + slot0, NT * 4, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
+    if (have_kept) {
+        kept.assign(ctx->mail->kept, ctx->mail->kept + NT);
+    } else {
+        CK(cudaMemcpyAsync(kept.data(), ctx->kept_count.as<uint32_t>() + slot0, NT * 4, cudaMemcpyDeviceToHost,
+                           ctx->st));
+        CK(cudaStreamSynchronize(ctx->st));
+    }
     row_off.assign(NT + 1, 0);
     uint32_t maxk = 0;
     for (int64_t t = 0; t < NT; t++) {
@@ -941,10 +954,18 @@ gt_status assemble_table(gt_ctx* ctx, int64_t NT, const std::vector<int64_t>& fr
     const int64_t N = row_off[NT];
     tab->n = N;
     const size_t n1 = std::max<int64_t>(N, 1);
-    CK(tab->frame.ensure(n1 * 8));
+    // every column in one allocation, particle and duration included (linking fills them)
+    const size_t c8 = (n1 * 8 + 255) & ~(size_t)255, c4 = (n1 * 4 + 255) & ~(size_t)255;
+    CK(tab->arena.ensure(3 * c8 + (GT_NUM_COLUMNS - 3) * c4));
+    uint8_t* at = tab->arena.as<uint8_t>();
+    for (TBuf* b : {&tab->frame, &tab->particle, &tab->duration}) {
+        b->part(at, c8);
+        at += c8;
+    }
     for (int c = 0; c < GT_NUM_COLUMNS; c++) {
         if (c == GT_COL_FRAME || c == GT_COL_PARTICLE || c == GT_COL_DURATION) continue;
-        CK(tab->col[c].ensure(n1 * 4));
+        tab->col[c].part(at, c4);
+        at += c4;
         tab->has[c] = true;
     }
     tab->has[GT_COL_FRAME] = true;
@@ -1068,7 +1089,7 @@ gt_status batch_impl(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_d
     std::vector<int64_t> row_off;
     {
         HostSpan hs(ctx, "host_assemble");
-        gt_status st = assemble_table(ctx, NT, fnum, log_style, tab, row_off);
+        gt_status st = assemble_table(ctx, NT, fnum, log_style, tab, row_off, 0, ctx->mail_kept);
         if (st != GT_OK) {
             sync_link_streams(ctx);
             return st;
@@ -1248,9 +1269,7 @@ gt_status charpoints_impl(gt_ctx* ctx, const gt_params& p0, const T* frames, boo
     std::vector<int32_t> gloc(G);
     for (int64_t g = 0; g < G; g++) gloc[g] = (int32_t)(g % F);
     CKS(upload(ctx, dgloc, gloc));
-    std::vector<int32_t> ident(F);
-    for (int i = 0; i < F; i++) ident[i] = i;
-    CKS(upload(ctx, ctx->ident, ident));
+    CKS(ensure_ident(ctx, F));
     std::vector<float2> atab;
     std::vector<int32_t> aoff;
     int max_rint = std::max(std::max(0, (c.circle - 1) / 2), (int)std::ceil(max_r));
@@ -1472,11 +1491,7 @@ gt_status batch_videos_ragged(gt_ctx* ctx, const gt_params& p, const LocateConst
         CK(ctx->rg_frames.ensure((size_t)kRaggedSlots * sizeof(RaggedFrame)));
         CK(ctx->rg_tasks.ensure((size_t)std::max<int64_t>(max_tasks, 1) * sizeof(StripTask)));
         CK(ctx->rg_ntasks.ensure(4));
-        {
-            std::vector<int32_t> ident(kRaggedSlots);
-            for (int i = 0; i < kRaggedSlots; i++) ident[i] = i;
-            CKS(upload(ctx, ctx->ident, ident));
-        }
+        CKS(ensure_ident(ctx, kRaggedSlots));
         CKS(upload(ctx, ctx->tabs_f, atab));
         CKS(upload(ctx, ctx->tabs_i, aoff));
         CKS(upload(ctx, ctx->tabs_s, dn));
@@ -2020,6 +2035,7 @@ void gt_destroy(gt_ctx* ctx) {
     sync_link_streams(ctx);
     drain_profile(ctx);
     for (auto e : ctx->event_pool) cudaEventDestroy(e);
+    if (ctx->mail) cudaFreeHost(ctx->mail);
     for (int i = 0; i < 2; i++) {
         if (ctx->used[i]) cudaEventDestroy(ctx->used[i]);
         if (ctx->filled[i]) cudaEventDestroy(ctx->filled[i]);

@@ -89,18 +89,26 @@ struct TBuf {
     size_t n = 0;
     int device = 0;
     cudaStream_t stream = nullptr;   // the call's compute stream
+    bool owned = true;               // false: part of another buffer
     TBuf() = default;
     TBuf(const TBuf&) = delete;
     TBuf& operator=(const TBuf&) = delete;
     // a table is freed only when no work on it is pending
     ~TBuf() {
-        if (p) cudaFreeAsync(p, cudaStreamPerThread);
+        if (p && owned) cudaFreeAsync(p, cudaStreamPerThread);
+    }
+    void part(void* at, size_t bytes) {
+        if (p && owned) cudaFreeAsync(p, stream);
+        p = at;
+        n = bytes;
+        owned = false;
     }
     cudaError_t ensure(size_t bytes) {
         if (bytes <= n && p) return cudaSuccess;
-        if (p) cudaFreeAsync(p, stream);
+        if (p && owned) cudaFreeAsync(p, stream);
         p = nullptr;
         n = 0;
+        owned = true;
         const size_t want = std::max<size_t>(bytes, 256);
         cudaMemPool_t pool = table_pool(device);
         if (!pool) return cudaErrorMemoryAllocation;
@@ -164,6 +172,17 @@ struct gt_ctx {
     DBuf w_rec, w_cells, w_geo, w_scan, w_scratch, w_ids, w_dur, w_state, w_cnt, w_flags, w_vgrp, w_reset;
     DBuf log_tab[9];                      // LoG: taps, offsets, norms, radii and tap pairs of the call
     DBuf cp_pts, cp_goff, cp_gloc;        // characterize_points: points, group offsets, group frames
+    // what a call reads back before it goes on, in pinned memory: the flags,
+    // the walk starts and the kept counts of up to kMailCounts frames
+    static constexpr int64_t kMailCounts = 16384;
+    struct Mail {
+        uint32_t flags, pad;
+        unsigned long long starts;
+        uint32_t kept[kMailCounts];
+    };
+    Mail* mail = nullptr;
+    bool mail_kept = false;   // mail->kept holds the last locate pass's counts
+    int32_t ident_n = 0;      // entries of ident that hold their own index
     // segments of the linker's frame loop: scratch of the speculative runs, their states, arrivals
     DBuf w_segs, w_segst, w_segarr, l_segs, l_segst, l_segarr;
     // two sets of window neighbour lists: the lists of window w + 1 are built
@@ -187,11 +206,12 @@ struct gt_ctx {
 struct gt_table {
     int device = 0;
     int64_t n = 0;
+    TBuf arena;                         // holds the columns
     TBuf frame, particle, duration;
     TBuf col[GT_NUM_COLUMNS];
     bool has[GT_NUM_COLUMNS] = {};
     gt_table(int dev, cudaStream_t st) : device(dev) {
-        for (TBuf* b : {&frame, &particle, &duration}) {
+        for (TBuf* b : {&arena, &frame, &particle, &duration}) {
             b->device = dev;
             b->stream = st;
         }
@@ -384,6 +404,17 @@ inline gt_status upload(gt_ctx* ctx, DBuf& b, const std::vector<T>& v) {
 cudaError_t upload_host(int device, void* dst, const void* src, size_t bytes, cudaStream_t st);
 // whether upload_host(src, bytes) would use the lanes, and so block
 bool upload_blocks(const void* src, size_t bytes);
+
+// ident[i] = i for at least n entries
+inline gt_status ensure_ident(gt_ctx* ctx, int n) {
+    if (n <= ctx->ident_n) return GT_OK;
+    std::vector<int32_t> v((size_t)n);
+    for (int i = 0; i < n; i++) v[(size_t)i] = i;
+    ctx->ident_n = 0;
+    CKS(upload(ctx, ctx->ident, v));
+    ctx->ident_n = n;
+    return GT_OK;
+}
 
 inline gt_status subset_groups(gt_ctx* ctx, const float* rows, int64_t n, int ncols, std::vector<int64_t>& goff,
                         std::vector<int64_t>& gframe) {
