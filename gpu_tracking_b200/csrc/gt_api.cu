@@ -385,6 +385,7 @@ struct PipeLink {
             segs.seg = ctx->w_segst.as<LinkSeg>();
             segs.arrived = ctx->w_segarr.as<uint32_t>();
             CK(cudaMemsetAsync(segs.arrived, 0, 4, ctx->lk));
+            CK(cudaMemsetAsync(segs.seg, 0, sizeof(LinkSeg) * (size_t)segs.max_segs, ctx->lk));
             CK(cudaMemsetAsync(ctx->w_dur.p, 0, NS * 8, ctx->lk));
         } else {
             // the per-point linker arrays start cleared: stamps -1, first positions 0

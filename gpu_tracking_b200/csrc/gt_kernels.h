@@ -319,6 +319,7 @@ struct LinkSeg {
     long long base;          // final id of the first id it gave in the segment
     int32_t head;            // ring slot that the next frame replaces
     int32_t final_ids;       // the ids it wrote are final
+    int32_t met, joined;     // runs at its first frame that have ended; whether their states agree
     uint32_t flags;          // error flags of a speculative run
 };
 
@@ -342,7 +343,7 @@ struct LinkSegs {
     uint8_t* base = nullptr;      // scratch of the speculative runs: nvideos x (max_segs - 1)
     size_t bytes = 0;             // link_segment_bytes of one
     int64_t points = 0;           // points that len + prefix frames hold at most (slot mode: slots)
-    LinkSeg* seg = nullptr;       // nvideos x max_segs
+    LinkSeg* seg = nullptr;       // nvideos x max_segs, zero before the first launch
     uint32_t* arrived = nullptr;  // per video, zero before the first launch
 };
 

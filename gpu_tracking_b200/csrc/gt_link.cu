@@ -1156,21 +1156,22 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
 // runs from the true state; each other one starts Q.prefix frames early from
 // an empty state, which the prefix replaces by the true one up to the names
 // of the ids: old entries are out of the ring after memory + 1 frames, and a
-// match they would have changed stops mattering soon after.  The CTA that
-// ends last then goes through the boundaries in order.  Where the state a
-// segment had reached holds the same detections in the same ring order as the
-// end of the segment before it, with ids that correspond one to one, every
-// later match of the segment is the sequential linker's, and its ids are its
-// own ones renamed: those of the boundary's detections by that
-// correspondence, the new ones by an offset.  Where it does not, that CTA
-// links the segment again from the true state.  The result is the sequential
-// linker's in every case, a boundary that does not hold costs its frames.
+// match they would have changed stops mattering soon after.  Of the two runs
+// at a boundary the one that ends later compares them: where the state the
+// later segment had reached holds the same detections in the same ring order
+// as the end of the one before, with ids that correspond one to one, every
+// later match is the sequential linker's, and the segment's ids are its own
+// ones renamed: those of the boundary's detections by that correspondence, the
+// new ones by an offset.  The CTA that ends last adds the offsets up, and links
+// a segment whose boundary does not hold again from the true state.  The
+// result is the sequential linker's in every case, a boundary that does not
+// hold costs its frames.
 // Measured on a B200, one video: 400 frames of 2000 given points, memory 3,
-// 16.4 ms in one CTA and 1.64 ms here (40 segments of 10 frames, each run
-// with a prefix of 10, then about 20 us a boundary); 512 located frames of
-// 2048^2 with 2000 spots: 4.4 ms of linking left after the last frame is
-// located and 1.1 ms here.  Boundaries that did not hold: none of 39 at
-// search_range 7 and step 1.4 px, 4 of 39 at search_range 5 (3.7 ms).
+// 16.4 ms in one CTA and 1.17 ms here (40 segments of 10 frames, each run with
+// a prefix of 10; 1.66 ms while the last CTA compared all boundaries in turn);
+// 512 located frames of 2048^2 with 2000 spots: 4.4 ms of linking left after
+// the last frame is located and 1 ms here.  Boundaries that did not hold: none
+// of 39 at search_range 7 and step 1.4 px, 4 of 39 at search_range 5 (3.4 ms).
 
 // Points of frames [g0, g1).
 __device__ __forceinline__ int64_t frames_points(const LinkInput& in, int g0, int g1) {
@@ -1180,14 +1181,44 @@ __device__ __forceinline__ int64_t frames_points(const LinkInput& in, int g0, in
     return n;
 }
 
-// final id of id `id` of segment q, gmap: final ids of its first q.c0 ids
-__device__ __forceinline__ int64_t segment_id(const LinkSeg& q, const int32_t* gmap, int64_t id) {
-    if (q.final_ids) return id;
-    return id < q.c0 ? (int64_t)__ldcg(gmap + id) : q.base + (id - q.c0);
-}
+// Where the runs of a video keep what joins them.  A speculative run's
+// first ids (those of the boundary it starts at) have partners in the run
+// before: partner[id] in the lower half of its unused start array; the upper
+// half takes, for the comparison at its end, the later run's id of each of its
+// own.
+struct SegmentRuns {
+    LinkSeg* seg;
+    uint8_t *mbase, *qbase;      // true-state scratch, speculative runs' scratch of the video
+    size_t bytes;
+    int64_t mNP, qNP;
+    size_t m_start, q_start;
+    __device__ __forceinline__ uint8_t* spec(int t) const { return qbase + (size_t)(t - 1) * bytes; }
+    __device__ __forceinline__ int32_t* partner(int t) const { return (int32_t*)(spec(t) + q_start); }
+    // the comparison array of the run that ended segment t
+    __device__ __forceinline__ int32_t* inverse(int t, bool true_run) const {
+        return true_run ? (int32_t*)(mbase + m_start) + mNP : (int32_t*)(spec(t) + q_start) + qNP;
+    }
+    // final id of an id of segment t: back through the boundaries to the
+    // segment that gave it
+    __device__ __forceinline__ int64_t final_id(int t, int64_t id) const {
+        while (!__ldcg(&seg[t].final_ids)) {
+            const long long c0 = __ldcg(&seg[t].c0);
+            if (id >= c0) return __ldcg(&seg[t].base) + (id - c0);
+            id = __ldcg(partner(t) + id);
+            t--;
+        }
+        return id;
+    }
+};
 
+// 640 threads: most of a frame is latency and barriers, and the frame loop
+// spills at the 64 registers of 1024.  Device time of the segments (B200) with
+// 512 / 640 / 768 / 1024 threads: 400 frames of 2000 points, memory 3, 1230 /
+// 1173 / 1177 / 1178 us; 160 frames of 500, memory 2, beside locating 689 /
+// 676 / 737 / 870; 64 frames of 4000, memory 3, 1633 / 1479 / 1405 / 1335.
+constexpr int kSegThreads = 640;
 template <typename SF>
-__global__ void __launch_bounds__(kLinkThreads)
+__global__ void __launch_bounds__(kSegThreads)
 link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, LinkWindow W, LinkSegs Q) {
     __shared__ LinkShared sh;
     __shared__ int sh_last;
@@ -1208,7 +1239,16 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
     uint8_t* const mbase = S.base + (size_t)v * S.bytes_per_video;
     const Lay ml = make_lay(G, S.max_edges, S.max_points, M, false);
     const Lay pl = make_lay(G, S.max_edges, Q.points, M, true);
-    auto spec_base = [&](int t) { return Q.base + ((size_t)v * (Q.max_segs - 1) + (t - 1)) * Q.bytes; };
+    SegmentRuns runs;
+    runs.seg = seg;
+    runs.mbase = mbase;
+    runs.qbase = Q.base + (size_t)v * (Q.max_segs - 1) * Q.bytes;
+    runs.bytes = Q.bytes;
+    runs.mNP = S.max_points;
+    runs.qNP = Q.points;
+    runs.m_start = ml.start;
+    runs.q_start = pl.start;
+    auto spec_base = [&](int t) { return runs.spec(t); };
     int32_t* const m_ring = (int32_t*)(mbase + ml.ring_pt);
     int32_t* const m_ring_n = (int32_t*)(mbase + ml.ring_n);
 
@@ -1260,7 +1300,7 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
     };
     const bool stopped = (*(volatile uint32_t*)(out.flags + v) & kLinkStopFlags) != 0;
     if (tid == 0) {
-        seg[s].flags = 0;
+        seg[s].flags = stopped ? kFlagScratch : 0;   // nothing to compare when the video has stopped
         seg[s].c0 = 0;
         sh.counter = 0;
         sh.frame = 0;
@@ -1327,6 +1367,86 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
             seg[s].base = 0;
         }
     }
+    // Compares the end of segment t - 1 (its run in the true-state scratch, or
+    // the speculative one) with the state that segment t's run had reached:
+    // the same detections in ring order, ids one to one.  Leaves the partners.
+    // Whole block.
+    __shared__ int sh_pre[kRingSmem + 2];
+    auto joins = [&](int t, bool true_run) -> bool {
+        uint8_t* const cb = true_run ? mbase : runs.spec(t - 1);
+        const uint8_t* const tb = runs.spec(t);
+        const int32_t* const c_ring = (const int32_t*)(cb + (true_run ? ml.ring_pt : pl.ring_pt));
+        const int32_t* const c_ring_n = (const int32_t*)(cb + (true_run ? ml.ring_n : pl.ring_n));
+        const int32_t* const t_ring = (const int32_t*)(tb + pl.snap);
+        const int32_t* const t_ring_n = t_ring + M * (int64_t)G;
+        const int64_t* const t_pids = (const int64_t*)(tb + pl.pids);
+        int32_t* const partner = runs.partner(t);
+        int32_t* const inverse = runs.inverse(t - 1, true_run);
+        const int ta = seg_first(t), head = __ldcg(&seg[t - 1].head);
+        const int64_t t_lp0 = gbase(in, max(ta - Q.prefix, w_lo)) - P0;
+        const int64_t pa = gbase(in, ta - 1) - P0;
+        const int pn = (int)gsize(in, ta - 1);
+        __syncthreads();
+        if (tid == 0) {
+            // detections of the last frame, then the ring's by age
+            // (a run that raised a flag has no state)
+            bool same = __ldcg(&seg[t].flags) == 0 && (true_run || __ldcg(&seg[t - 1].flags) == 0) &&
+                        !(__ldcg(out.flags + v) & kLinkStopFlags);
+            int tot = pn;
+            for (int q = 0; q < M; q++) {
+                sh_pre[q] = tot;
+                const int n = __ldcg(t_ring_n + q);
+                if (__ldcg(c_ring_n + (head + q) % M) != n) same = false;
+                tot += n;
+            }
+            sh_pre[M] = same ? tot : -1;
+        }
+        __syncthreads();
+        const int tot = sh_pre[M];
+        if (tot < 0) return false;
+        for (int pass = 0; pass < 2; pass++) {
+            bool ok = true;
+            for (int e = tid; e < tot; e += nth) {
+                int64_t lp = pa + e;
+                if (e >= pn) {
+                    int q = 0;
+                    while (sh_pre[q + 1] <= e) q++;
+                    const int32_t a = __ldcg(c_ring + ((head + q) % M) * (int64_t)G + (e - sh_pre[q]));
+                    if (a != __ldcg(t_ring + q * (int64_t)G + (e - sh_pre[q]))) {
+                        ok = false;
+                        break;
+                    }
+                    lp = a;
+                }
+                const int32_t idc = (int32_t)__ldcg(ids + P0 + lp), idt = (int32_t)__ldcg(t_pids + lp - t_lp0);
+                if (pass == 0) {
+                    partner[idt] = idc;
+                    inverse[idc] = idt;
+                } else {
+                    ok &= __ldcg(partner + idt) == idc && __ldcg(inverse + idc) == idt;
+                }
+            }
+            __threadfence_block();
+            if (!__syncthreads_and(ok)) return false;
+        }
+        return true;
+    };
+    // the later of the two runs at a boundary compares them
+    for (int t = max(s, 1); t <= min(s + 1, nseg - 1); t++) {
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            sh_last = atomicAdd(&seg[t].met, 1) == 1 ? 1 : 0;
+            __threadfence();
+        }
+        __syncthreads();
+        if (!sh_last) continue;
+        const bool ok = joins(t, t == 1);
+        if (tid == 0) {
+            seg[t].joined = ok ? 1 : 0;
+            seg[t].met = 0;
+        }
+    }
     __syncthreads();
     if (tid == 0) {
         __threadfence();
@@ -1336,110 +1456,63 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
     __syncthreads();
     if (!sh_last) return;
 
-    // ---- the last CTA resolves the boundaries in order
+    // ---- the last CTA joins the segments in order
     if (tid == 0) Q.arrived[v] = 0;
+    if (*(volatile uint32_t*)(out.flags + v) & kLinkStopFlags) return;
     int cur = 0;               // last segment whose ids are known
     bool cur_true = true;      // its run worked in the true-state scratch
-    long long gcount = *(volatile long long*)&seg[0].counter;   // ids given so far
-    for (;;) {
-        if (*(volatile uint32_t*)(out.flags + v) & kLinkStopFlags) return;
-        bool again = false;
-        for (int t = cur + 1; t < nseg && !again; t++) {
-            // compare the end of segment cur = t - 1 with what segment t reached
-            const LinkSeg qc = seg[cur], qt = seg[t];
-            uint8_t* const cb = cur_true ? mbase : spec_base(cur);
-            const int64_t cNP = cur_true ? S.max_points : Q.points;
-            const int32_t* const c_ring = (const int32_t*)(cb + (cur_true ? ml.ring_pt : pl.ring_pt));
-            const int32_t* const c_ring_n = (const int32_t*)(cb + (cur_true ? ml.ring_n : pl.ring_n));
-            // two arrays of ids in the runs' unused start arrays: the final
-            // ids of a run's first ids, and the partner of an id at the
-            // boundary after the run
-            int32_t* const c_gmap = (int32_t*)(cb + (cur_true ? ml.start : pl.start));
-            int32_t* const c_inv = c_gmap + cNP;
-            uint8_t* const tb = spec_base(t);
-            int32_t* const t_gmap = (int32_t*)(tb + pl.start);
-            const int32_t* const t_ring = (const int32_t*)(tb + pl.snap);
-            const int32_t* const t_ring_n = t_ring + M * (int64_t)G;
-            const int64_t* const t_pids = (const int64_t*)(tb + pl.pids);
-            const int ta = seg_first(t);
-            const int64_t t_lp0 = gbase(in, max(ta - Q.prefix, w_lo)) - P0;
-            const int64_t pa = gbase(in, ta - 1) - P0, pn = gsize(in, ta - 1);
-            bool same = qt.flags == 0;
-            for (int q = 0; q < M; q++)
-                if (__ldcg(c_ring_n + (qc.head + q) % M) != __ldcg(t_ring_n + q)) same = false;
-            if (same) {
-                auto pair = [&](int64_t lp, bool check) -> bool {
-                    const int64_t idc = __ldcg(ids + P0 + lp), idt = __ldcg(t_pids + lp - t_lp0);
-                    const int32_t gid = (int32_t)segment_id(qc, c_gmap, idc);
-                    if (check) return __ldcg(t_gmap + idt) == gid && __ldcg(c_inv + idc) == (int32_t)idt;
-                    t_gmap[idt] = gid;
-                    c_inv[idc] = (int32_t)idt;
-                    return true;
-                };
-                for (int pass = 0; pass < 2 && same; pass++) {
-                    bool ok = true;
-                    for (int64_t i = tid; i < pn; i += nth) ok &= pair(pa + i, pass == 1);
-                    for (int q = 0; q < M; q++) {
-                        const int n = __ldcg(t_ring_n + q);
-                        const int32_t* const cr = c_ring + ((qc.head + q) % M) * (int64_t)G;
-                        for (int e = tid; e < n; e += nth) {
-                            const int32_t lp = __ldcg(cr + e);
-                            if (lp != __ldcg(t_ring + q * (int64_t)G + e)) {
-                                ok = false;
-                                break;
-                            }
-                            ok &= pair(lp, pass == 1);
-                        }
-                    }
-                    __threadfence_block();
-                    same = __syncthreads_and(ok) != 0;
-                }
-            }
-            if (same) {
-                if (tid == 0) seg[t].base = gcount;
-                gcount += qt.counter - qt.c0;
-                cur = t;
-                cur_true = false;
-                __syncthreads();
-                continue;
-            }
-            // final ids for all of segment cur, its ring to the true-state
-            // scratch, and segment t once more from there
-            if (!qc.final_ids)
-                for (int g = seg_first(cur); g < ta; g++) {
-                    const int64_t x = gbase(in, g), n = gsize(in, g);
-                    for (int64_t i = x + tid; i < x + n; i += nth) ids[i] = segment_id(qc, c_gmap, __ldcg(ids + i));
-                }
-            if (!cur_true)
-                for (int q = 0; q < M; q++) {
-                    const int n = __ldcg(c_ring_n + q);
-                    for (int e = tid; e < n; e += nth) m_ring[q * G + e] = __ldcg(c_ring + q * (int64_t)G + e);
-                }
-            __syncthreads();
-            for (int i = tid; i <= M; i += nth) sh.ring_n[i] = __ldcg(c_ring_n + i);
-            if (tid == 0) {
-                seg[cur].final_ids = 1;
-                sh.counter = gcount;
-                sh.prevg = ta - 1;
-                sh.head = qc.head;
-            }
-            __syncthreads();
-            begin_true(t);
-            __syncthreads();
+    bool again = false;        // it was linked a second time
+    long long gcount = __ldcg(&seg[0].counter);   // ids given so far
+    for (int t = 1; t < nseg; t++) {
+        if (again ? joins(t, true) : __ldcg(&seg[t].joined) != 0) {
+            if (tid == 0) seg[t].base = gcount;
+            gcount += __ldcg(&seg[t].counter) - __ldcg(&seg[t].c0);
             cur = t;
-            cur_true = true;
-            again = true;
+            cur_true = false;
+            again = false;
+            continue;
         }
-        if (!again) break;
+        // final ids for all of segment cur, its ring to the true-state
+        // scratch, and segment t once more from there
+        uint8_t* const cb = cur_true ? mbase : runs.spec(cur);
+        const int32_t* const c_ring = (const int32_t*)(cb + (cur_true ? ml.ring_pt : pl.ring_pt));
+        const int32_t* const c_ring_n = (const int32_t*)(cb + (cur_true ? ml.ring_n : pl.ring_n));
+        const int head = __ldcg(&seg[cur].head);
+        __syncthreads();
+        if (!cur_true) {
+            for (int g = seg_first(cur); g < seg_first(t); g++) {
+                const int64_t x = gbase(in, g), n = gsize(in, g);
+                for (int64_t i = x + tid; i < x + n; i += nth) ids[i] = runs.final_id(cur, __ldcg(ids + i));
+            }
+            for (int q = 0; q < M; q++) {
+                const int n = __ldcg(c_ring_n + q);
+                for (int e = tid; e < n; e += nth) m_ring[q * G + e] = __ldcg(c_ring + q * (int64_t)G + e);
+            }
+        }
+        for (int i = tid; i <= M; i += nth) sh.ring_n[i] = __ldcg(c_ring_n + i);
+        __syncthreads();
+        if (tid == 0) {
+            seg[cur].final_ids = 1;
+            sh.counter = gcount;
+            sh.prevg = seg_first(t) - 1;
+            sh.head = head;
+        }
+        __syncthreads();
+        begin_true(t);
+        __syncthreads();
         link_frames<SF, true>(in, L, S, out, gb, run, sh_lo, sh_hi, sh);
         __syncthreads();
+        if (*(volatile uint32_t*)(out.flags + v) & kLinkStopFlags) return;
         gcount = sh.counter;
         for (int i = tid; i <= M; i += nth) m_ring_n[i] = sh.ring_n[i];
         if (tid == 0) {
-            seg[cur].head = sh.head;
-            seg[cur].counter = gcount;
-            seg[cur].final_ids = 1;
+            seg[t].head = sh.head;
+            seg[t].counter = gcount;
+            seg[t].final_ids = 1;
         }
+        cur = t;
+        cur_true = true;
+        again = true;
         __syncthreads();
     }
     // the state the next window starts from
@@ -1461,7 +1534,7 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
             st.counter = gcount;
             st.frame = 0;
             st.prevg = w_hi - 1;
-            st.head = seg[cur].head;
+            st.head = __ldcg(&seg[cur].head);
             W.state[v] = st;
         }
     }
@@ -1489,8 +1562,12 @@ __global__ void segment_ids_kernel(LinkInput in, LinkScratch S, LinkOutput out, 
     int64_t id = out.ids[p];
     if (!q.final_ids) {
         const Lay pl = make_lay(S.max_group, S.max_edges, Q.points, in.memory, true);
-        const uint8_t* b = Q.base + ((size_t)v * (Q.max_segs - 1) + (t - 1)) * Q.bytes;
-        id = segment_id(q, (const int32_t*)(b + pl.start), id);
+        SegmentRuns runs;
+        runs.seg = Q.seg + (size_t)v * Q.max_segs;
+        runs.qbase = Q.base + (size_t)v * (Q.max_segs - 1) * Q.bytes;
+        runs.bytes = Q.bytes;
+        runs.q_start = pl.start;
+        id = runs.final_id(t, id);
         out.ids[p] = id;
     }
     if (out.dur_range) {
@@ -1632,11 +1709,11 @@ cudaError_t link_run_segments(const LinkInput& in, const LinkLists& L, const Lin
     if (fmax >= 0 && fmax < (int64_t)INT32_MAX) {
         constexpr size_t bytes = link_smem_bytes<int32_t>();
         cudaFuncSetAttribute(link_segments_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        link_segments_kernel<int32_t><<<grid, kLinkThreads, bytes, st>>>(in, L, S, out, w, q);
+        link_segments_kernel<int32_t><<<grid, kSegThreads, bytes, st>>>(in, L, S, out, w, q);
     } else {
         constexpr size_t bytes = link_smem_bytes<int64_t>();
         cudaFuncSetAttribute(link_segments_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        link_segments_kernel<int64_t><<<grid, kLinkThreads, bytes, st>>>(in, L, S, out, w, q);
+        link_segments_kernel<int64_t><<<grid, kSegThreads, bytes, st>>>(in, L, S, out, w, q);
     }
     if (p1 > p0)
         segment_ids_kernel<<<(unsigned)((p1 - p0 + 255) / 256), 256, 0, st>>>(in, S, out, w, q, p0, p1);

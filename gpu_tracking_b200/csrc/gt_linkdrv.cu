@@ -182,6 +182,7 @@ gt_status run_link(gt_ctx* ctx, const LinkJob& job, const float* px, const float
         segs.seg = ctx->l_segst.as<LinkSeg>();
         segs.arrived = ctx->l_segarr.as<uint32_t>();
         CK(cudaMemsetAsync(segs.arrived, 0, (size_t)nvideos * 4, ctx->st));
+        CK(cudaMemsetAsync(segs.seg, 0, sizeof(LinkSeg) * (size_t)segs.max_segs * nvideos, ctx->st));
         out.dur_range = row_dur ? 1 : 0;
         if (row_dur) CK(cudaMemsetAsync(out.dur, 0, (size_t)std::max<int64_t>(N, 1) * 8, ctx->st));
     }
