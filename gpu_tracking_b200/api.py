@@ -319,7 +319,7 @@ def link(to_link, search_range, memory=0):
         to_link_np = to_link[["frame", "y", "x"]].to_numpy()
     else:
         to_link_np = to_link
-    arr = np.ascontiguousarray(np.asarray(to_link_np).astype("float32"))
+    arr = np.ascontiguousarray(np.asarray(to_link_np).astype("float32", copy=False))
     if arr.ndim != 2 or arr.shape[1] != 3:
         raise ValueError("link expects (N, 3) rows of frame, y, x")
     ctx = _ffi.context(_DEVICE)
