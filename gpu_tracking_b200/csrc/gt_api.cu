@@ -601,7 +601,18 @@ gt_status locate_pass(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_
     const uint32_t cand_cap = ctx->cand_cap, feat_cap = ctx->feat_cap;
     // super-chunks of SC frames: located chunk by chunk (F frames per launch),
     // then finalized together (one CTA per frame fills the GPU)
-    const int per_super = std::max(1, (int)std::min<int64_t>(128 / F, (NT + F - 1) / F));
+    int super_frames = 128;
+    if (!on_device && !upload_blocks(frames, (size_t)NT * npx * sizeof(T))) {
+        // Pinned frames arrive beside the kernels, but nothing runs beside the
+        // first copy: 64 MB of frames at a time (256 frames of 2048^2 u16: 46.2
+        // ms in copies of a gigabyte, 41.5 so, 41.5 at 32 MB).  Pageable frames
+        // come through the upload lanes, whose threads start for every copy
+        // (64.5 ms in copies of a gigabyte, 70 in copies of 64 MB).
+        const int64_t frame_bytes = (int64_t)(npx * sizeof(T));
+        super_frames = (int)std::min<int64_t>(128, std::max<int64_t>(8, ((int64_t)64 << 20) / frame_bytes));
+        F = std::min(F, super_frames);
+    }
+    const int per_super = std::max(1, (int)std::min<int64_t>(super_frames / F, (NT + F - 1) / F));
     const int SC = F * per_super;
     const int nsuper = (int)((NT + SC - 1) / SC);
     CK(ctx->processed.ensure((size_t)F * npx * 4));
