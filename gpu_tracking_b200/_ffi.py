@@ -211,30 +211,42 @@ class _Block:
 
 
 class ResultPool:
-    """Pinned host memory for result tables, in blocks of a power of two.
+    """Host memory for result tables, in blocks of a power of two.
 
-    Results arrive in pinned memory in one copy without work of the host's
-    (104 MB of columns: 1.9 ms; into fresh pageable memory 8 ms, of which half
-    are page faults), but pinning costs more than a result saves.  So a block
-    is pinned only for a size of which results have been dropped before: a
-    program that keeps every table never pays for it.  At most `limit` bytes
-    are pinned, in use and idle together; other results take ordinary memory.
+    The memory of a dropped result serves the next result of its size (104 MB
+    of columns: 7.1 ms into fresh memory, which faults page by page, 3.8 ms
+    into memory used before).  Results arrive in pinned memory in one copy
+    without work of the host's (2.2 ms; 200 KB: 0.20 instead of 0.28), but
+    pinning 128 MB takes 55 ms, 8 MB 9 ms and 64 KB 0.9 ms, what 11 to 34
+    results save.  So a size earns a pinned block by each `PIN_AFTER` results
+    of it that were dropped: a program that keeps its tables, or makes few,
+    does not pay for it.  Blocks above a quarter of `limit` are never pinned
+    (512 MB: 210 ms).  At most `limit` bytes are pinned, in use and idle
+    together, and at most as many idle bytes of ordinary memory are kept.
     """
+
+    PIN_AFTER = 12
 
     def __init__(self, limit=512 << 20):
         self._lock = threading.RLock()   # a block may go while another is taken
-        self._limit, self._pinned = limit, 0
-        self._idle, self._dropped = {}, {}
+        self._limit, self._pinned, self._kept = limit, 0, 0
+        self._idle, self._ordinary, self._dropped = {}, {}, {}
 
     def take(self, nbytes):
         size = 1 << max(16, int(nbytes).bit_length())
+        keep = None
         with self._lock:
             idle = self._idle.get(size)
             if idle:
                 return _Block(self, size, idle.pop())
-            pin = self._dropped.get(size, 0) > 0 and self._pinned + size <= self._limit
+            ordinary = self._ordinary.get(size)
+            if ordinary:
+                keep = ordinary.pop()
+                self._kept -= size
+            pin = (self._dropped.get(size, 0) >= self.PIN_AFTER and size <= self._limit // 4
+                   and self._pinned + size <= self._limit)
             if pin:
-                self._dropped[size] -= 1
+                self._dropped[size] -= self.PIN_AFTER
                 self._pinned += size
         if pin:
             address = lib().gt_host_alloc(size)
@@ -242,22 +254,26 @@ class ResultPool:
                 return _Block(self, size, address)
             with self._lock:
                 self._pinned -= size
-        keep = np.empty(max(int(nbytes), 1), np.uint8)
-        block = _Block(self, len(keep), keep.ctypes.data, keep)
-        block._size_class = size
-        return block
+        if keep is None:
+            keep = np.empty(size, np.uint8)
+        return _Block(self, size, keep.ctypes.data, keep)
 
     def _back(self, block):
+        size = block._size
         with self._lock:
             if block.pinned:
-                self._idle.setdefault(block._size, []).append(block._address)
-            else:
-                self._dropped[block._size_class] = min(2, self._dropped.get(block._size_class, 0) + 1)
+                self._idle.setdefault(size, []).append(block._address)
+                return
+            self._dropped[size] = min(2 * self.PIN_AFTER, self._dropped.get(size, 0) + 1)
+            if self._kept + size <= self._limit:
+                self._ordinary.setdefault(size, []).append(block._keep)
+                self._kept += size
 
     def trim(self):
         """Gives the idle blocks back to the system."""
         with self._lock:
             idle, self._idle = self._idle, {}
+            self._ordinary, self._kept = {}, 0
             for size, addresses in idle.items():
                 self._pinned -= size * len(addresses)
         for addresses in idle.values():

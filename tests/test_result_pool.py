@@ -1,5 +1,5 @@
 """The pool of pinned result blocks: bounded, a block is never in two results
-at once, pinned only for sizes whose results are dropped; and on a GPU the
+at once, pinned only for sizes of which many results were dropped; and on a GPU the
 pinned and the pageable way of a table, and of frames large enough for the
 upload lanes, give the same values."""
 import gc
@@ -41,7 +41,8 @@ def test_kept_results_are_never_pinned(fake):
 
 def test_dropped_results_are_pinned_and_reused(fake):
     pool = _ffi.ResultPool(limit=8 << 20)
-    for _ in range(6):
+    for k in range(pool.PIN_AFTER + 6):
+        assert bool(fake.live) == (k > pool.PIN_AFTER)
         a = np.asarray(pool.take(1 << 20))[: 1 << 20].view(np.float64)[7:]   # views keep the block
         a[:] = 3.0
         del a
@@ -56,6 +57,21 @@ def test_dropped_results_are_pinned_and_reused(fake):
     del v
     gc.collect()
     pool.trim()
+    assert not fake.live
+
+
+def test_ordinary_blocks_are_reused_within_the_limit(fake):
+    pool = _ffi.ResultPool(limit=8 << 20)
+    held = [pool.take((2 << 20) - 1) for _ in range(6)]
+    addresses = {b.address for b in held}
+    del held
+    gc.collect()
+    assert pool._kept == 8 << 20
+    again = [pool.take((2 << 20) - 1) for _ in range(4)]
+    assert {b.address for b in again} <= addresses and pool._kept == 0
+    for _ in range(2 * pool.PIN_AFTER):
+        pool.take(3 << 20)               # a block of half the limit: never pinned
+        gc.collect()
     assert not fake.live
 
 
@@ -85,7 +101,7 @@ def test_limit_and_threads(fake):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [np.uint8, np.float32])
-def test_table_and_upload_ways_agree(dtype):
+def test_table_and_upload_ways_agree(dtype, monkeypatch):
     import pandas as pd
     import torch
 
@@ -95,6 +111,7 @@ def test_table_and_upload_ways_agree(dtype):
                  read_noise=3.0 if dtype == np.float32 else None)
     assert f.nbytes > 5 << 20            # several slots of every lane
     kw = dict(minmass=60.0, search_range=4.0, memory=1, tqdm=False)
+    monkeypatch.setattr(_ffi.ResultPool, "PIN_AFTER", 1)
     first = gt.batch(f, 7, **kw)         # pageable result, pageable frames
     copy = first.copy(deep=True)
     dropped = gt.batch(f, 7, **kw)
