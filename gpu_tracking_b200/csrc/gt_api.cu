@@ -1072,8 +1072,9 @@ gt_status batch_impl(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_d
     for (int attempt = 0;; attempt++) {
         uint32_t fl = 0;
         HostSpan hs(ctx, "host_locate");
-        // frames link while later frames are located when every frame's
-        // detections sort in shared memory (the group sort's limit)
+        // frames link while later frames are located unless a frame may hold
+        // more detections than a link window's buffers are sized for (lists
+        // and edges of up to 4096 points a frame)
         windowed = p.has_search_range && ctx->feat_cap <= 4096u;
         gt_status st = locate_pass<T>(ctx, p, frames, on_device, NT, H, W, c, log_style ? &lt : nullptr, F, &fl,
                                       windowed ? &pl : nullptr, &reset, net);

@@ -1,6 +1,6 @@
 """The linker's frame loop cut into segments that run side by side.
 
-Segments of at least 8 frames (more with memory) start from an empty state a
+Segments of memory + 2 frames and more start from an empty state a
 few frames early; boundaries whose states do not agree are linked again.  Ids
 must equal the oracle's whole-video linker whatever the number of frames
 (below, at and above whole segments), the memory, the crowding (dense sets,
@@ -31,7 +31,7 @@ def rows(frames, n, side, seed, seen=0.8, D=1.0, empty=()):
 
 
 @pytest.mark.parametrize("memory", [0, 1, 3, 5])
-@pytest.mark.parametrize("frames", [7, 8, 9, 16, 17, 31, 100])
+@pytest.mark.parametrize("frames", [2, 3, 4, 5, 6, 7, 8, 9, 15, 16, 17, 31, 100])
 def test_link_over_segment_edges(oracle, memory, frames):
     r = rows(frames, 60, 120.0, seed=frames + 10 * memory)
     assert np.array_equal(gt.link(r, 4.0, memory), oracle.link(r, 4.0, memory))
