@@ -219,13 +219,17 @@ class ResultPool:
     without work of the host's (2.2 ms; 200 KB: 0.20 instead of 0.28), but
     pinning 128 MB takes 55 ms, 8 MB 9 ms and 64 KB 0.9 ms, what 11 to 34
     results save.  So a size earns a pinned block by each `PIN_AFTER` results
-    of it that were dropped: a program that keeps its tables, or makes few,
-    does not pay for it.  Blocks above a quarter of `limit` are never pinned
+    of it that were dropped (a third of them up to 8 MB, where pinning never
+    takes 10 ms): a program that keeps its tables, or makes few, does not pay
+    for it.  Blocks above a quarter of `limit` are never pinned
     (512 MB: 210 ms).  At most `limit` bytes are pinned, in use and idle
     together, and at most as many idle bytes of ordinary memory are kept.
     """
 
     PIN_AFTER = 12
+
+    def earned(self, size):
+        return self.PIN_AFTER if size > 8 << 20 else max(1, self.PIN_AFTER // 3)
 
     def __init__(self, limit=512 << 20):
         self._lock = threading.RLock()   # a block may go while another is taken
@@ -243,10 +247,10 @@ class ResultPool:
             if ordinary:
                 keep = ordinary.pop()
                 self._kept -= size
-            pin = (self._dropped.get(size, 0) >= self.PIN_AFTER and size <= self._limit // 4
+            pin = (self._dropped.get(size, 0) >= self.earned(size) and size <= self._limit // 4
                    and self._pinned + size <= self._limit)
             if pin:
-                self._dropped[size] -= self.PIN_AFTER
+                self._dropped[size] -= self.earned(size)
                 self._pinned += size
         if pin:
             address = lib().gt_host_alloc(size)

@@ -41,8 +41,9 @@ def test_kept_results_are_never_pinned(fake):
 
 def test_dropped_results_are_pinned_and_reused(fake):
     pool = _ffi.ResultPool(limit=8 << 20)
-    for k in range(pool.PIN_AFTER + 6):
-        assert bool(fake.live) == (k > pool.PIN_AFTER)
+    assert pool.earned(2 << 20) < pool.earned(64 << 20)
+    for k in range(pool.earned(2 << 20) + 6):
+        assert bool(fake.live) == (k > pool.earned(2 << 20))
         a = np.asarray(pool.take(1 << 20))[: 1 << 20].view(np.float64)[7:]   # views keep the block
         a[:] = 3.0
         del a
@@ -62,6 +63,7 @@ def test_dropped_results_are_pinned_and_reused(fake):
 
 def test_ordinary_blocks_are_reused_within_the_limit(fake):
     pool = _ffi.ResultPool(limit=8 << 20)
+    pool.PIN_AFTER = 30
     held = [pool.take((2 << 20) - 1) for _ in range(6)]
     addresses = {b.address for b in held}
     del held
