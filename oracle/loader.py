@@ -38,7 +38,7 @@ def build():
     """Compile the oracle (and the reference translation when the checkout exists)."""
     subprocess.run(["make", "-s", "-C", HERE], check=True)
     ref = reference_root()
-    if os.path.isdir(ref):
+    if os.path.isdir(os.path.join(ref, "src", "shaders")):   # an empty directory is no checkout
         subprocess.run(["make", "-s", "-C", HERE, "ref", "REF=" + ref], check=True)
 
 
