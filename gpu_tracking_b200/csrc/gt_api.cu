@@ -1920,6 +1920,14 @@ GT_API gt_status gt__set_link_window_caps(gt_ctx* ctx, int64_t list_entries, int
     return GT_OK;
 }
 
+// Test hook: what the last call left them at (a call that overflows one grows it).
+GT_API gt_status gt__get_link_window_caps(const gt_ctx* ctx, int64_t* list_entries, int64_t* edges_per_frame) {
+    if (!ctx || !list_entries || !edges_per_frame) return GT_ERR_INVALID_ARGUMENT;
+    *list_entries = ctx->w_list_cap;
+    *edges_per_frame = ctx->w_edge_cap;
+    return GT_OK;
+}
+
 // Test hook (exported, not part of the public header): the per-frame
 // candidate and detection capacities the next gt_batch starts from (values
 // <= 0 keep the current ones).  Small values make the kernels report overflow

@@ -879,6 +879,7 @@ __device__ __forceinline__ void link_frames(const LinkInput& in, const LinkLists
             return;
         }
         // ---- P5: branch and bound per subnet (recurse2, linking.rs:687-766)
+        bool spent = false;   // a subnet of this thread's ran out of steps
         for (int q = tid; q < nroots; q += nth) {
             const int r = roots[q];
             const int od = comp_off[r], os = comp_soff[r];
@@ -949,14 +950,16 @@ __device__ __forceinline__ void link_frames(const LinkInput& in, const LinkLists
                     opt[level] = op + 1;
                 }
             }
-            if (over) atomicOr(run.flags, kFlagSubnetBudget);
+            spent |= over;
             for (int l = 0; l < nd; l++) {
                 int ch = has_best ? bst[l] : -1;
                 out_src[pathD[od + l]] = (ch >= 0) ? pathS[os + ch] : -1;
             }
         }
-        __syncthreads();
-        if (*(volatile uint32_t*)run.flags & kFlagSubnetBudget) return;
+        if (__syncthreads_or(spent)) {
+            if (tid == 0) atomicOr(run.flags, kFlagSubnetBudget);
+            return;
+        }
         // ---- P6: ids (new ones in destination order, src/linking.rs:788-798)
         {
             int newtot = 0;
@@ -1039,15 +1042,28 @@ __device__ __forceinline__ void link_frames(const LinkInput& in, const LinkLists
     }
 }
 
+// Whether the video's linking has stopped, the same answer for every thread of
+// the block: the CTA of the video's first segment and the list kernels of the
+// next window raise flags while this one runs, so a thread's own read must not
+// decide about a barrier.  Whole block; `sh` is free again at the next barrier
+// after the call.
+__device__ __forceinline__ bool link_stopped(const uint32_t* flags, int* sh) {
+    __syncthreads();
+    if (threadIdx.x == 0) *sh = (*(const volatile uint32_t*)flags & kLinkStopFlags) != 0 ? 1 : 0;
+    __syncthreads();
+    return *sh != 0;
+}
+
 // Every video (or the next window of one) by one CTA, frame after frame.
 template <typename SF>
 __global__ void __launch_bounds__(kLinkThreads)
 link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, LinkWindow W) {
     __shared__ LinkShared sh;
+    __shared__ int sh_stop;
     const int v = blockIdx.x;
     const int gb = in.vgrp[v], ge = in.vgrp[v + 1];
     const int g_lo = (W.g0 < 0) ? gb : W.g0, g_hi = (W.g0 < 0) ? ge : W.g1;
-    if (out.flags[v] & kLinkStopFlags) return;  // an earlier window stopped this video
+    if (link_stopped(out.flags + v, &sh_stop)) return;  // an earlier window stopped this video
     const int64_t P0 = gbase(in, gb);
     const int64_t NP = in.slot_stride ? (int64_t)(ge - gb) * in.slot_stride : in.goff[ge] - P0;
     const int M = in.memory, K = M + 1;
@@ -1108,11 +1124,11 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
     run.c0 = nullptr;
     run.spec = false;
     link_frames<SF, false>(in, L, S, out, gb, run, g_lo, g_hi, sh);
-    __syncthreads();
+    const bool stopped = link_stopped(out.flags + v, &sh_stop);
     if (!W.last) {
         if (ring_smem)
             for (int i = tid; i <= M; i += nth) ring_n[i] = ringN[i];
-        if (tid == 0 && !(out.flags[v] & kLinkStopFlags)) {
+        if (tid == 0 && !stopped) {
             LinkState st;
             st.counter = sh.counter;
             st.frame = sh.frame;
@@ -1123,7 +1139,7 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
         return;
     }
     // ---- Linker::finish (src/linking.rs:505-520)
-    if (!(out.flags[v] & kLinkStopFlags)) {
+    if (!stopped) {
         const long long frame = sh.frame;
         if (M > 0) {
             for (int q = 0; q < M; q++) {
@@ -1298,7 +1314,7 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
                 }
         }
     };
-    const bool stopped = (*(volatile uint32_t*)(out.flags + v) & kLinkStopFlags) != 0;
+    const bool stopped = link_stopped(out.flags + v, &sh_last);
     if (tid == 0) {
         seg[s].flags = stopped ? kFlagScratch : 0;   // nothing to compare when the video has stopped
         seg[s].c0 = 0;
@@ -1458,7 +1474,7 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
 
     // ---- the last CTA joins the segments in order
     if (tid == 0) Q.arrived[v] = 0;
-    if (*(volatile uint32_t*)(out.flags + v) & kLinkStopFlags) return;
+    if (link_stopped(out.flags + v, &sh_last)) return;
     int cur = 0;               // last segment whose ids are known
     bool cur_true = true;      // its run worked in the true-state scratch
     bool again = false;        // it was linked a second time
@@ -1501,8 +1517,7 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
         begin_true(t);
         __syncthreads();
         link_frames<SF, true>(in, L, S, out, gb, run, sh_lo, sh_hi, sh);
-        __syncthreads();
-        if (*(volatile uint32_t*)(out.flags + v) & kLinkStopFlags) return;
+        if (link_stopped(out.flags + v, &sh_last)) return;
         gcount = sh.counter;
         for (int i = tid; i <= M; i += nth) m_ring_n[i] = sh.ring_n[i];
         if (tid == 0) {
