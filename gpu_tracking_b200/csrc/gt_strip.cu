@@ -40,6 +40,7 @@
 // fma(x, zh, x*zl).
 #include <math.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -664,7 +665,7 @@ int strip_rows(int nx, int H, int nframes, int resident) {
     const int first = (H + 511) / 512;
     int best = 0;
     int64_t best_cost = INT64_MAX;
-    for (int n = first; n <= 128; n++) {
+    for (int n = first; n <= std::max(first, 128); n++) {   // the first one whatever the height
         const int rows = n == 1 ? H : ((H + n - 1) / n + kStepRows - 1) / kStepRows * kStepRows;
         if (n > first && rows < kStepRows) break;
         const int64_t tiles = (int64_t)nx * ((H + rows - 1) / rows) * nframes;
