@@ -368,16 +368,23 @@ struct PipeLink {
         // Without linker resets the frames of a window link in segments, one
         // CTA each.  16 frames a segment beside locating (8 SMs for less than
         // a millisecond a window); the shortest ones in the last window, which
-        // nothing is left to hide.
+        // nothing is left to hide.  Longer ones where the runs' scratch would
+        // pass its bound (the edge buffer grows with the most crowded call so
+        // far), and the sequential kernel where not even two segments fit.
         segmented = memory <= kLinkSegMemory && std::find(reset.begin(), reset.end(), 1) == reset.end();
+        if (segmented) {
+            segs.prefix = link_segment_prefix(memory);
+            for (seg_len_last = link_segment_min(memory);; seg_len_last *= 2) {
+                seg_len = std::max(16, seg_len_last);
+                segs.max_segs = std::max((SC + seg_len_last - 1) / seg_len_last, 1);
+                segs.points = (int64_t)(seg_len + segs.prefix) * C;
+                segs.bytes = link_segment_bytes(S.max_group, S.max_edges, segs.points, memory);
+                if (segs.bytes * (size_t)(segs.max_segs - 1) <= kLinkSegScratch) break;
+            }
+            segmented = segs.max_segs >= 2 || SC <= link_segment_min(memory);
+        }
         out.dur_range = segmented ? 1 : 0;
         if (segmented) {
-            seg_len_last = link_segment_min(memory);
-            seg_len = std::max(16, seg_len_last);
-            segs.prefix = link_segment_prefix(memory);
-            segs.max_segs = std::max((SC + seg_len_last - 1) / seg_len_last, 1);
-            segs.points = (int64_t)(seg_len + segs.prefix) * C;
-            segs.bytes = link_segment_bytes(S.max_group, S.max_edges, segs.points, memory);
             CK(ctx->w_segs.ensure(segs.bytes * (size_t)(segs.max_segs - 1)));
             CK(ctx->w_segst.ensure(sizeof(LinkSeg) * (size_t)segs.max_segs));
             CK(ctx->w_segarr.ensure(4));

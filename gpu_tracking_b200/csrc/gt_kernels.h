@@ -336,6 +336,9 @@ constexpr int link_segment_prefix(int memory) { return memory == 0 ? 1 : 2 * (me
 // with memory 3, 785 -> 640 with 1, 455 -> 345 with 0; 64 frames of 3900
 // points, memory 3, 1519 -> 1132 us.
 constexpr int link_segment_min(int memory) { return memory + 2; }
+// Bytes of all speculative runs of a launch at most: segments get longer, up to
+// one, until their scratch fits.
+constexpr size_t kLinkSegScratch = (size_t)2 << 30;
 constexpr int kLinkSegMemory = 16;   // larger memories keep the sequential linker (prefixes of 36 frames and more)
 
 // Segments of `len` frames (at least memory + 2), each run from `prefix`

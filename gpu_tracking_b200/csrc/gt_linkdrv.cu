@@ -16,8 +16,6 @@ using namespace gt::rt;
 namespace gt {
 namespace rt {
 
-constexpr size_t kLinkSegScratch = (size_t)2 << 30;   // bytes of all speculative runs of a call
-
 // pgroup[i] = g for the points i of group g (goff: group offsets)
 __global__ void fill_pgroup_kernel(const int64_t* __restrict__ goff, int ngroups, int32_t* __restrict__ pgroup) {
     for (int g = blockIdx.x; g < ngroups; g += gridDim.x)
