@@ -2046,7 +2046,7 @@ gt_status gt_create(int32_t device, gt_ctx** out) {
         cudaEventCreateWithFlags(&ctx->located, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->linked, cudaEventDisableTiming) != cudaSuccess) {
         delete ctx;
-        return GT_ERR_CUDA;
+        return cuda_failed();
     }
     for (int i = 0; i < 2; i++) {
         if (cudaEventCreateWithFlags(&ctx->used[i], cudaEventDisableTiming) != cudaSuccess ||
@@ -2054,7 +2054,7 @@ gt_status gt_create(int32_t device, gt_ctx** out) {
             cudaEventCreateWithFlags(&ctx->listed[i], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ctx->w_linked[i], cudaEventDisableTiming) != cudaSuccess) {
             gt_destroy(ctx);
-            return GT_ERR_CUDA;
+            return cuda_failed();
         }
     }
     *out = ctx;

@@ -237,7 +237,10 @@ static gt_status noalloc_fail(gt_ctx* ctx, gt_status st, const char* msg) {
 #define NA_CK(expr)                                                                \
     do {                                                                           \
         cudaError_t e_ = (expr);                                                   \
-        if (e_ != cudaSuccess) return noalloc_fail(ctx, GT_ERR_CUDA, cudaGetErrorString(e_)); \
+        if (e_ != cudaSuccess) {                                                   \
+            cudaGetLastError(); /* the thread's next call must not find it */      \
+            return noalloc_fail(ctx, GT_ERR_CUDA, cudaGetErrorString(e_));         \
+        }                                                                          \
     } while (0)
 
 extern "C" gt_status gt_link_noalloc(gt_ctx* ctx, const float* d_fyx, int64_t n, float search_range,

@@ -42,8 +42,10 @@ gt_status fail(gt_ctx* ctx, gt_status st, const std::string& msg) {
 #define PK(expr)                                                                                          \
     do {                                                                                                  \
         cudaError_t e_ = (expr);                                                                          \
-        if (e_ != cudaSuccess)                                                                            \
+        if (e_ != cudaSuccess) {                                                                          \
+            cudaGetLastError(); /* the thread's next call must not find it */                             \
             return fail(ctx, GT_ERR_CUDA, std::string("CUDA error ") + cudaGetErrorString(e_) + " at " #expr); \
+        }                                                                                                 \
     } while (0)
 
 // Device buffers of one call, freed on every exit path.  With `keep` (a list of

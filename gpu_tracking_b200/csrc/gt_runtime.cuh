@@ -242,12 +242,19 @@ inline gt_status set_err(gt_ctx* ctx, gt_status st, const char* fmt, ...) {
     return st;
 }
 
-#define CK(expr)                                                                                             \
-    do {                                                                                                     \
-        cudaError_t e_ = (expr);                                                                             \
-        if (e_ != cudaSuccess)                                                                               \
-            return set_err(ctx, GT_ERR_CUDA, "CUDA error %s at %s:%d (%s)", cudaGetErrorString(e_), __FILE__, \
-                           __LINE__, #expr);                                                                 \
+// A failed call leaves no error behind: CUDA keeps the last one per thread, and
+// the thread's next call would find it.
+inline gt_status cuda_failed() {
+    cudaGetLastError();
+    return GT_ERR_CUDA;
+}
+
+#define CK(expr)                                                                                               \
+    do {                                                                                                       \
+        cudaError_t e_ = (expr);                                                                               \
+        if (e_ != cudaSuccess)                                                                                 \
+            return set_err(ctx, cuda_failed(), "CUDA error %s at %s:%d (%s)", cudaGetErrorString(e_), __FILE__, \
+                           __LINE__, #expr);                                                                   \
     } while (0)
 
 #define CKS(expr)                        \

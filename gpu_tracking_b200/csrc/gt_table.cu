@@ -28,11 +28,11 @@ gt_status gt_table_column_f32(const gt_table* t, int32_t column, float* dst) {
     if (column == GT_COL_FRAME || column == GT_COL_PARTICLE || column == GT_COL_DURATION) {
         std::vector<int64_t> v(t->n);
         const TBuf& b = column == GT_COL_FRAME ? t->frame : (column == GT_COL_PARTICLE ? t->particle : t->duration);
-        if (cudaMemcpy(v.data(), b.p, t->n * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return GT_ERR_CUDA;
+        if (cudaMemcpy(v.data(), b.p, t->n * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return cuda_failed();
         for (int64_t i = 0; i < t->n; i++) dst[i] = (float)v[i];
         return GT_OK;
     }
-    if (cudaMemcpy(dst, t->col[column].p, t->n * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return GT_ERR_CUDA;
+    if (cudaMemcpy(dst, t->col[column].p, t->n * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return cuda_failed();
     return GT_OK;
 }
 
@@ -44,7 +44,7 @@ gt_status gt_table_column_i64(const gt_table* t, int32_t column, int64_t* dst) {
     if (t->n == 0) return GT_OK;
     cudaSetDevice(t->device);
     const TBuf& b = column == GT_COL_FRAME ? t->frame : (column == GT_COL_PARTICLE ? t->particle : t->duration);
-    if (cudaMemcpy(dst, b.p, t->n * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return GT_ERR_CUDA;
+    if (cudaMemcpy(dst, b.p, t->n * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return cuda_failed();
     return GT_OK;
 }
 
@@ -155,7 +155,7 @@ gt_status table_export_impl(const gt_table* t, const int32_t* columns, int32_t n
     ExportPool* pool = export_pool(t->device);
     if (!pool) return GT_ERR_INVALID_ARGUMENT;
     std::lock_guard<std::mutex> lock(pool->mu);
-    if (cudaSetDevice(t->device) != cudaSuccess || export_pool_init(*pool) != cudaSuccess) return GT_ERR_CUDA;
+    if (cudaSetDevice(t->device) != cudaSuccess || export_pool_init(*pool) != cudaSuccess) return cuda_failed();
     // lanes: one per 256k rows, at most kExportLanes and half the host threads
     const int hw = std::max(1, (int)std::thread::hardware_concurrency() / 2);
     const int lanes = (int)std::max<int64_t>(1, std::min<int64_t>({kExportLanes, hw, (N + (1 << 18) - 1) >> 18}));
@@ -192,7 +192,7 @@ gt_status table_export_impl(const gt_table* t, const int32_t* columns, int32_t n
     err[0] = export_lane(t->device, pool->lane[0], work[0]);
     for (auto& x : th) x.join();
     for (cudaError_t e : err)
-        if (e != cudaSuccess) return GT_ERR_CUDA;
+        if (e != cudaSuccess) return cuda_failed();
     return GT_OK;
 }
 
@@ -236,22 +236,21 @@ gt_status gt_table_export_pinned(const gt_table* t, const int32_t* columns, int3
                                       : (id == GT_COL_PARTICLE ? t->particle.p
                                                                : (id == GT_COL_DURATION ? t->duration.p : t->col[id].p));
     }
-    if (cudaSetDevice(t->device) != cudaSuccess) return GT_ERR_CUDA;
+    if (cudaSetDevice(t->device) != cudaSuccess) return cuda_failed();
     const cudaStream_t st = cudaStreamPerThread;   // the call that made the table has finished its work on it
     TBuf tmp;
     tmp.device = t->device;
     tmp.stream = st;
     const size_t bytes = (size_t)ncolumns * (size_t)t->n * 8;
     if (tmp.ensure(bytes) != cudaSuccess) {
-        cudaGetLastError();
-        return GT_ERR_CUDA;
+        return cuda_failed();
     }
     const dim3 grid((unsigned)std::min<int64_t>((t->n + 255) / 256, 1024), ncolumns);
     widen_columns_kernel<<<grid, 256, 0, st>>>(c, t->n, tmp.as<unsigned long long>());
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(block, tmp.p, bytes, cudaMemcpyDeviceToHost, st);
     const cudaError_t e2 = cudaStreamSynchronize(st);
-    return e == cudaSuccess && e2 == cudaSuccess ? GT_OK : GT_ERR_CUDA;
+    return e == cudaSuccess && e2 == cudaSuccess ? GT_OK : cuda_failed();
 }
 
 void* gt_host_alloc(size_t bytes) {

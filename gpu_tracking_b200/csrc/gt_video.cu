@@ -686,7 +686,9 @@ gt_status read_frames_device(gt_video* v, gt_ctx* ctx, const int64_t* keys, int6
     uint64_t dec_bytes = 0;
     auto flush = [&]() -> gt_status {
         if (blocks.empty()) return GT_OK;
-        auto cuda_err = [](cudaError_t e) { return verr(GT_ERR_CUDA, std::string("CUDA error ") + cudaGetErrorString(e)); };
+        auto cuda_err = [](cudaError_t e) {
+            return verr(gt::rt::cuda_failed(), std::string("CUDA error ") + cudaGetErrorString(e));
+        };
         cudaError_t e;
         if ((e = ctx->vd_src.ensure(std::max<size_t>(hsrc.size(), 16))) != cudaSuccess) return cuda_err(e);
         if ((e = ctx->vd_dec.ensure(std::max<uint64_t>(dec_bytes, 16))) != cudaSuccess) return cuda_err(e);
