@@ -370,7 +370,8 @@ struct PipeLink {
         // a millisecond a window); the shortest ones in the last window, which
         // nothing is left to hide.  Longer ones where the runs' scratch would
         // pass its bound (the edge buffer grows with the most crowded call so
-        // far), and the sequential kernel where not even two segments fit.
+        // far), and the sequential kernel where not even two segments fit or
+        // there is no memory for them.
         segmented = memory <= kLinkSegMemory && std::find(reset.begin(), reset.end(), 1) == reset.end();
         if (segmented) {
             segs.prefix = link_segment_prefix(memory);
@@ -381,11 +382,11 @@ struct PipeLink {
                 segs.bytes = link_segment_bytes(S.max_group, S.max_edges, segs.points, memory);
                 if (segs.bytes * (size_t)(segs.max_segs - 1) <= kLinkSegScratch) break;
             }
-            segmented = segs.max_segs >= 2 || SC <= link_segment_min(memory);
+            segmented = (segs.max_segs >= 2 || SC <= link_segment_min(memory)) &&
+                        try_ensure(ctx, ctx->w_segs, segs.bytes * (size_t)(segs.max_segs - 1));
         }
         out.dur_range = segmented ? 1 : 0;
         if (segmented) {
-            CK(ctx->w_segs.ensure(segs.bytes * (size_t)(segs.max_segs - 1)));
             CK(ctx->w_segst.ensure(sizeof(LinkSeg) * (size_t)segs.max_segs));
             CK(ctx->w_segarr.ensure(4));
             segs.base = ctx->w_segs.as<uint8_t>();
@@ -1932,6 +1933,14 @@ GT_API gt_status gt__get_link_window_caps(const gt_ctx* ctx, int64_t* list_entri
     if (!ctx || !list_entries || !edges_per_frame) return GT_ERR_INVALID_ARGUMENT;
     *list_entries = ctx->w_list_cap;
     *edges_per_frame = ctx->w_edge_cap;
+    return GT_OK;
+}
+
+// Test hook: buffers that calls can do without, above this many bytes, are not
+// to be had (0: no limit).
+GT_API gt_status gt__set_optional_limit(gt_ctx* ctx, uint64_t bytes) {
+    if (!ctx) return GT_ERR_INVALID_ARGUMENT;
+    ctx->optional_limit = (size_t)bytes;
     return GT_OK;
 }
 

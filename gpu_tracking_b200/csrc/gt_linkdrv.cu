@@ -151,7 +151,8 @@ gt_status run_link(gt_ctx* ctx, const LinkJob& job, const float* px, const float
     out.vpoff = nullptr;
     out.flags = ctx->l_flags.as<uint32_t>();
     // segments of the frame loop: as many CTAs as there are SMs for the
-    // videos, none shorter than link_segment_min, scratch bounded
+    // videos, none shorter than link_segment_min, scratch bounded; without
+    // memory for it the sequential kernel
     LinkSegs segs;
     int max_frames = 0;
     for (int v = 0; v < nvideos; v++) max_frames = std::max(max_frames, job.vgrp[v + 1] - job.vgrp[v]);
@@ -171,9 +172,9 @@ gt_status run_link(gt_ctx* ctx, const LinkJob& job, const float* px, const float
             if (segs.bytes * (size_t)(segs.max_segs - 1) * nvideos <= kLinkSegScratch) break;
         }
     }
-    const bool segmented = segs.max_segs >= 2;
+    const bool segmented = segs.max_segs >= 2 &&
+                           try_ensure(ctx, ctx->l_segs, segs.bytes * (size_t)(segs.max_segs - 1) * nvideos);
     if (segmented) {
-        CK(ctx->l_segs.ensure(segs.bytes * (size_t)(segs.max_segs - 1) * nvideos));
         CK(ctx->l_segst.ensure(sizeof(LinkSeg) * (size_t)segs.max_segs * nvideos));
         CK(ctx->l_segarr.ensure((size_t)nvideos * 4));
         segs.base = ctx->l_segs.as<uint8_t>();

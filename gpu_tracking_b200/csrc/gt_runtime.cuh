@@ -183,6 +183,7 @@ struct gt_ctx {
     Mail* mail = nullptr;
     bool mail_kept = false;   // mail->kept holds the last locate pass's counts
     int32_t ident_n = 0;      // entries of ident that hold their own index
+    size_t optional_limit = 0;   // test hook: bytes a buffer of try_ensure may have (0: no limit)
     // segments of the linker's frame loop: scratch of the speculative runs, their states, arrivals
     DBuf w_segs, w_segst, w_segarr, l_segs, l_segst, l_segarr;
     // two sets of window neighbour lists: the lists of window w + 1 are built
@@ -411,6 +412,15 @@ inline gt_status upload(gt_ctx* ctx, DBuf& b, const std::vector<T>& v) {
 cudaError_t upload_host(int device, void* dst, const void* src, size_t bytes, cudaStream_t st);
 // whether upload_host(src, bytes) would use the lanes, and so block
 bool upload_blocks(const void* src, size_t bytes);
+
+// A buffer that a call can do without: false, and no error left behind, where
+// there is no memory for it.
+inline bool try_ensure(gt_ctx* ctx, DBuf& b, size_t bytes) {
+    if (ctx->optional_limit > 0 && bytes > ctx->optional_limit) return false;
+    if (b.ensure(bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
 
 // ident[i] = i for at least n entries
 inline gt_status ensure_ident(gt_ctx* ctx, int n) {

@@ -56,3 +56,16 @@ def test_bounded_for_large_edge_buffers(oracle, movie, ctx, edges, memory):
     ctx.check(hook("gt__set_link_window_caps", ctypes.c_int64, ctypes.c_int64)(ctx.handle, 0, edges))
     linked(oracle, movie, memory)
     assert used() - before < 8 * edges * 1.2 + 2.3 * GIB
+
+
+@pytest.mark.parametrize("memory", [0, 2])
+def test_sequential_when_there_is_no_memory(oracle, movie, ctx, memory):
+    limit = hook("gt__set_optional_limit", ctypes.c_uint64)
+    kw = dict(minmass=300.0, search_range=6.0, memory=memory)
+    tab = oracle.batch(trackpy_params(9, **kw), movie.astype(np.float32))
+    r = rows(300, 300, 250.0, seed=3)
+    ids = oracle.link(r, 4.0, memory)
+    for bytes_ in (1 << 16, 0):
+        ctx.check(limit(ctx.handle, bytes_))
+        assert_same(gt.batch(movie, 9, tqdm=False, **kw), tab, LINK_COLS)
+        assert np.array_equal(gt.link(r, 4.0, memory), ids)
