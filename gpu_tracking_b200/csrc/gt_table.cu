@@ -1,8 +1,8 @@
 // gt_table.cu — result tables of the C ABI: row counts, single columns and
-// gt_table_export, which copies several columns at once through per-device
-// pools of pinned staging lanes and widens them to the dtypes of the
-// reference's DataFrame (gpu_tracking_macros/src/lib.rs:138-147) on host
-// threads.
+// gt_table_export, which widens several columns at once to the dtypes of the
+// reference's DataFrame (gpu_tracking_macros/src/lib.rs:138-147): on the device
+// into pinned destinations, else on host threads through per-device pools of
+// pinned staging lanes.
 #include <memory>
 #include <thread>
 
@@ -144,6 +144,77 @@ cudaError_t export_lane(int device, ExportLane& L, const std::vector<ExportItem>
 
 namespace {
 
+// Columns widened on the device into pinned host columns of 8-byte values: a
+// float column as doubles, an integer column as it is.  Blocks of threads
+// stride over the rows of column blockIdx.y and store across PCIe: no staging
+// on the device or the host.
+struct PinnedColumns {
+    const void* src[GT_NUM_COLUMNS];
+    unsigned long long* dst[GT_NUM_COLUMNS];
+    uint8_t widen[GT_NUM_COLUMNS];
+};
+__global__ void widen_columns_kernel(const PinnedColumns c, int64_t n) {
+    const int k = blockIdx.y;
+    unsigned long long* const o = c.dst[k];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        if (!c.widen[k]) {
+            o[i] = ((const unsigned long long*)c.src[k])[i];
+            continue;
+        }
+        const unsigned u = ((const unsigned*)c.src[k])[i];
+        // a NaN keeps its sign and payload, as the host's conversion does
+        o[i] = (u & 0x7FFFFFFFu) > 0x7F800000u
+                   ? ((unsigned long long)(u >> 31) << 63) | 0x7FF8000000000000ull |
+                         ((unsigned long long)(u & 0x7FFFFFu) << 29)
+                   : (unsigned long long)__double_as_longlong((double)__uint_as_float(u));
+    }
+}
+
+// Where the device stores to host memory `p` of `bytes` bytes, 8-byte aligned
+// and inside one pinned allocation; nullptr for other memory.
+unsigned long long* pinned_address(void* p, size_t bytes) {
+    cudaPointerAttributes at, end;
+    if ((uintptr_t)p % 8 != 0 || cudaPointerGetAttributes(&at, p) != cudaSuccess ||
+        cudaPointerGetAttributes(&end, (char*)p + bytes - 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    const bool one = at.type == cudaMemoryTypeHost && end.type == cudaMemoryTypeHost && at.devicePointer &&
+                     (char*)end.devicePointer == (char*)at.devicePointer + bytes - 1;
+    return one ? (unsigned long long*)at.devicePointer : nullptr;
+}
+
+const TBuf& table_column(const gt_table* t, int32_t c) {
+    return c == GT_COL_FRAME ? t->frame
+                             : (c == GT_COL_PARTICLE ? t->particle : (c == GT_COL_DURATION ? t->duration : t->col[c]));
+}
+
+bool integer_column(int32_t c) { return c == GT_COL_FRAME || c == GT_COL_PARTICLE || c == GT_COL_DURATION; }
+
+// The export into pinned columns; false where one of them is not.
+bool export_to_pinned(const gt_table* t, const int32_t* columns, int32_t ncolumns, void* const* dst, gt_status* st) {
+    if (ncolumns > GT_NUM_COLUMNS) return false;
+    if (cudaSetDevice(t->device) != cudaSuccess) {
+        *st = cuda_failed();
+        return true;
+    }
+    PinnedColumns c;
+    for (int32_t k = 0; k < ncolumns; k++) {
+        c.dst[k] = pinned_address(dst[k], (size_t)t->n * 8);
+        if (!c.dst[k]) return false;
+        c.src[k] = table_column(t, columns[k]).p;
+        c.widen[k] = integer_column(columns[k]) ? 0 : 1;
+    }
+    const cudaStream_t ps = cudaStreamPerThread;   // the call that made the table has finished its work on it
+    const dim3 grid((unsigned)std::min<int64_t>((t->n + 255) / 256, 1024), ncolumns);
+    widen_columns_kernel<<<grid, 256, 0, ps>>>(c, t->n);
+    cudaError_t e = cudaGetLastError();
+    const cudaError_t e2 = cudaStreamSynchronize(ps);
+    if (e == cudaSuccess) e = e2;
+    *st = e == cudaSuccess ? GT_OK : cuda_failed();
+    return true;
+}
+
 gt_status table_export_impl(const gt_table* t, const int32_t* columns, int32_t ncolumns, void* const* dst) {
     if (!t || ncolumns < 0 || (ncolumns > 0 && (!columns || !dst))) return GT_ERR_INVALID_ARGUMENT;
     for (int32_t k = 0; k < ncolumns; k++) {
@@ -152,6 +223,8 @@ gt_status table_export_impl(const gt_table* t, const int32_t* columns, int32_t n
     }
     const int64_t N = t->n;
     if (N == 0 || ncolumns == 0) return GT_OK;
+    gt_status st = GT_OK;
+    if (export_to_pinned(t, columns, ncolumns, dst, &st)) return st;
     ExportPool* pool = export_pool(t->device);
     if (!pool) return GT_ERR_INVALID_ARGUMENT;
     std::lock_guard<std::mutex> lock(pool->mu);
@@ -164,10 +237,8 @@ gt_status table_export_impl(const gt_table* t, const int32_t* columns, int32_t n
         const int64_t r0 = N * l / lanes, r1 = N * (l + 1) / lanes;
         for (int32_t k = 0; k < ncolumns; k++) {
             const int32_t c = columns[k];
-            const bool integer = c == GT_COL_FRAME || c == GT_COL_PARTICLE || c == GT_COL_DURATION;
-            const TBuf& b = c == GT_COL_FRAME ? t->frame
-                                              : (c == GT_COL_PARTICLE ? t->particle
-                                                                      : (c == GT_COL_DURATION ? t->duration : t->col[c]));
+            const bool integer = integer_column(c);
+            const TBuf& b = table_column(t, c);
             const int64_t chunk = (int64_t)(kExportSlot / (integer ? 8 : 4));
             for (int64_t r = r0; r < r1; r += chunk) {
                 ExportItem it;
@@ -198,59 +269,12 @@ gt_status table_export_impl(const gt_table* t, const int32_t* columns, int32_t n
 
 }  // namespace
 
-// Columns widened on the device into one block of 8-byte columns: a float
-// column as doubles, an integer column as it is.  Blocks of threads stride over
-// the rows of column blockIdx.y.
-struct BlockColumns {
-    const void* src[GT_NUM_COLUMNS];
-    uint8_t widen[GT_NUM_COLUMNS];
-};
-__global__ void widen_columns_kernel(const BlockColumns c, int64_t n, unsigned long long* __restrict__ out) {
-    const int k = blockIdx.y;
-    unsigned long long* const o = out + (size_t)k * n;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        if (!c.widen[k]) {
-            o[i] = ((const unsigned long long*)c.src[k])[i];
-            continue;
-        }
-        const unsigned u = ((const unsigned*)c.src[k])[i];
-        // a NaN keeps its sign and payload, as the host's conversion does
-        o[i] = (u & 0x7FFFFFFFu) > 0x7F800000u
-                   ? ((unsigned long long)(u >> 31) << 63) | 0x7FF8000000000000ull |
-                         ((unsigned long long)(u & 0x7FFFFFu) << 29)
-                   : (unsigned long long)__double_as_longlong((double)__uint_as_float(u));
-    }
-}
-
 gt_status gt_table_export_pinned(const gt_table* t, const int32_t* columns, int32_t ncolumns, void* block) {
     if (!t || ncolumns < 0 || ncolumns > GT_NUM_COLUMNS || (ncolumns > 0 && (!columns || !block)))
         return GT_ERR_INVALID_ARGUMENT;
-    if (t->n == 0 || ncolumns == 0) return GT_OK;
-    BlockColumns c;
-    for (int32_t k = 0; k < ncolumns; k++) {
-        const int32_t id = columns[k];
-        if (id < 0 || id >= GT_NUM_COLUMNS || !t->has[id]) return GT_ERR_INVALID_ARGUMENT;
-        const bool integer = id == GT_COL_FRAME || id == GT_COL_PARTICLE || id == GT_COL_DURATION;
-        c.widen[k] = integer ? 0 : 1;
-        c.src[k] = id == GT_COL_FRAME ? t->frame.p
-                                      : (id == GT_COL_PARTICLE ? t->particle.p
-                                                               : (id == GT_COL_DURATION ? t->duration.p : t->col[id].p));
-    }
-    if (cudaSetDevice(t->device) != cudaSuccess) return cuda_failed();
-    const cudaStream_t st = cudaStreamPerThread;   // the call that made the table has finished its work on it
-    TBuf tmp;
-    tmp.device = t->device;
-    tmp.stream = st;
-    const size_t bytes = (size_t)ncolumns * (size_t)t->n * 8;
-    if (tmp.ensure(bytes) != cudaSuccess) {
-        return cuda_failed();
-    }
-    const dim3 grid((unsigned)std::min<int64_t>((t->n + 255) / 256, 1024), ncolumns);
-    widen_columns_kernel<<<grid, 256, 0, st>>>(c, t->n, tmp.as<unsigned long long>());
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(block, tmp.p, bytes, cudaMemcpyDeviceToHost, st);
-    const cudaError_t e2 = cudaStreamSynchronize(st);
-    return e == cudaSuccess && e2 == cudaSuccess ? GT_OK : cuda_failed();
+    void* dst[GT_NUM_COLUMNS];
+    for (int32_t k = 0; k < ncolumns; k++) dst[k] = (char*)block + (size_t)k * (size_t)t->n * 8;
+    return gt_table_export(t, columns, ncolumns, dst);
 }
 
 void* gt_host_alloc(size_t bytes) {

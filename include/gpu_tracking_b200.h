@@ -149,9 +149,10 @@ GT_API gt_status gt_table_column_i64(const gt_table* t, int32_t column, int64_t*
  * destinations may be ordinary pageable memory.  Returns
  * GT_ERR_INVALID_ARGUMENT for a column the table does not have. */
 GT_API gt_status gt_table_export(const gt_table* t, const int32_t* columns, int32_t ncolumns, void* const* dst);
-/* The same columns into one block of ncolumns x rows 8-byte values in pinned
- * memory (gt_host_alloc), column after column: the rows are widened on the
- * device and arrive in one copy, without work of the host's. */
+/* The same columns into one block of ncolumns x rows 8-byte values, column
+ * after column.  Into pinned memory (gt_host_alloc; for gt_table_export every
+ * destination) the device stores the widened values itself: no work of the
+ * host's and no device memory besides the table's. */
 GT_API gt_status gt_table_export_pinned(const gt_table* t, const int32_t* columns, int32_t ncolumns, void* block);
 /* Pinned host memory (NULL when there is none to be had). */
 GT_API void* gt_host_alloc(size_t bytes);
