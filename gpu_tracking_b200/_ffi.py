@@ -188,11 +188,11 @@ class Context:
 
 
 class _Block:
-    """Host memory of one result.  The arrays made from it keep it alive; when
-    the last of them goes, its memory goes back to the pool."""
+    """Host memory of one result column.  The arrays made from it keep it alive;
+    when the last of them goes, its memory goes back to the pool."""
 
-    def __init__(self, pool, size, address, keep=None):
-        self._pool, self._size, self._address, self._keep = pool, size, address, keep
+    def __init__(self, pool, size, address, keep=None, slab=None):
+        self._pool, self._size, self._address, self._keep, self._slab = pool, size, address, keep, slab
         self.__array_interface__ = {"shape": (size,), "typestr": "|u1", "data": (address, False), "version": 3}
 
     @property
@@ -210,79 +210,108 @@ class _Block:
             pass
 
 
-class ResultPool:
-    """Host memory for result tables, in blocks of a power of two.
+class _Slab:
+    """Blocks that were pinned together; `out` of them are in results."""
 
-    The memory of a dropped result serves the next result of its size (104 MB
-    of columns: 7.1 ms into fresh memory, which faults page by page, 3.8 ms
-    into memory used before).  Results arrive in pinned memory in one copy
-    without work of the host's (2.2 ms; 200 KB: 0.20 instead of 0.28), but
-    pinning 128 MB takes 55 ms, 8 MB 9 ms and 64 KB 0.9 ms, what 11 to 34
-    results save.  So a size earns a pinned block by each `PIN_AFTER` results
-    of it that were dropped (a third of them up to 8 MB, where pinning never
-    takes 10 ms): a program that keeps its tables, or makes few, does not pay
-    for it.  Blocks above a quarter of `limit` are never pinned
-    (512 MB: 210 ms).  At most `limit` bytes are pinned, in use and idle
-    together, and at most as many idle bytes of ordinary memory are kept.
+    def __init__(self, address, size, parts):
+        self.address, self.size, self.parts, self.out = address, size, parts, parts
+
+
+class ResultPool:
+    """Host memory for the columns of large results.
+
+    Every column has a block of its own (an eighth larger than the column at
+    most), so a column that is kept keeps nothing else.  The memory of a
+    dropped column serves the next one of its size (88 MB of columns: 5.6-7.6
+    ms into fresh memory, which faults page by page, 2.9-3.8 ms into memory
+    used before).  Pinned memory the device fills by itself (1.7 ms; 26 MB 0.5
+    instead of 1.4-1.9, 3.5 MB 0.09 instead of 0.25), but pinning takes about
+    0.4 ms a megabyte and 2.4 ms at least: what 12 to 20 tables save up to 32
+    MB and 30 to 36 above.  So the columns of a table are pinned, all at once,
+    when `earned` tables of their size were dropped: a program that keeps its
+    tables, or makes few, does not pay for it.  Tables above a quarter of
+    `limit` are never pinned.  At most `limit` bytes are pinned, in use and
+    idle together, and at most as many idle bytes of ordinary memory are kept.
     """
 
-    PIN_AFTER = 12
+    PIN_AFTER = 18
 
     def earned(self, size):
-        return self.PIN_AFTER if size > 8 << 20 else max(1, self.PIN_AFTER // 3)
+        return self.PIN_AFTER if size <= 4 << 20 else 2 * self.PIN_AFTER
 
     def __init__(self, limit=512 << 20):
         self._lock = threading.RLock()   # a block may go while another is taken
         self._limit, self._pinned, self._kept = limit, 0, 0
         self._idle, self._ordinary, self._dropped = {}, {}, {}
 
+    @staticmethod
+    def block_size(nbytes):
+        """The size of the block for nbytes: eight sizes to a power of two, at least 64 KB."""
+        top = 1 << max(16, (max(int(nbytes), 1) - 1).bit_length())
+        step = top // 16 if top > 1 << 16 else top
+        return -(-max(int(nbytes), 1) // step) * step
+
     def take(self, nbytes):
-        size = 1 << max(16, int(nbytes).bit_length())
-        keep = None
+        return self.take_columns(nbytes, 1)[0]
+
+    def take_columns(self, nbytes, count):
+        """`count` blocks of nbytes, pinned all of them or none."""
+        size = self.block_size(nbytes)
+        kept = []
         with self._lock:
-            idle = self._idle.get(size)
-            if idle:
-                return _Block(self, size, idle.pop())
-            ordinary = self._ordinary.get(size)
-            if ordinary:
-                keep = ordinary.pop()
-                self._kept -= size
-            pin = (self._dropped.get(size, 0) >= self.earned(size) and size <= self._limit // 4
-                   and self._pinned + size <= self._limit)
+            idle = self._idle.get(size, [])
+            if len(idle) >= count:
+                return [self._out(size, *idle.pop()) for _ in range(count)]
+            ordinary = self._ordinary.get(size, [])
+            need = self.earned(size) * count
+            pin = (self._dropped.get(size, 0) >= need and size * count <= self._limit // 4
+                   and self._pinned + size * count <= self._limit)
             if pin:
-                self._dropped[size] -= self.earned(size)
-                self._pinned += size
+                self._dropped[size] -= need
+                self._pinned += size * count
+            else:
+                kept = [ordinary.pop() for _ in range(min(count, len(ordinary)))]
+                self._kept -= size * len(kept)
         if pin:
-            address = lib().gt_host_alloc(size)
+            address = lib().gt_host_alloc(size * count)
             if address:
-                return _Block(self, size, address)
+                slab = _Slab(address, size, count)
+                return [_Block(self, size, address + size * k, slab=slab) for k in range(count)]
             with self._lock:
-                self._pinned -= size
-        if keep is None:
-            keep = np.empty(size, np.uint8)
-        return _Block(self, size, keep.ctypes.data, keep)
+                self._pinned -= size * count
+        kept += [np.empty(size, np.uint8) for _ in range(count - len(kept))]
+        return [_Block(self, size, a.ctypes.data, a) for a in kept]
+
+    def _out(self, size, address, slab):
+        slab.out += 1
+        return _Block(self, size, address, slab=slab)
 
     def _back(self, block):
         size = block._size
         with self._lock:
             if block.pinned:
-                self._idle.setdefault(size, []).append(block._address)
+                block._slab.out -= 1
+                self._idle.setdefault(size, []).append((block._address, block._slab))
                 return
-            self._dropped[size] = min(2 * self.PIN_AFTER, self._dropped.get(size, 0) + 1)
+            # as many as a table of every column pins, twice
+            self._dropped[size] = min(2 * 32 * self.earned(size), self._dropped.get(size, 0) + 1)
             if self._kept + size <= self._limit:
                 self._ordinary.setdefault(size, []).append(block._keep)
                 self._kept += size
 
     def trim(self):
-        """Gives the idle blocks back to the system."""
+        """Gives the idle memory back to the system (pinned blocks when all
+        that were pinned with them are idle)."""
+        free = {}
         with self._lock:
-            idle, self._idle = self._idle, {}
             self._ordinary, self._kept = {}, 0
-            for size, addresses in idle.items():
-                self._pinned -= size * len(addresses)
-        for addresses in idle.values():
-            for a in addresses:
-                lib().gt_host_free(a)
+            for size, idle in self._idle.items():
+                free.update((slab.address, slab) for _, slab in idle if not slab.out)
+                self._idle[size] = [part for part in idle if part[1].out]
+            for slab in free.values():
+                self._pinned -= slab.size * slab.parts
+        for address in free:
+            lib().gt_host_free(address)
 
 
 results = ResultPool()

@@ -102,6 +102,7 @@ class _Frames:
         self.T, self.H, self.W = t.shape
 
 
+_SMALL_RESULT = 1 << 20   # bytes that the library hands over in one piece
 _SHORT_PIXELS = 1 << 23   # locating these takes about a millisecond
 
 
@@ -145,6 +146,14 @@ def _run(ctx, fn, show_progress, short=False):
     return result["status"]
 
 
+def _columns(rows, count):
+    """`count` int64 arrays for a result, each with memory of its own: small
+    results in fresh memory, large ones in the pool's."""
+    if 8 * rows * count <= _SMALL_RESULT:
+        return [np.empty(rows, np.int64) for _ in range(count)]
+    return [np.asarray(b)[:8 * rows].view(np.int64) for b in _ffi.results.take_columns(8 * rows, count)]
+
+
 def _table_to_frame(ctx, handle, params, has_r=None):
     L = _ffi.lib()
     try:
@@ -153,20 +162,15 @@ def _table_to_frame(ctx, handle, params, has_r=None):
         if has_r is not None and not has_r:
             cols = [c for c in cols if c[0] != "r"]
         # the DataFrame's own dtypes (int64 / float64) filled by one library
-        # call, column after column in one block of host memory; the frame
-        # takes the columns as they are, without a copy
-        block = _ffi.results.take(8 * n * len(cols))
-        columns = np.asarray(block)[:8 * n * len(cols)].reshape(len(cols), 8 * n)
+        # call; the frame takes the arrays as they are, without a copy
+        arrays = _columns(n, len(cols))
         if n and cols:
             idx = (ctypes.c_int32 * len(cols))(*[COLUMN_INDEX[name] for name, _ in cols])
-            if block.pinned:
-                ctx.check(L.gt_table_export_pinned(handle, idx, len(cols), block.address))
-            else:
-                ptrs = (ctypes.c_void_p * len(cols))(*[block.address + 8 * n * k for k in range(len(cols))])
-                ctx.check(L.gt_table_export(handle, idx, len(cols), ptrs))
+            ptrs = (ctypes.c_void_p * len(cols))(*[a.__array_interface__["data"][0] for a in arrays])
+            ctx.check(L.gt_table_export(handle, idx, len(cols), ptrs))
     finally:
         L.gt_table_free(handle)
-    data = {name: columns[k].view(np.int64 if ty == "int" else np.float64) for k, (name, ty) in enumerate(cols)}
+    data = {name: a if ty == "int" else a.view(np.float64) for a, (name, ty) in zip(arrays, cols)}
     pd = _pandas()
     return pd.DataFrame(data, index=pd.RangeIndex(n), copy=False)
 
@@ -323,7 +327,7 @@ def link(to_link, search_range, memory=0):
     if arr.ndim != 2 or arr.shape[1] != 3:
         raise ValueError("link expects (N, 3) rows of frame, y, x")
     ctx = _ffi.context(_DEVICE)
-    ids = np.asarray(_ffi.results.take(8 * len(arr)))[:8 * len(arr)].view(np.int64)
+    ids = _columns(len(arr), 1)[0]
     ctx.check(_ffi.lib().gt_link(ctx.handle, arr.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), len(arr),
                                  float(search_range), int(memory or 0),
                                  ids.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))))

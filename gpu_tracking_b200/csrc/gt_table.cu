@@ -191,27 +191,28 @@ const TBuf& table_column(const gt_table* t, int32_t c) {
 
 bool integer_column(int32_t c) { return c == GT_COL_FRAME || c == GT_COL_PARTICLE || c == GT_COL_DURATION; }
 
+// Columns of the table widened into the pinned columns c.dst (on a stream of
+// the caller's: the call that made the table has finished its work on it).
+gt_status widen_columns(const gt_table* t, const int32_t* columns, int32_t ncolumns, PinnedColumns& c,
+                        cudaStream_t st) {
+    for (int32_t k = 0; k < ncolumns; k++) {
+        c.src[k] = table_column(t, columns[k]).p;
+        c.widen[k] = integer_column(columns[k]) ? 0 : 1;
+    }
+    const dim3 grid((unsigned)std::min<int64_t>((t->n + 255) / 256, 1024), ncolumns);
+    widen_columns_kernel<<<grid, 256, 0, st>>>(c, t->n);
+    const cudaError_t e = cudaGetLastError(), e2 = cudaStreamSynchronize(st);
+    return e == cudaSuccess && e2 == cudaSuccess ? GT_OK : cuda_failed();
+}
+
 // The export into pinned columns; false where one of them is not.
 bool export_to_pinned(const gt_table* t, const int32_t* columns, int32_t ncolumns, void* const* dst, gt_status* st) {
-    if (ncolumns > GT_NUM_COLUMNS) return false;
-    if (cudaSetDevice(t->device) != cudaSuccess) {
-        *st = cuda_failed();
-        return true;
-    }
     PinnedColumns c;
     for (int32_t k = 0; k < ncolumns; k++) {
         c.dst[k] = pinned_address(dst[k], (size_t)t->n * 8);
         if (!c.dst[k]) return false;
-        c.src[k] = table_column(t, columns[k]).p;
-        c.widen[k] = integer_column(columns[k]) ? 0 : 1;
     }
-    const cudaStream_t ps = cudaStreamPerThread;   // the call that made the table has finished its work on it
-    const dim3 grid((unsigned)std::min<int64_t>((t->n + 255) / 256, 1024), ncolumns);
-    widen_columns_kernel<<<grid, 256, 0, ps>>>(c, t->n);
-    cudaError_t e = cudaGetLastError();
-    const cudaError_t e2 = cudaStreamSynchronize(ps);
-    if (e == cudaSuccess) e = e2;
-    *st = e == cudaSuccess ? GT_OK : cuda_failed();
+    *st = widen_columns(t, columns, ncolumns, c, cudaStreamPerThread);
     return true;
 }
 
@@ -223,12 +224,25 @@ gt_status table_export_impl(const gt_table* t, const int32_t* columns, int32_t n
     }
     const int64_t N = t->n;
     if (N == 0 || ncolumns == 0) return GT_OK;
+    if (cudaSetDevice(t->device) != cudaSuccess) return cuda_failed();
     gt_status st = GT_OK;
-    if (export_to_pinned(t, columns, ncolumns, dst, &st)) return st;
+    if (ncolumns <= GT_NUM_COLUMNS && export_to_pinned(t, columns, ncolumns, dst, &st)) return st;
     ExportPool* pool = export_pool(t->device);
     if (!pool) return GT_ERR_INVALID_ARGUMENT;
     std::lock_guard<std::mutex> lock(pool->mu);
-    if (cudaSetDevice(t->device) != cudaSuccess || export_pool_init(*pool) != cudaSuccess) return cuda_failed();
+    if (export_pool_init(*pool) != cudaSuccess) return cuda_failed();
+    const size_t bytes = (size_t)N * 8;
+    if (ncolumns <= GT_NUM_COLUMNS && bytes * ncolumns <= kExportSlot) {
+        // a result of one slot: widened on the device into the slot, one copy a
+        // column from there (2000 rows of 11 columns: 31 us; a copy and an
+        // event a column: 74)
+        ExportLane& L = pool->lane[0];
+        PinnedColumns c;
+        for (int32_t k = 0; k < ncolumns; k++) c.dst[k] = (unsigned long long*)(L.slot[0] + bytes * k);
+        if ((st = widen_columns(t, columns, ncolumns, c, L.st)) != GT_OK) return st;
+        for (int32_t k = 0; k < ncolumns; k++) memcpy(dst[k], L.slot[0] + bytes * k, bytes);
+        return GT_OK;
+    }
     // lanes: one per 256k rows, at most kExportLanes and half the host threads
     const int hw = std::max(1, (int)std::thread::hardware_concurrency() / 2);
     const int lanes = (int)std::max<int64_t>(1, std::min<int64_t>({kExportLanes, hw, (N + (1 << 18) - 1) >> 18}));
