@@ -158,16 +158,11 @@ void set_fast_div(gt_ctx* ctx, LocateConsts& c) {
     c.fast_div = 1;
 }
 
-// (sin 2θ, cos 2θ) tables per integer radius 0..max_rint (characterize.wgsl:120-124)
-// The tables of smaller radii are the first part of those of larger ones: one
-// list for the process, grown to the largest radius asked for.
-void angle_tables(int max_rint, std::vector<float2>& tab, std::vector<int32_t>& off) {
-    static std::mutex mu;
-    static std::vector<float2> all;
-    static std::vector<int32_t> starts;
-    std::lock_guard<std::mutex> lock(mu);
-    for (int r = (int)starts.size(); r <= max_rint; r++) {
-        starts.push_back((int32_t)all.size());
+// (sin 2θ, cos 2θ) tables per integer radius 0..max_rint (characterize.wgsl:120-124):
+// appends those of the radii from off.size() on.
+void append_angle_tables(int max_rint, std::vector<float2>& tab, std::vector<int32_t>& off) {
+    for (int r = (int)off.size(); r <= max_rint; r++) {
+        off.push_back((int32_t)tab.size());
         for (int i = -r; i <= r; i++)
             for (int j = -r; j <= r; j++) {
                 float x = (float)i, y = (float)j;
@@ -176,12 +171,35 @@ void angle_tables(int max_rint, std::vector<float2>& tab, std::vector<int32_t>& 
                     float theta = std::atan2(y, x);
                     v = make_float2(std::sin(2.0f * theta), std::cos(2.0f * theta));
                 }
-                all.push_back(v);
+                tab.push_back(v);
             }
     }
-    const int n = std::max(max_rint + 1, 0);
-    off.assign(starts.begin(), starts.begin() + n);
-    tab.assign(all.begin(), n < (int)starts.size() ? all.begin() + starts[(size_t)n] : all.end());
+}
+
+// The tables of smaller radii are the first part of those of larger ones: one
+// list for the process, grown to the largest radius asked for, but not past
+// kSharedAngles (2.9 MB).  Larger ones, which grow with the cube of the radius,
+// belong to the call.
+constexpr int kSharedAngles = 64;
+void angle_tables(int max_rint, std::vector<float2>& tab, std::vector<int32_t>& off) {
+    static std::mutex mu;
+    static std::vector<float2> all;
+    static std::vector<int32_t> starts;
+    const int n = std::min(std::max(max_rint, -1), kSharedAngles) + 1;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        const bool have = n <= (int)starts.size();
+        off.assign(starts.begin(), have ? starts.begin() + n : starts.end());
+        tab.assign(all.begin(), n < (int)starts.size() ? all.begin() + starts[(size_t)n] : all.end());
+        if (!have) {
+            append_angle_tables(n - 1, tab, off);
+            std::vector<float2> t(tab);
+            std::vector<int32_t> o(off);
+            all.swap(t);
+            starts.swap(o);
+        }
+    }
+    append_angle_tables(max_rint, tab, off);
 }
 
 // circle_inds / annulus_inds (src/kernels.rs:138-171)
