@@ -1933,6 +1933,7 @@ gt_status gt__device_span_check(gt_ctx* ctx, const void* p, size_t bytes, const 
     return GT_OK;
 }
 cudaStream_t gt__ctx_stream(const gt_ctx* ctx) { return ctx->st; }
+ScratchPool* gt__ctx_train_scratch(gt_ctx* ctx) { return &ctx->train_scratch; }
 void gt__ctx_set_error(gt_ctx* ctx, const char* msg) { ctx->err = msg; }
 
 // Test hook (exported, not part of the public header): the entries of each

@@ -16,6 +16,7 @@
 extern "C" int gt__ctx_device(const gt_ctx* ctx);
 extern "C" cudaStream_t gt__ctx_stream(const gt_ctx* ctx);
 extern "C" void gt__ctx_set_error(gt_ctx* ctx, const char* msg);
+extern "C" ScratchPool* gt__ctx_train_scratch(gt_ctx* ctx);
 
 namespace gt {
 
@@ -48,57 +49,72 @@ gt_status fail(gt_ctx* ctx, gt_status st, const std::string& msg) {
         }                                                                                                 \
     } while (0)
 
-// Device buffers of one call, freed on every exit path.  With `keep` (a list of
-// buffers that outlives the call) the k-th request takes the k-th buffer of
-// the list where it is large enough, and the call's buffers stay there for the
-// next one unless they hold more than kScratchKeep bytes together.
+// Device buffers of one call, freed on every exit path.  With a pool the k-th
+// request takes the k-th buffer that the last call left there where it is large
+// enough, and the call's buffers go back unless they hold more than
+// kScratchKeep bytes together or another call's are there already.
 constexpr size_t kScratchKeep = (size_t)512 << 20;
 struct Scratch {
-    std::vector<ScratchBuf> bufs;
-    std::vector<ScratchBuf>* keep;
+    std::vector<ScratchBuf> bufs, old;   // this call's, and the pool's that it has not used
+    ScratchPool* pool;
     cudaStream_t stream;   // what runs on the buffers
-    explicit Scratch(std::vector<ScratchBuf>* k = nullptr, cudaStream_t st = nullptr) : keep(k), stream(st) {}
+    explicit Scratch(ScratchPool* p = nullptr, cudaStream_t st = nullptr) : pool(p), stream(st) {
+        if (!pool) return;
+        std::lock_guard<std::mutex> lock(pool->mu);
+        old.swap(pool->bufs);
+    }
     Scratch(const Scratch&) = delete;
     Scratch& operator=(const Scratch&) = delete;
-    cudaError_t get(void** p, size_t bytes) {
-        *p = nullptr;
-        const size_t at = bufs.size();
-        if (keep && at < keep->size()) {
-            ScratchBuf& b = (*keep)[at];
-            if (b.bytes >= bytes) {
-                bufs.push_back(b);
-                b = ScratchBuf();
-                *p = bufs.back().p;
-                return cudaSuccess;
-            }
+    static void release(std::vector<ScratchBuf>& v) {
+        for (ScratchBuf& b : v) {
             if (b.p) cudaFree(b.p);
             b = ScratchBuf();
         }
+    }
+    cudaError_t get(void** p, size_t bytes) {
+        *p = nullptr;
+        const size_t at = bufs.size();
         ScratchBuf n;
-        n.bytes = std::max<size_t>(bytes, 256);
-        cudaError_t e = cudaMalloc(&n.p, n.bytes);
-        if (e != cudaSuccess) return e;
+        if (at < old.size()) {
+            std::swap(n, old[at]);
+            if (n.p && n.bytes < bytes) {
+                cudaFree(n.p);
+                n = ScratchBuf();
+            }
+        }
+        if (!n.p) {
+            n.bytes = std::max<size_t>(bytes, 256);
+            cudaError_t e = cudaMalloc(&n.p, n.bytes);
+            if (e != cudaSuccess) {
+                // once more without what the pool still holds
+                cudaGetLastError();
+                release(old);
+                e = cudaMalloc(&n.p, n.bytes);
+                if (e != cudaSuccess) return e;
+            }
+        }
         bufs.push_back(n);
         *p = n.p;
-        return e;
+        return cudaSuccess;
     }
     template <class T>
     cudaError_t get(T** p, size_t bytes) {
         return get((void**)p, bytes);
     }
     ~Scratch() {
-        if (keep) cudaStreamSynchronize(stream);   // a call that failed may have left work behind
-        size_t total = 0;
-        for (const ScratchBuf& b : bufs) total += b.bytes;
-        if (keep && total <= kScratchKeep) {
-            for (size_t i = 0; i < bufs.size(); i++) {
-                if (i >= keep->size()) keep->resize(i + 1);
-                if ((*keep)[i].p) cudaFree((*keep)[i].p);
-                (*keep)[i] = bufs[i];
+        if (pool) {
+            cudaStreamSynchronize(stream);   // a call that failed may have left work behind
+            for (size_t i = bufs.size(); i < old.size(); i++) {
+                bufs.push_back(old[i]);
+                old[i] = ScratchBuf();
             }
-            return;
+            size_t total = 0;
+            for (const ScratchBuf& b : bufs) total += b.bytes;
+            std::lock_guard<std::mutex> lock(pool->mu);
+            if (total <= kScratchKeep && pool->bufs.empty()) pool->bufs.swap(bufs);
         }
-        for (const ScratchBuf& b : bufs) cudaFree(b.p);
+        release(bufs);
+        release(old);
     }
 };
 
@@ -294,7 +310,6 @@ GT_API void gt_proposal_destroy(gt_proposal* p) {
     cudaSetDevice(p->device);
     for (void* q : {(void*)p->params, (void*)p->adam_m, (void*)p->adam_v, (void*)p->grad, (void*)p->packed})
         if (q) cudaFree(q);
-    for (const ScratchBuf& b : p->scratch) cudaFree(b.p);
     cudaSetDevice(cur);
     delete p;
 }
@@ -351,7 +366,7 @@ GT_API gt_status gt_proposal_train(gt_ctx* ctx, gt_proposal* p, const void* fram
     cudaStream_t st = gt__ctx_stream(ctx);
     const int sms = num_sms(p->device);
     const int Hc = (H + 3) / 4, Wc = (W + 3) / 4, CH = o.crop / 4, CW = o.crop / 4;
-    Scratch s(&p->scratch, st);
+    Scratch s(gt__ctx_train_scratch(ctx), st);
     const void* dframes = nullptr;
     {
         gt_status r = device_frames(ctx, s, frames, dtype, T, H, W, &dframes, st);

@@ -2,6 +2,7 @@
 // gt_proposal handle (device parameters, Adam state, packed UMMA operands).
 #pragma once
 
+#include <mutex>
 #include <vector>
 
 #include "gt_kernels.h"
@@ -10,6 +11,16 @@
 struct ScratchBuf {
     void* p = nullptr;
     size_t bytes = 0;
+};
+
+// A context's working memory for training, kept between calls whatever network
+// they train; a call takes all of it and puts it back.
+struct ScratchPool {
+    std::mutex mu;
+    std::vector<ScratchBuf> bufs;
+    ~ScratchPool() {
+        for (const ScratchBuf& b : bufs) cudaFree(b.p);
+    }
 };
 
 struct gt_proposal {
@@ -26,7 +37,6 @@ struct gt_proposal {
     size_t off_f[gt::kCnnLayers] = {};
     size_t off_d[gt::kCnnLayers] = {};
     size_t packed_bytes = 0;
-    std::vector<ScratchBuf> scratch;   // training's working memory, kept between calls
 
     gt::CnnNet views() const {
         gt::CnnNet n;

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "gt_kernels.h"
+#include "gt_proposal.h"
 
 namespace gt {
 namespace rt {
@@ -164,6 +165,7 @@ struct gt_ctx {
     // windowed linking inside gt_batch (slot mode)
     DBuf fstd, std_scratch, amask, astatus, acount;   // snr / minmass_snr / adaptive_background
     DBuf illum_taps, illum_shared, illum_prof, illum_corr, illum_norm;  // illumination correction
+    ScratchPool train_scratch;            // network training
     DBuf cnn_x, cnn_p, cnn_q, cnn_head;   // learned proposals: network input, activations, outputs
     DBuf walk_starts;                     // walk starts of the current call (u64)
     DBuf vd_src, vd_dec, vd_blk, vd_bad;  // video files decoded on the device: streams, bytes, blocks, flag
