@@ -406,11 +406,12 @@ struct PipeLink {
         out.dur_range = segmented ? 1 : 0;
         if (segmented) {
             CK(ctx->w_segst.ensure(sizeof(LinkSeg) * (size_t)segs.max_segs));
-            CK(ctx->w_segarr.ensure(4));
+            CK(ctx->w_segarr.ensure(12));
             segs.base = ctx->w_segs.as<uint8_t>();
             segs.seg = ctx->w_segst.as<LinkSeg>();
             segs.arrived = ctx->w_segarr.as<uint32_t>();
-            CK(cudaMemsetAsync(segs.arrived, 0, 4, ctx->lk));
+            segs.again = segs.arrived + 1;
+            CK(cudaMemsetAsync(segs.arrived, 0, 12, ctx->lk));
             CK(cudaMemsetAsync(segs.seg, 0, sizeof(LinkSeg) * (size_t)segs.max_segs, ctx->lk));
             CK(cudaMemsetAsync(ctx->w_dur.p, 0, NS * 8, ctx->lk));
         } else {
@@ -1952,6 +1953,17 @@ GT_API gt_status gt__get_link_window_caps(const gt_ctx* ctx, int64_t* list_entri
     if (!ctx || !list_entries || !edges_per_frame) return GT_ERR_INVALID_ARGUMENT;
     *list_entries = ctx->w_list_cap;
     *edges_per_frame = ctx->w_edge_cap;
+    return GT_OK;
+}
+
+// Test hook: segments that the last gt_batch with segmented windows linked
+// again, before its last window and in it.
+GT_API gt_status gt__relinked_segments(gt_ctx* ctx, uint32_t* before_last, uint32_t* in_last) {
+    uint32_t n[3] = {};
+    if (!ctx || !before_last || !in_last) return GT_ERR_INVALID_ARGUMENT;
+    if (ctx->w_segarr.p) CK(cudaMemcpy(n, ctx->w_segarr.p, sizeof(n), cudaMemcpyDeviceToHost));
+    *before_last = n[1];
+    *in_last = n[2];
     return GT_OK;
 }
 

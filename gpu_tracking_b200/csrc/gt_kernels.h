@@ -350,6 +350,7 @@ struct LinkSegs {
     int64_t points = 0;           // points that len + prefix frames hold at most (slot mode: slots)
     LinkSeg* seg = nullptr;       // nvideos x max_segs, zero before the first launch
     uint32_t* arrived = nullptr;  // per video, zero before the first launch
+    uint32_t* again = nullptr;    // optional: segments linked again, [0] before the last window and [1] in it
 };
 
 cudaError_t link_sort_groups(const LinkInput& in, uint32_t* srt, uint8_t* scratch, size_t scratch_per_group,

@@ -1554,6 +1554,7 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
             seg[t].head = sh.head;
             seg[t].counter = gcount;
             seg[t].final_ids = 1;
+            if (Q.again) atomicAdd(Q.again + (W.last ? 1 : 0), 1u);
         }
         cur = t;
         cur_true = true;
