@@ -1085,7 +1085,7 @@ gt_status batch_impl(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_d
             return set_err(ctx, GT_ERR_INVALID_ARGUMENT,
                            "adaptive_background >= 2 needs snr or minmass_snr (the image std between passes)");
     }
-    const int F = pick_chunk(NT, H, W, (log_style && !lt.fused()) ? (int)lt.radii.size() : 0);
+    int F = pick_chunk(NT, H, W, (log_style && !lt.fused()) ? (int)lt.radii.size() : 0);
     ctx->total = NT;
     ctx->done = 0;
     std::vector<int64_t> fnum(NT);
@@ -1098,6 +1098,7 @@ gt_status batch_impl(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_d
     bool windowed = false;
     for (int attempt = 0;; attempt++) {
         uint32_t fl = 0;
+        ctx->no_memory = false;
         HostSpan hs(ctx, "host_locate");
         // frames link while later frames are located unless a frame may hold
         // more detections than a link window's buffers are sized for (lists
@@ -1107,6 +1108,16 @@ gt_status batch_impl(gt_ctx* ctx, const gt_params& p, const T* frames, bool on_d
                                       windowed ? &pl : nullptr, &reset, net);
         if (st != GT_OK) {
             sync_link_streams(ctx);
+            if (st == GT_ERR_CUDA && ctx->no_memory && F > 1) {
+                // once more with half the frames a launch
+                CK(cudaStreamSynchronize(ctx->st));
+                for (DBuf* b : {&ctx->processed, &ctx->planes, &ctx->cand_keys, &ctx->illum_corr, &ctx->illum_prof,
+                                &ctx->std_scratch, &ctx->amask, &ctx->cnn_x, &ctx->cnn_p, &ctx->cnn_q, &ctx->cnn_head})
+                    b->release();
+                F = (F + 1) / 2;
+                attempt--;
+                continue;
+            }
             return st;
         }
         if (fl & (kFlagTensorTimeout | kFlagLocalWalk)) {
@@ -1291,9 +1302,16 @@ gt_status charpoints_impl(gt_ctx* ctx, const gt_params& p0, const T* frames, boo
     if (bandpass_smem_bytes(c.R, 1, false) > 227 * 1024)
         return set_err(ctx, GT_ERR_INVALID_ARGUMENT, "smoothing_size too large for the tile kernel");
     const size_t npx = (size_t)H * W;
-    const int F = pick_chunk(G, H, W, 0);
+    int F = pick_chunk(G, H, W, 0);
     const uint32_t feat_cap = (uint32_t)std::max<int64_t>(maxg, 1);
     if (feat_cap >= (1u << 24)) return set_err(ctx, GT_ERR_CAPACITY_EXCEEDED, "too many points in one frame");
+    // fewer frames a launch where there is no memory for them
+    while (F > 1 && !(try_ensure(ctx, ctx->processed, (size_t)F * npx * 4) &&
+                      try_ensure(ctx, ctx->feats_raw, (size_t)F * feat_cap * sizeof(Feature)) &&
+                      (on_device || try_ensure(ctx, ctx->stage[0], (size_t)F * npx * sizeof(T))))) {
+        for (DBuf* b : {&ctx->processed, &ctx->feats_raw, &ctx->stage[0]}) b->release();
+        F = (F + 1) / 2;
+    }
     CK(ctx->processed.ensure((size_t)F * npx * 4));
     CK(ctx->feats_raw.ensure((size_t)F * feat_cap * sizeof(Feature)));
     CK(ctx->feat_count.ensure((size_t)F * 4));

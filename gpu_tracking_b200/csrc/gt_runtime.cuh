@@ -33,11 +33,14 @@ struct DBuf {
     ~DBuf() {
         if (p) cudaFree(p);
     }
-    cudaError_t ensure(size_t bytes) {
-        if (bytes <= n && p) return cudaSuccess;
+    void release() {
         if (p) cudaFree(p);
         p = nullptr;
         n = 0;
+    }
+    cudaError_t ensure(size_t bytes) {
+        if (bytes <= n && p) return cudaSuccess;
+        release();
         // an eighth of headroom at most, so that inputs of about the same size
         // (detections differ from video to video) do not allocate again
         size_t want = 256;
@@ -185,6 +188,7 @@ struct gt_ctx {
     Mail* mail = nullptr;
     bool mail_kept = false;   // mail->kept holds the last locate pass's counts
     int32_t ident_n = 0;      // entries of ident that hold their own index
+    bool no_memory = false;      // a CK of this context failed for want of device memory
     size_t optional_limit = 0;   // test hook: bytes a buffer of try_ensure may have (0: no limit)
     // segments of the linker's frame loop: scratch of the speculative runs, their states, arrivals
     DBuf w_segs, w_segst, w_segarr, l_segs, l_segst, l_segarr;
@@ -255,9 +259,11 @@ inline gt_status cuda_failed() {
 #define CK(expr)                                                                                               \
     do {                                                                                                       \
         cudaError_t e_ = (expr);                                                                               \
-        if (e_ != cudaSuccess)                                                                                 \
+        if (e_ != cudaSuccess) {                                                                               \
+            ctx->no_memory = e_ == cudaErrorMemoryAllocation;                                                  \
             return set_err(ctx, cuda_failed(), "CUDA error %s at %s:%d (%s)", cudaGetErrorString(e_), __FILE__, \
                            __LINE__, #expr);                                                                   \
+        }                                                                                                      \
     } while (0)
 
 #define CKS(expr)                        \
