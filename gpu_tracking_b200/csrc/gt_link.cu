@@ -1344,9 +1344,12 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
                 }
         }
     };
-    const bool stopped = link_stopped(out.flags + v, &sh_last);
+    // A window that stopped has left no state for the next one.  (The counts of
+    // arrivals that this leaves open are cleared before the next call's first
+    // launch; until then every CTA returns here.)
+    if (link_stopped(out.flags + v, &sh_last)) return;
     if (tid == 0) {
-        seg[s].flags = stopped ? kFlagScratch : 0;   // nothing to compare when the video has stopped
+        seg[s].flags = 0;
         seg[s].c0 = 0;
         sh.counter = 0;
         sh.frame = 0;
@@ -1401,7 +1404,7 @@ link_segments_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, L
     }
     __syncthreads();
 
-    if (!stopped) link_frames<SF, true>(in, L, S, out, gb, run, sh_lo, sh_hi, sh);
+    link_frames<SF, true>(in, L, S, out, gb, run, sh_lo, sh_hi, sh);
     __syncthreads();
     {
         int32_t* const rn = (int32_t*)(run.base + (run.spec ? pl.ring_n : ml.ring_n));

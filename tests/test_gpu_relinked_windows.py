@@ -8,9 +8,8 @@ import numpy as np
 import pytest
 
 import gpu_tracking_b200 as gt
-from gpu_tracking_b200 import _ffi
 from gpu_tracking_b200._params import trackpy_params
-from test_gpu_link_stops import LINK_COLS, hook
+from test_gpu_link_stops import LINK_COLS, ctx, hook  # noqa: F401
 from test_gpu_parity import assert_same
 
 pytestmark = pytest.mark.gpu
@@ -32,14 +31,13 @@ def blinking(frames, n, seed, side=96, seen=0.6, step=1.6):
 
 
 @pytest.mark.parametrize("memory,seed,frames", [(0, 0, 290), (1, 1, 290), (3, 0, 290), (3, 2, 290), (3, 0, 400)])
-def test_relinked_before_the_last_window(oracle, memory, seed, frames):
+def test_relinked_before_the_last_window(oracle, ctx, memory, seed, frames):
     f = blinking(frames, 40, seed)
     kw = dict(minmass=300.0, separation=6, search_range=9.0, memory=memory)
     tab = oracle.batch(trackpy_params(7, **kw), f.astype(np.float32))
     assert_same(gt.batch(f, 7, tqdm=False, **kw), tab, LINK_COLS)
     n = (ctypes.c_uint32(), ctypes.c_uint32())
     P = ctypes.POINTER(ctypes.c_uint32)
-    ctx = _ffi.context(0)
     ctx.check(hook("gt__relinked_segments", P, P)(ctx.handle, ctypes.byref(n[0]), ctypes.byref(n[1])))
     if memory:      # without memory a boundary's state is its detections alone, and always holds
         assert n[0].value > 0

@@ -8,25 +8,15 @@ import numpy as np
 import pytest
 
 import gpu_tracking_b200 as gt
-from gpu_tracking_b200 import _ffi
 from gpu_tracking_b200._params import trackpy_params
 from synth import video
 from test_gpu_link_segments import rows
-from test_gpu_link_stops import LINK_COLS, hook
+from test_gpu_link_stops import LINK_COLS, ctx, hook  # noqa: F401
 from test_gpu_parity import assert_same
 
 pytestmark = pytest.mark.gpu
 
 GIB = 1 << 30
-
-
-@pytest.fixture
-def ctx(monkeypatch):
-    """A context of its own: what its buffers hold is this test's."""
-    c = _ffi.Context(0)
-    monkeypatch.setitem(_ffi._contexts, 0, c)
-    yield c
-    c.close()
 
 
 @pytest.fixture(scope="module")
