@@ -1213,11 +1213,12 @@ link_video_kernel(LinkInput in, LinkLists L, LinkScratch S, LinkOutput out, Link
 // result is the sequential linker's in every case, a boundary that does not
 // hold costs its frames.
 // Measured on a B200, one video: 400 frames of 2000 given points, memory 3,
-// 16.4 ms in one CTA and 1.17 ms here (40 segments of 10 frames, each run with
-// a prefix of 10; 1.66 ms while the last CTA compared all boundaries in turn);
-// 512 located frames of 2048^2 with 2000 spots: 4.4 ms of linking left after
-// the last frame is located and 1 ms here.  Boundaries that did not hold: none
-// of 39 at search_range 7 and step 1.4 px, 4 of 39 at search_range 5 (3.4 ms).
+// 16.4 ms in one CTA and 0.98 ms here (80 segments of 5 frames, each run with a
+// prefix of 10; 1.55 ms where the points mix freely); 512 located frames of
+// 2048^2 with 2000 spots: 4.4 ms of linking left after the last frame is located
+// and 1 ms here.  Boundaries that did not hold, freely mixing points, step 1.4
+// px: none of 79 at search_range 7 or 9, 7 of 79 at search_range 5 (4.3 ms); none
+// with memory 0 or 1.
 
 // Points of frames [g0, g1).
 __device__ __forceinline__ int64_t frames_points(const LinkInput& in, int g0, int g1) {
